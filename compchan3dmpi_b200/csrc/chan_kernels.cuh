@@ -79,16 +79,12 @@ struct KParams {
     void *qout;
     double *wp;
     const double *cs;
-    // per-k tables [nP3+2]
-    const double *czh;    // 0.5*invdXi*invJac(k)
-    const double *cz8;    // invdXi*invJac(k)/8
-    const double *cz12;   // invdXi*invJac(k)/12
-    const double *pez;    // Re*dXi*jac(k)
-    const float *tabf;    // the same four tables in float, [4][nP3+2] (mixed precision)
+    const double *czh;    // 0.5*invdXi*invJac(k), [nP3+2]
+    // the stage kernel's constants of each plane (KTab), [nP3+2][8], in its ring type
+    const void *ktab;
     // forcing / stats
     double *stat;         // stat1[7*n3] | stat2[7*n3] | corr[9*n3] | tau[2]
     double *tacc;         // running sums of the same 23*n3+2 numbers over statistics steps
-    double *hwt;          // [4][nP2+2][px] hD on the top wall plane, staged by the last k-chunk
     DevStatus *status;
     // physics
     double invRe, ggM, ggMh, gM2, inv_gM2, kq, two3rd;
@@ -102,6 +98,7 @@ struct KParams {
     double f1[3], f2[3], b1[3], b2[3];  // wall one-sided coefficients
     // RK stage
     double rk_a, rk_b, rk_cdt;
+    double rk_eps;        // a + b - 1 of the rounded a, b (0 but for a = 1/3, b = 2/3)
     int rk_mode;          // 0: in + cdt*R ; 1: base + cdt*R ; 2: a*base + b*in + cdt*R
     int check;            // last stage of a step: run the blow-up test
     int force_on;
@@ -144,6 +141,24 @@ __device__ __forceinline__ void flag_nonfinite(DevStatus *st, int i, int j, int 
     }
 }
 
+// Single-rounding multiply-add in the ring type.  The viscous fluxes are
+// written with explicit FMAs so that every place that evaluates one (own
+// columns, halo lanes, the k-march prologue) rounds it the same way, and a
+// point's result does not depend on the launch shape that computed it.
+template <typename R>
+__device__ __forceinline__ R fmaR(R a, R b, R c);
+template <>
+__device__ __forceinline__ double fmaR<double>(double a, double b, double c) { return __fma_rn(a, b, c); }
+template <>
+__device__ __forceinline__ float fmaR<float>(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+// an add the compiler may not fuse with a product feeding it
+template <typename R>
+__device__ __forceinline__ R addR(R a, R b);
+template <>
+__device__ __forceinline__ double addR<double>(double a, double b) { return __dadd_rn(a, b); }
+template <>
+__device__ __forceinline__ float addR<float>(float a, float b) { return __fadd_rn(a, b); }
+
 // ---------------------------------------------------------------------------
 // Inviscid stencil weights.  Both branches of the reference's hybrid scheme are
 // linear in the conservative variable once the velocities are fixed, so a
@@ -163,51 +178,48 @@ __device__ __forceinline__ void quick_weights(R um1, R u0, R up1, R s8, R w[5])
     const R ae_m1 = e ? R(-1) : R(0), ae_0 = e ? R(6) : R(3), ae_1 = e ? R(3) : R(6), ae_2 = e ? R(0) : R(-1);
     const R bw_m2 = f ? R(-1) : R(0), bw_m1 = f ? R(6) : R(3), bw_0 = f ? R(3) : R(6), bw_1 = f ? R(0) : R(-1);
     w[0] = -R2 * bw_m2;
-    w[1] = R1 * ae_m1 - R2 * bw_m1;
-    w[2] = R1 * ae_0 - R2 * bw_0;
-    w[3] = R1 * ae_1 - R2 * bw_1;
+    w[1] = fmaR(R1, ae_m1, -(R2 * bw_m1));
+    w[2] = fmaR(R1, ae_0, -(R2 * bw_0));
+    w[3] = fmaR(R1, ae_1, -(R2 * bw_1));
     w[4] = R1 * ae_2;
 }
 
+// s12o: the outer pair's coefficient (s12, or 0 where the scheme next to a wall
+// uses the inner pair alone)
 template <typename R>
-__device__ __forceinline__ void central_weights(R um2, R um1, R up1, R up2, R s12, R w[5])
+__device__ __forceinline__ void central_weights(R um2, R um1, R up1, R up2, R s12, R s12o, R w[5])
 {
-    w[0] = um2 * s12;
+    w[0] = um2 * s12o;
     w[1] = R(-8) * um1 * s12;
     w[2] = R(0);
     w[3] = R(8) * up1 * s12;
-    w[4] = -(up2 * s12);
+    w[4] = -(up2 * s12o);
 }
 
 template <typename R>
-__device__ __forceinline__ void inv_weights(R um2, R um1, R u0, R up1, R up2, bool quick, R s8, R s12, R w[5])
+__device__ __forceinline__ void inv_weights(R um2, R um1, R u0, R up1, R up2, bool quick, R s8, R s12, R s12o, R w[5])
 {
     // Both weight sets, then a select per weight.  The switch differs from lane
     // to lane where the cell Peclet number crosses its limit, and a branch there
     // runs both paths one after the other (2.6% of the FP64 stage time, 1% of the
-    // float one together with the top-plane hoist below).
-#ifndef CHAN_INV_BRANCH
-    constexpr bool sel = true;
-#else
-    constexpr bool sel = false;
-#endif
-    if (sel) {
-        R a[5], b[5];
-        quick_weights(um1, u0, up1, s8, a);
-        central_weights(um2, um1, up1, up2, s12, b);
+    // float one).
+    R a[5], b[5];
+    quick_weights(um1, u0, up1, s8, a);
+    central_weights(um2, um1, up1, up2, s12, s12o, b);
 #pragma unroll
-        for (int m = 0; m < 5; m++) w[m] = quick ? a[m] : b[m];
-    } else if (quick) {
-        quick_weights(um1, u0, up1, s8, w);
-    } else {
-        central_weights(um2, um1, up1, up2, s12, w);
-    }
+    for (int m = 0; m < 5; m++) w[m] = quick ? a[m] : b[m];
 }
 
+// the first four terms of sum_m w[m] q[m], in the order of the offsets
+template <typename R>
+__device__ __forceinline__ R wsum4(const R w[5], R q0, R q1, R q2, R q3)
+{
+    return fmaR(w[3], q3, fmaR(w[2], q2, fmaR(w[0], q0, w[1] * q1)));
+}
 template <typename R>
 __device__ __forceinline__ R wsum(const R w[5], R q0, R q1, R q2, R q3, R q4)
 {
-    return (((w[0] * q0 + w[1] * q1) + w[2] * q2) + w[3] * q3) + w[4] * q4;
+    return fmaR(w[4], q4, wsum4(w, q0, q1, q2, q3));
 }
 
 // ---------------------------------------------------------------------------
@@ -220,35 +232,13 @@ struct SlotT {
     const R *U, *V, *W, *T;
 };
 
-// pressure at box point b.  With a pressure ring (PRING) PR is the ring's
-// pressure slot; without one PR is the density slot and p is rho*T/(gama*Ma^2)
-// formed on the spot (one multiply against two shared loads).  On interior
-// planes both give the same bits in FP64: the ring's p is formed by the same
-// two products of the same values.
-template <typename R, bool PRING = (sizeof(R) == 8)>
-__device__ __forceinline__ R pres_at(const FluxC<R> &C, const SlotT<R> &s, const R *PR, int b)
+// pressure at box point b, rho*T/(gama*Ma^2) from the density RHO of the Q ring
+// and T of the primitive ring (interior planes only)
+template <typename R>
+__device__ __forceinline__ R pres_at(const FluxC<R> &C, const SlotT<R> &s, const R *RHO, int b)
 {
-    if constexpr (!PRING) return (PR[b] * s.T[b]) * C.inv_gM2;
-    else return PR[b];
+    return (RHO[b] * s.T[b]) * C.inv_gM2;
 }
-
-// Single-rounding multiply-add in the ring type.  The viscous fluxes are
-// written with explicit FMAs so that every place that evaluates one (own
-// columns, halo lanes, the k-march prologue) rounds it the same way, and a
-// point's result does not depend on the launch shape that computed it.
-template <typename R>
-__device__ __forceinline__ R fmaR(R a, R b, R c);
-template <>
-__device__ __forceinline__ double fmaR<double>(double a, double b, double c) { return __fma_rn(a, b, c); }
-template <>
-__device__ __forceinline__ float fmaR<float>(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-// an add the compiler may not fuse with a product feeding it
-template <typename R>
-__device__ __forceinline__ R addR(R a, R b);
-template <>
-__device__ __forceinline__ double addR<double>(double a, double b) { return __dadd_rn(a, b); }
-template <>
-__device__ __forceinline__ float addR<float>(float a, float b) { return __fadd_rn(a, b); }
 
 // fD from the gradients at one point: [p + 2/3 mu/Re div - 2 mu/Re u_x,
 // -mu/Re (v_x+u_y), -mu/Re (w_x+u_z), -kq mu T_x + ggM (u fD2 + v fD3 + w fD4)]
@@ -288,9 +278,9 @@ __device__ __forceinline__ void gd_point(const FluxC<R> &C, R mu, R pr, R u0, R 
 // The flux helpers below take plane t's primitives from the ring slot s, plane
 // t+1's from sp, and plane t-1's values at point b as scalars (um, vm, wm),
 // which the caller keeps outside the ring.
-template <int BX, typename R, bool PRING = (sizeof(R) == 8)>
+template <int BX, typename R>
 __device__ __forceinline__ void visc_fx(const FluxC<R> &C, const SlotT<R> &s, R um, R wm, const SlotT<R> &sp,
-                                        const R *MU, const R *PR, int b, R czt, R f[4])
+                                        const R *MU, const R *RHO, int b, R czt, R f[4])
 {
     const R ux = (s.U[b + 1] - s.U[b - 1]) * C.hdx;
     const R uy = (s.U[b + BX] - s.U[b - BX]) * C.hdy;
@@ -300,12 +290,12 @@ __device__ __forceinline__ void visc_fx(const FluxC<R> &C, const SlotT<R> &s, R 
     const R Tx = (s.T[b + 1] - s.T[b - 1]) * C.hdx;
     const R uz = (sp.U[b] - um) * czt;
     const R wz = (sp.W[b] - wm) * czt;
-    fd_point(C, MU[b], pres_at<R, PRING>(C, s, PR, b), s.U[b], s.V[b], s.W[b], ux, vy, wz, vx, uy, wx, uz, Tx, f);
+    fd_point(C, MU[b], pres_at(C, s, RHO, b), s.U[b], s.V[b], s.W[b], ux, vy, wz, vx, uy, wx, uz, Tx, f);
 }
 
-template <int BX, typename R, bool PRING = (sizeof(R) == 8)>
+template <int BX, typename R>
 __device__ __forceinline__ void visc_fy(const FluxC<R> &C, const SlotT<R> &s, R vm, R wm, const SlotT<R> &sp,
-                                        const R *MU, const R *PR, int b, R czt, R g[4])
+                                        const R *MU, const R *RHO, int b, R czt, R g[4])
 {
     const R ux = (s.U[b + 1] - s.U[b - 1]) * C.hdx;
     const R uy = (s.U[b + BX] - s.U[b - BX]) * C.hdy;
@@ -315,30 +305,7 @@ __device__ __forceinline__ void visc_fy(const FluxC<R> &C, const SlotT<R> &s, R 
     const R Ty = (s.T[b + BX] - s.T[b - BX]) * C.hdy;
     const R vz = (sp.V[b] - vm) * czt;
     const R wz = (sp.W[b] - wm) * czt;
-    gd_point(C, MU[b], pres_at<R, PRING>(C, s, PR, b), s.U[b], s.V[b], s.W[b], ux, vy, wz, vx, uy, wy, vz, Ty, g);
-}
-
-// fD and gD together at one point: they share eight gradients, the shear
-// stress mu*(dv/dx+du/dy) (fD3 = gD2) and p + 2/3*mu*div.
-template <int BX, typename R, bool PRING = (sizeof(R) == 8)>
-__device__ __forceinline__ void visc_fxy(const FluxC<R> &C, const SlotT<R> &s, R um, R vm, R wm, const SlotT<R> &sp,
-                                         const R *MU, const R *PR, int b, R czt, R f[4], R g[4])
-{
-    const R ux = (s.U[b + 1] - s.U[b - 1]) * C.hdx;
-    const R uy = (s.U[b + BX] - s.U[b - BX]) * C.hdy;
-    const R vx = (s.V[b + 1] - s.V[b - 1]) * C.hdx;
-    const R vy = (s.V[b + BX] - s.V[b - BX]) * C.hdy;
-    const R wx = (s.W[b + 1] - s.W[b - 1]) * C.hdx;
-    const R wy = (s.W[b + BX] - s.W[b - BX]) * C.hdy;
-    const R Tx = (s.T[b + 1] - s.T[b - 1]) * C.hdx;
-    const R Ty = (s.T[b + BX] - s.T[b - BX]) * C.hdy;
-    const R uz = (sp.U[b] - um) * czt;
-    const R vz = (sp.V[b] - vm) * czt;
-    const R wz = (sp.W[b] - wm) * czt;
-    const R mu = MU[b], pr = pres_at<R, PRING>(C, s, PR, b);
-    const R u0 = s.U[b], v0 = s.V[b], w0 = s.W[b];
-    fd_point(C, mu, pr, u0, v0, w0, ux, vy, wz, vx, uy, wx, uz, Tx, f);
-    gd_point(C, mu, pr, u0, v0, w0, ux, vy, wz, vx, uy, wy, vz, Ty, g);
+    gd_point(C, MU[b], pres_at(C, s, RHO, b), s.U[b], s.V[b], s.W[b], ux, vy, wz, vx, uy, wy, vz, Ty, g);
 }
 
 template <typename R>
@@ -354,16 +321,6 @@ __device__ __forceinline__ void visc_fz_vals(const FluxC<R> &C, R ux, R vy, R wx
     h[1] = h3;
     h[2] = h4;
     h[3] = fmaR(C.ggM, fmaR(w, h4, fmaR(v, h3, u * h2)), -(kqm * Tz));
-}
-
-// hD at the thread's own column; z-derivatives supplied by the caller
-template <int BX, typename R>
-__device__ __forceinline__ void visc_fz(const FluxC<R> &C, const SlotT<R> &s, R mu, R pr, int b, R uz, R vz, R wz,
-                                        R Tz, R h[4])
-{
-    visc_fz_vals(C, (s.U[b + 1] - s.U[b - 1]) * C.hdx, (s.V[b + BX] - s.V[b - BX]) * C.hdy,
-                 (s.W[b + 1] - s.W[b - 1]) * C.hdx, (s.W[b + BX] - s.W[b - BX]) * C.hdy, s.U[b], s.V[b], s.W[b],
-                 mu, pr, uz, vz, wz, Tz, h);
 }
 
 // periodic image of index i in 0..n+1 (duplicate-point period n-2):
@@ -489,16 +446,19 @@ __device__ __forceinline__ void prims_from_q(const KParams &P, const double q[5]
 // The fused stage kernel.
 //
 // A CTA owns a TI x TJ tile of interior (i,j) columns and marches a chunk of
-// interior planes k = kb..ke.  Shared memory holds, for the tile plus a
-// 2-point halo box ((TI+4) x (TJ+4)):
+// interior planes k = kb..ke.  A thread owns two neighbouring x columns (i, i+1),
+// i even, so that every shared and global access of its own pair, of its y
+// neighbours and of its x stencil is an aligned 16-byte (FP64) or 8-byte (float)
+// one.  Shared memory holds, for the tile plus a 2-point halo box
+// ((TI+4) x (TJ+4)):
 //   Q (5 vars)      of planes t, t+1, t+2   (3-slot ring; t+2 in flight)
 //   prims u,v,w,T   of planes t, t+1        (2-slot ring)
-//   mu, p           of planes t, t+1        (2-slot ring; mu only with float rings)
+//   mu              of planes t, t+1        (2-slot ring; p is rho T / (gama Ma^2))
 //   fD, gD          of plane t on the tile plus a 1-point halo
-// Plane t-1 is kept where it is still read: each thread's own column (Q, u,
-// v, w) in registers, and the halo points of the halo-flux lanes in a small
-// shared array.  Each thread also keeps its own column's Q and w at t-2 and
-// hD at t-1, t, t+1 in registers.
+// Plane t-1 is kept where it is still read: each thread's own columns (Q, u,
+// v, w, T) in registers, and the halo points of the halo-flux lanes in a small
+// shared array.  Each thread also keeps its own columns' Q and w at t-2, hD at
+// t-1 and the unfinished sums of plane t-1 in registers.
 //
 // The Q box of each plane arrives by one tiled bulk tensor copy (TMA) issued
 // about two thirds of a plane ahead by one thread and completed on an mbarrier,
@@ -509,8 +469,8 @@ __device__ __forceinline__ void prims_from_q(const KParams &P, const double q[5]
 // in, float rings) loads its boxes with per-thread loads instead.
 //
 // A plane takes two CTA barriers: after the box conversion (with which the
-// inviscid x/y sums of the plane and the next own-column conversion share one
-// straight-line block) and after the viscous fluxes.  None ends the plane, so
+// inviscid x/y sums of the plane share one straight-line block) and after the
+// viscous fluxes.  None ends the plane, so
 // warps that finish the update early go on into the next plane's loads and
 // conversion while the others complete theirs.
 //
@@ -520,39 +480,26 @@ __device__ __forceinline__ void prims_from_q(const KParams &P, const double q[5]
 // intermediate stage states in float and evaluates the fluxes in float; the
 // primitive recovery (T from the total energy), the RK update against the
 // double base state, the forcing and the blow-up test stay in double.
-#ifndef CHAN_MINB
-#define CHAN_MINB 2   // resident 256-thread CTAs per SM the register budget is sized for (FP64 rings)
-#endif
-#ifndef CHAN_MINB_F
-#define CHAN_MINB_F 3 // the same with float rings (half the shared memory)
-#endif
+// constants of plane k: 0.5*invdXi*invJac; invdXi*invJac/8 (QUICK); the central
+// scheme's factor of the inner and of the outer pair, invdXi*invJac/12 both, but
+// next to a wall, where the scheme is the second-order (-w(k-1), 0, w(k+1)) * czh,
+// czh/8 and 0; Re*dXi*jac (the Peclet factor), -infinity next to a wall, so that the
+// switch never picks QUICK there.
+enum KTab { kCzh = 0, kS8 = 1, kS12 = 2, kS12o = 3, kPez = 4, kTabWords = 8 };
 
 template <int TI, int TJ, typename R>
 struct StageShape {
-    static constexpr int BX = TI + 4, BY = TJ + 4, NB = BX * BY, NT = TI * TJ;
-    // FP64 rings with 32-wide tiles: the own point's RK base arrives by a bulk
-    // copy of the tile (tma_base); the room for it comes from forming p from
-    // rho and T (no p ring) and exchanging fD along x by warp shuffles (a warp
-    // is a row of the tile), which leaves only the two halo columns in sF.
-#ifdef CHAN_TMA_BASE
-    static constexpr bool tma_base = sizeof(R) == 8 && TI == 32;
-#else
-    static constexpr bool tma_base = false;
-#endif
-    static constexpr bool fx_shfl = tma_base;
-    // where the own column of plane t+2 is read (measured per ring type: the FP64
-    // kernel 7% faster reading its Q twice than holding it in registers, whose
-    // spills it removes; the float kernels 2-3% faster loading it in phase C)
-#if defined(CHAN_EARLY_T2)
-    static constexpr bool late_t2 = false, late_qp2 = false;
-#else
-    static constexpr bool late_t2 = sizeof(R) == 4, late_qp2 = sizeof(R) == 8;
-#endif
-    static constexpr int NFX = fx_shfl ? 2 * TJ : TJ * (TI + 2), NGY = (TJ + 2) * TI;
-    // float rings keep mu only and form p from rho and T where it is used;
-    // FP64 rings keep (mu, p) unless the RK base takes the room
-    static constexpr bool p_ring = sizeof(R) == 8 && !tma_base;
-    static constexpr int MPW = p_ring ? 2 : 1;                       // words per box point in the (mu, p) ring
+    // NT threads of PX neighbouring x points each, TX per row of the tile.  Two points
+    // share their loads, addresses and loop overhead (32% fewer instructions), but
+    // need twice the registers: that pays in float (0.343 against 0.59 ms per launch at
+    // 256x193x192 with one point, in 80 registers); in FP64 two points of 255 registers
+    // leave two warps per scheduler and spill (0.715 against 0.502 ms).
+    static constexpr int PX = sizeof(R) == 4 ? 2 : 1;
+    static constexpr int BX = TI + 4, BY = TJ + 4, NB = BX * BY, TX = TI / PX, NT = TX * TJ;
+    // fD rows: [left halo, TI own points, right halo], padded so that own pairs are
+    // aligned; own points from FO on.  fD3 = gD2 is one array with both halos.
+    static constexpr int FO = PX, FP = TI + 2 * FO;
+    static constexpr int NFX = TJ * FP, NGY = (TJ + 2) * TI, NXY = (TJ + 2) * FP;
     // one Q slot: the 5-variable box of one plane, rounded up to 128 bytes
     // (the alignment of a bulk tensor copy's shared-memory destination)
     static constexpr size_t box_bytes = (size_t)5 * NB * sizeof(R);
@@ -560,24 +507,26 @@ struct StageShape {
     static constexpr int QSLOT = (int)(qslot_bytes / sizeof(R));     // slot stride in R elements
     static constexpr size_t q_bytes = 3 * qslot_bytes;
     static constexpr int pr_words = 2 * 4 * NB;
-    static constexpr int mp_words = 2 * MPW * NB;
-    static constexpr int fg_words = 4 * NFX + 4 * NGY;
-    // float rings leave room to stage the RK base of every thread's own point
-    // (double) by cp.async; the FP64 rings do not fit it beside two CTAs per SM
-    static constexpr bool prefetch_base = sizeof(R) == 4;
-    static constexpr bool base_slot = prefetch_base || tma_base;
-    // the base slot is a bulk-copy destination: 128-byte aligned
-    static constexpr size_t base_off = (q_bytes + sizeof(R) * (size_t)(pr_words + mp_words + fg_words) + 127) / 128 * 128;
-    // plane t-1 values (u or v, and w) of the halo-flux lanes' points, by lane
-    static constexpr int NHL = 32 + 2 * TI;
-    static constexpr size_t hl_off = base_off + (base_slot ? sizeof(double) * 5 * (size_t)NT : 0);
+    static constexpr int mu_words = 2 * NB;
+    static constexpr int fg_words = 3 * NFX + 3 * NGY + NXY;
+    // the tile's RK base of one plane (double), by bulk tensor copy: 128-byte aligned
+    static constexpr size_t base_off = (q_bytes + sizeof(R) * (size_t)(pr_words + mu_words + fg_words) + 127) / 128 * 128;
+    static constexpr size_t base_bytes = sizeof(double) * 5 * TI * TJ;
+    // per plane (4 slots): its constants (KTab) and 16 bytes of the forcing's density
+    static constexpr size_t tab_off = base_off + base_bytes;
+    static constexpr size_t tab_bytes = kTabWords * sizeof(R), rb_off = tab_off + 4 * tab_bytes;
+    // plane t-1 values (u or v, and w) of the halo-flux points: 2*TJ of the two
+    // x-halo columns, then 2*TI of the two y-halo rows
+    static constexpr int NHL = 2 * TJ + 2 * TI;
+    static constexpr size_t hl_off = rb_off + 4 * 16;
     static constexpr size_t bar_off = (hl_off + sizeof(R) * 2 * (size_t)NHL + 7) / 8 * 8;
-    static constexpr size_t bytes = bar_off + 4 * sizeof(unsigned long long) + 2 * sizeof(int);
-    // resident CTAs per SM the register budget is sized for: 128 (FP64) or 80
-    // (float) registers per thread at 256 threads, but never more CTAs than
-    // the 228 KB of shared memory per SM holds (1 KB of it reserved per CTA)
-    static constexpr int minb_regs = (sizeof(R) == 4 ? CHAN_MINB_F : CHAN_MINB) * 256 / NT;
+    static constexpr size_t bytes = bar_off + 5 * sizeof(unsigned long long) + 2 * sizeof(int);
+    // resident CTAs per SM the register budget is sized for: as many as the
+    // 228 KB of shared memory per SM hold (1 KB of it reserved per CTA), and
+    // never fewer registers than a thread needs for its two points (MINR)
+    static constexpr int MINR = PX == 2 ? (sizeof(R) == 4 ? 128 : 224) : (sizeof(R) == 4 ? 80 : 128);
     static constexpr int minb_smem = (int)(233472 / (bytes + 1024));
+    static constexpr int minb_regs = 65536 / (MINR * NT);
     static constexpr int minb = minb_regs < minb_smem ? minb_regs : minb_smem;
 };
 
@@ -587,20 +536,6 @@ template <>
 __device__ __forceinline__ const FluxC<double> &fluxc<double>(const KParams &P) { return P.cd; }
 template <>
 __device__ __forceinline__ const FluxC<float> &fluxc<float>(const KParams &P) { return P.cf; }
-
-// per-k tables: 0 czh, 1 cz8, 2 cz12, 3 pez
-template <typename R>
-__device__ __forceinline__ R ktab(const KParams &P, int which, int k);
-template <>
-__device__ __forceinline__ double ktab<double>(const KParams &P, int which, int k)
-{
-    return which == 0 ? P.czh[k] : (which == 1 ? P.cz8[k] : (which == 2 ? P.cz12[k] : P.pez[k]));
-}
-template <>
-__device__ __forceinline__ float ktab<float>(const KParams &P, int which, int k)
-{
-    return P.tabf[which * (P.n3 + 2) + k];
-}
 
 // mu = T^0.7 in the ring type: pow07 in double; exp2(0.7 log2 T) in float
 template <typename R>
@@ -612,24 +547,64 @@ __device__ __forceinline__ float mu_of<float>(double T)
 {
     // the hardware log2 and exp2 approximations (relative error about 2^-21, well
     // inside the float path's own rounding); the library log2f/exp2f cost 2.5% of
-    // the float stage kernel (CHAN_LIBM_MU_F)
-#ifndef CHAN_LIBM_MU_F
+    // the float stage kernel
     return seed_exp2(0.7f * seed_log2((float)T));
-#else
-    return exp2f(0.7f * log2f((float)T));
-#endif
 }
 
-// a load of state written earlier in the same launch by other CTAs (the
-// persistent ensemble kernel) must not use the read-only path
-template <bool COHERENT, typename T>
-__device__ __forceinline__ double ldq_c(const T *p) { return COHERENT ? (double)*p : (double)__ldg(p); }
+// PX neighbouring elements in one access (the address is a multiple of its size)
+template <typename T>
+struct Pair;
+template <>
+struct Pair<double> { using V = double2; };
+template <>
+struct Pair<float> { using V = float2; };
+template <int PX, typename T, typename R>
+__device__ __forceinline__ void ldp(const T *p, R out[PX])
+{
+    if constexpr (PX == 2) {
+        const typename Pair<T>::V v = *reinterpret_cast<const typename Pair<T>::V *>(p);
+        out[0] = (R)v.x;
+        out[1] = (R)v.y;
+    } else {
+        out[0] = (R)*p;
+    }
+}
+template <int PX, typename T, typename R>
+__device__ __forceinline__ void stp(T *p, const R in[PX])
+{
+    if constexpr (PX == 2) {
+        typename Pair<T>::V v;
+        v.x = (T)in[0];
+        v.y = (T)in[1];
+        *reinterpret_cast<typename Pair<T>::V *>(p) = v;
+    } else {
+        *p = (T)in[0];
+    }
+}
+// the same from global memory, as doubles.  State written earlier in the same
+// launch by other CTAs (the persistent ensemble kernel, COHERENT) must not use
+// the read-only path.
+template <int PX, bool COHERENT, typename T>
+__device__ __forceinline__ void ldgp(const T *p, double out[PX])
+{
+    if constexpr (PX == 2) {
+        const auto *q = reinterpret_cast<const typename Pair<T>::V *>(p);
+        const typename Pair<T>::V v = COHERENT ? *q : __ldg(q);
+        out[0] = (double)v.x;
+        out[1] = (double)v.y;
+    } else {
+        out[0] = COHERENT ? (double)*p : (double)__ldg(p);
+    }
+}
 
-// 8-byte asynchronous global->shared copy (no register staging)
-__device__ __forceinline__ void cp_async8(double *dst, const double *src)
+
+// asynchronous global->shared copy of PX doubles (no register staging)
+template <int PX>
+__device__ __forceinline__ void cp_async_d(double *dst, const double *src)
 {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+    if constexpr (PX == 2) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -647,13 +622,26 @@ __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier
 // visible to this thread by a CTA barrier) before its later async-proxy writes
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// the 4-D box at (x, y, z, w) of the tensor map into dst; bytes = box size.
-// No multicast: the box lands in this CTA's shared memory only.
+// one arrival on the barrier, which then waits for `bytes` of copies
+__device__ __forceinline__ void mbar_expect(unsigned long long *bar, unsigned bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32addr(bar)), "r"(bytes)
+                 : "memory");
+}
+// `bytes` (a multiple of 16) from global memory at src (16-byte aligned) into dst
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes, unsigned long long *bar)
+{
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32addr(dst)),
+        "l"(src), "r"(bytes), "r"(smem_u32addr(bar))
+        : "memory");
+}
+// the 4-D box at (x, y, z, w) of the tensor map into dst.  No multicast: the box
+// lands in this CTA's shared memory only.
 __device__ __forceinline__ void tma_load_box(void *dst, const CUtensorMap *map, int x, int y, int z, int w,
-                                             unsigned long long *bar, unsigned bytes)
+                                             unsigned long long *bar)
 {
     const unsigned b = smem_u32addr(bar);
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
         "%5}], [%6];" ::"r"(smem_u32addr(dst)),
@@ -700,30 +688,33 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long *bar, unsig
 // was written earlier in the same launch: coherent loads instead of the
 // read-only path, and a proxy fence before the first box copy.
 template <int TI, int TJ, typename QI, typename QO, typename R, int BUOYM, bool PERSIST>
-__device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *tmq, const CUtensorMap *tmb, int bx,
-                                           int by, int bz, int tx, int ty, unsigned char *smem_raw)
+__device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *tmq, const CUtensorMap *tmb, int bx, int by,
+                                           int bz, int tx, int ty, unsigned char *smem_raw)
 {
     using S = StageShape<TI, TJ, R>;
     using Slot = SlotT<R>;
-    constexpr bool late_t2 = S::late_t2, late_qp2 = S::late_qp2;
-    constexpr int BX = S::BX, BY = S::BY, NB = S::NB, NT = S::NT, MPW = S::MPW, QSLOT = S::QSLOT;
+    constexpr int BX = S::BX, NB = S::NB, NT = S::NT, QSLOT = S::QSLOT, FP = S::FP, PX = S::PX;
+    constexpr int FO = S::FO, NHL = S::NHL;
+    // FP64: the wall-normal terms are folded into the carried sum as they come;
+    // the float kernels keep the order of the one-pass sum
+    constexpr bool FOLD = sizeof(R) == 8;
     // boxes by bulk tensor copy when the input is stored in the ring type
-#ifdef CHAN_NO_TMA
-    constexpr bool TMA = false;   // measurement variant: per-thread box loads into the same ring
-#else
     constexpr bool TMA = std::is_same<QI, R>::value;
-#endif
-    static_assert(2 * TJ <= 32 && 32 + 2 * TI <= NT, "halo-flux lane layout needs 2*TJ <= 32 and 32+2*TI <= TI*TJ");
+    static_assert(TI % PX == 0 && 2 * TJ <= 32 && NT >= 32, "tile layout");
     R *sQ = reinterpret_cast<R *>(smem_raw);                       // [3 slots][5][NB]
     R *sPr = reinterpret_cast<R *>(smem_raw + S::q_bytes);         // [2][4][NB] u,v,w,T
-    R *sMP = sPr + S::pr_words;                                    // [2][MPW][NB] mu (, p)
-    R *sF = sMP + S::mp_words;                                     // [4][TJ][TI+2]
-    R *sG = sF + 4 * S::NFX;                                       // [4][TJ+2][TI]
-    double *sQB = reinterpret_cast<double *>(smem_raw + S::base_off);   // [5][NT] (float rings only)
+    R *sMU = sPr + S::pr_words;                                    // [2][NB] mu
+    R *sF = sMU + S::mu_words;                                     // fD2, fD4, fD5 [3][TJ][FP], own points from FO on
+    R *sG = sF + 3 * S::NFX;                                       // gD3, gD4, gD5 [3][TJ+2][TI]
+    R *sX = sG + 3 * S::NGY;                                       // fD3 = gD2 [TJ+2][FP]
+    double *sQB = reinterpret_cast<double *>(smem_raw + S::base_off);   // [5][TJ][TI]
+    R *sT = reinterpret_cast<R *>(smem_raw + S::tab_off);               // [4][kTabWords]
+    double *sRB = reinterpret_cast<double *>(smem_raw + S::rb_off);     // [4][2]
     R *sH = reinterpret_cast<R *>(smem_raw + S::hl_off);                // [2][NHL]
     // (the 8-byte rounding is a no-op: bar_off is a multiple of 8)
-    unsigned long long *bar = reinterpret_cast<unsigned long long *>(reinterpret_cast<size_t>(smem_raw + S::bar_off) & ~(size_t)7);   // [3]
-    int *sflag = reinterpret_cast<int *>(bar + 4);   // [0] the CTA leaves at once, [1] slots with a copy in flight
+    unsigned long long *bar = reinterpret_cast<unsigned long long *>(reinterpret_cast<size_t>(smem_raw + S::bar_off) & ~(size_t)7);   // [4]: Q slots, RK base
+    double *stau = reinterpret_cast<double *>(bar + 4);   // tauL - tauU
+    int *sflag = reinterpret_cast<int *>(bar + 5);   // [0] the CTA leaves at once, [1] copies in flight
     const FluxC<R> &C = fluxc<R>(P);
     // the state pointers are read from the parameter space at each use: held
     // in registers across the kernel they cost spills
@@ -731,21 +722,20 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
     auto qout = [&]() { return static_cast<QO *>(P.qout); };
 
     const bool buoy = BUOYM == 2 ? P.buoy_on != 0 : BUOYM == 1;
-    const int tid = ty * TI + tx;
+    const int tid = ty * S::TX + tx;
     if (tid == 0) {
         sflag[0] = frozen(P.status, kstep(P)) ? 1 : 0;
         sflag[1] = 0;
         // state written by other CTAs of this launch, read next by box copies
         if (PERSIST) asm volatile("fence.proxy.async.global;" ::: "memory");
         // a bulk copy needs a 128-byte aligned destination
-        if (TMA && (smem_u32addr(smem_raw) & 127u)) {
+        if (smem_u32addr(smem_raw) & 127u) {
             sflag[0] = 1;
             atomicExch(&P.status->stall, 2);
         }
-        if (TMA || S::tma_base) {
-            for (int s = 0; s < 4; s++) mbar_init_one(&bar[s]);
-            fence_mbar_init();
-        }
+        for (int s = 0; s < 4; s++) mbar_init_one(&bar[s]);
+        fence_mbar_init();
+        *stau = P.stat[23 * P.n3 + 0] - P.stat[23 * P.n3 + 1];
     }
     __syncthreads();
     if (sflag[0]) return;
@@ -755,38 +745,61 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
     const int ke = min(kb + P.kchunk - 1, P.n3 - 1);
     if (kb > ke) return;
     const int n1 = P.n1, n2 = P.n2, n3 = P.n3;
-    const int i = i0 + tx, j = j0 + ty;
+    const int i = i0 + PX * tx, j = j0 + ty;
+    // the pair is loaded and its fluxes formed when its first point is a stored
+    // one: the row pitch px >= nP1+2 is even, so the pair lies inside the row
     const bool col_ok = (i <= n1) && (j <= n2);
-    const bool out_ok = (i <= n1 - 1) && (j <= n2 - 1);
-    const int bc = (ty + 2) * BX + (tx + 2);
+    const bool out0 = (i <= n1 - 1) && (j <= n2 - 1), out1 = (i + PX - 1 <= n1 - 1) && (j <= n2 - 1);
+    const int bc = (ty + 2) * BX + PX * tx + 2;
+    // offset of the own points' periodic image in x (0: none; the points of a pair that
+    // have one have the same)
+    const int xim = i <= 3 ? n1 - 2 : (i + PX - 1 >= n1 - 2 ? 2 - n1 : 0);
     const long long vol = P.vol, plane = P.plane;
     const long long colo = (long long)j * P.px + i;
 
     // ring slots by role, rotated once per plane: Q slots (indices 0..2) of
-    // planes t, t+1, t+2; prims offsets of t, t+1; (mu,p) offsets of t, t+1
+    // planes t, t+1, t+2; prims offsets of t, t+1; mu offsets of t, t+1
     int iZ = 1, iP = 2, iN = 0;
-    int pZ = 0, pP = 4 * NB, mZ = 0, mP = MPW * NB;
-    unsigned ph = 0u;   // parity of the next wait, per Q slot
+    int pZ = 0, pP = 4 * NB, mZ = 0, mP = NB;
+    unsigned ph = 0u;   // parity of the next wait, per barrier
     auto slot = [&](int o) -> Slot {
         return Slot{sPr + o, sPr + o + NB, sPr + o + 2 * NB, sPr + o + 3 * NB};
     };
-    auto smu = [&](int o) { return sMP + o; };
+    auto smu = [&](int o) { return sMU + o; };
     auto sq = [&](int s, int v) { return sQ + s * QSLOT + v * NB; };
-    // what the flux helpers read the pressure from (pres_at): the p slot of
-    // the (mu,p) ring at mo, or the density of the Q slot s
-    auto spr = [&](int mo, int s) { return S::p_ring ? sMP + mo + NB : sq(s, 0); };
+    // plane k's constants and forcing density, staged with its box
+    auto ktab = [&](int which, int k) { return sT[(k & 3) * kTabWords + which]; };
+    auto rbar = [&](int k) { return sRB[(k & 3) * 2 + ((k - 1) & 1)]; };
 
-    // plane m's Q box into Q slot s (one thread; bulk tensor copy)
+    // plane m's Q box into Q slot s, with the plane's constants and forcing density
+    // (one thread; bulk copies).  Everything a plane reads per thread then comes from
+    // shared memory: as plain loads, L1 hits most of them, the constants, the density
+    // and the RK base below held up the warps for 18% of the FP64 stage time.
     auto issue = [&](int m, int s) {
-        if (TMA && tid == 0) {
+        if (tid == 0) {
             fence_proxy_async_smem();
-            tma_load_box(sq(s, 0), tmq, i0 - 2, j0 - 2, m, 0, &bar[s], (unsigned)S::box_bytes);
+            mbar_expect(&bar[s], (unsigned)((TMA ? S::box_bytes : 0) + S::tab_bytes + 16));
+            if (TMA) tma_load_box(sq(s, 0), tmq, i0 - 2, j0 - 2, m, 0, &bar[s]);
+            bulk_load(sT + (m & 3) * kTabWords, static_cast<const R *>(P.ktab) + (size_t)m * kTabWords,
+                      (unsigned)S::tab_bytes, &bar[s]);
+            bulk_load(sRB + (m & 3) * 2, P.stat + ((m - 1) & ~1), 16u, &bar[s]);
             sflag[1] |= 1 << s;
         }
     };
-    // wait for Q slot s; false if the copy did not complete in time
+    // the mixed path's first stage never has a base, its others always do
+    const bool need_base = FOLD ? P.rk_mode != 0 : TMA;
+    constexpr bool CHK = std::is_same<QO, double>::value;   // a step's last stage may be this kernel
+    // FP64: the tile's RK base of plane m into its slot (barrier 3)
+    auto issue_base = [&](int m) {
+        if (FOLD && need_base && tid == 0) {
+            fence_proxy_async_smem();
+            mbar_expect(&bar[3], (unsigned)S::base_bytes);
+            tma_load_box(sQB, tmb, i0, j0, m, 0, &bar[3]);
+            sflag[1] |= 1 << 3;
+        }
+    };
+    // wait for barrier s; false if its copies did not complete in time
     auto wait_slot = [&](int s) -> bool {
-        if (s < 3 ? !TMA : !S::tma_base) return true;
         const bool ok = mbar_wait_bounded(&bar[s], (ph >> s) & 1u);
         ph ^= 1u << s;
         if (ok && tid == 0) sflag[1] &= ~(1 << s);
@@ -801,30 +814,38 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
                 if (sflag[1] & (1 << s)) mbar_wait_bounded(&bar[s], (ph >> s) & 1u);
         }
     };
-    // the tile's RK base of plane m into the base slot (barrier 3)
-    auto issue_base = [&](int m) {
-        if (S::tma_base && tid == 0) {
-            fence_proxy_async_smem();
-            tma_load_box(sQB, tmb, i0, j0, m, 0, &bar[3], (unsigned)(sizeof(double) * 5 * NT));
-            sflag[1] |= 1 << 3;
-        }
-    };
 
-    // box points this thread converts: the same columns for every plane
-    // lp: box index | 0x10000 if the point is in R1 (tile plus a 1-point cross
-    // halo, where mu and p are needed); -1 if outside the array.  lo: column offset.
-    constexpr int NL = (NB + NT - 1) / NT;
+
+    // own columns, carried from plane to plane: Q at t-1 and t-2, u, v, w, T at
+    // t-1, w at t-2, hD at t-1; and what is known of plane t-1's update, which only
+    // lacks what plane t+1 brings: Fs (FP64: the RK increment on Q; float rings: the
+    // flux derivatives in x and y), its wall-normal switch (qk) and the QUICK weight of
+    // Q(t+1) (w4).  Float rings add the wall-normal terms in the order of the one-pass
+    // sum and carry them apart (H1p: that sum but its last term, hm: hD(t-2)).
+    R qm2[5][PX], qm1[5][PX], Fs[PX][5], h1[PX][4], hm[PX][4], H1p[PX][5], w4[PX];
+    R wm2[PX], um1[PX], vm1[PX], wm1[PX], Tm1[PX];
+    bool qk[PX] = {}, qz[PX] = {};   // the wall-normal switch of planes t-1 and t
+#pragma unroll
+    for (int a = 0; a < PX; a++) {
+#pragma unroll
+        for (int c = 0; c < 5; c++) qm2[c][a] = qm1[c][a] = Fs[a][c] = H1p[a][c] = R(0);
+#pragma unroll
+        for (int c = 0; c < 4; c++) h1[a][c] = hm[a][c] = R(0);
+        wm2[a] = um1[a] = vm1[a] = wm1[a] = Tm1[a] = w4[a] = R(0);
+    }
+    // box pairs this thread converts: the same columns for every plane
+    // lp: box index of the pair's first point, -1 if that is outside the array
+    // (its second point may be one past the array: converted from the copy's zero
+    // fill or from the row's padding, stored, and read by no one).  lo: column offset.
+    constexpr int NL = (NB / PX + NT - 1) / NT;
     int lp[NL];
     int lo[NL];
 #pragma unroll
     for (int l = 0; l < NL; l++) {
-        const int p = tid + l * NT;
+        const int p = PX * (tid + l * NT);
         const int bj = p / BX, bi = p - bj * BX;
         const int gi = i0 - 2 + bi, gj = j0 - 2 + bj;
-        const bool ok = p < NB && gi <= n1 + 1 && gj <= n2 + 1;
-        const bool r1 = (bi >= 1 && bi <= BX - 2 && bj >= 2 && bj <= BY - 3) ||
-                        (bi >= 2 && bi <= BX - 3 && bj >= 1 && bj <= BY - 2);
-        lp[l] = ok ? (p | (r1 ? 0x10000 : 0)) : -1;
+        lp[l] = p < NB && gi <= n1 + 1 && gj <= n2 + 1 ? p : -1;
         lo[l] = gj * P.px + gi;
     }
 
@@ -832,102 +853,153 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
     // t's Q box and u, v, which the previous plane converted: they are formed in
     // phase A, in the same straight-line block as the conversion of plane t+1's
     // box, whose dependency chains (reciprocal, power) they fill (1.7% of the
-    // FP64 stage time, 2.4% of the float one, against forming them in phase E;
-    // in phase C, beside the viscous fluxes, they were 2.8% slower than in E).
-    // CHAN_XY_IN_E keeps them in phase E, for measurement.
-#ifdef CHAN_XY_IN_E
-    constexpr bool xy_a = false;
-#else
-    constexpr bool xy_a = true;
-#endif
-    R Fxy[5] = {0, 0, 0, 0, 0};
-    auto inv_xy = [&]() {
-        const R mu0 = smu(mZ)[bc];
-        const R *U = sPr + pZ, *V = sPr + pZ + NB;
-        const bool qx = (C.pex * fabs(sq(iZ, 1)[bc])) > C.PexVal * mu0;
-        const bool qy = (C.pey * fabs(sq(iZ, 2)[bc])) > C.PeyVal * mu0;
-        R wx[5], wy[5];
-        inv_weights(U[bc - 2], U[bc - 1], U[bc], U[bc + 1], U[bc + 2], qx, C.sx8, C.sx12, wx);
-        inv_weights(V[bc - 2 * BX], V[bc - BX], V[bc], V[bc + BX], V[bc + 2 * BX], qy, C.sy8, C.sy12, wy);
+    // FP64 stage time, 2.4% of the float one, against forming them in phase E).
+    // a row of the x stencil: PX + 4 values around the own points
+    auto row = [&](const R *f, R x[PX + 4]) {
+        if constexpr (PX == 2) {
+            ldp<2>(f - 2, x);
+            ldp<2>(f, x + 2);
+            ldp<2>(f + 2, x + 4);
+        } else {
 #pragma unroll
-        for (int c = 0; c < 5; c++) {
-            const R *Q = sq(iZ, c);
-            Fxy[c] = wsum(wx, Q[bc - 2], Q[bc - 1], Q[bc], Q[bc + 1], Q[bc + 2]) +
-                     wsum(wy, Q[bc - 2 * BX], Q[bc - BX], Q[bc], Q[bc + BX], Q[bc + 2 * BX]);
+            for (int m = 0; m < 5; m++) x[m] = f[m - 2];
+        }
+    };
+    // FP64: what it leaves is W = a*(Qbase - Q) - cdt*(F1 + G1 + the wall-normal terms
+    // of Q(t-2) and hD(t-1)), the part known so far of the RK update's increment on Q
+    // (a*Qbase + b*Q = Q + a*(Qbase - Q) + eps*Q, eps = a + b - 1 the rounding of a and
+    // b; the increment is small beside Q, so only its addition rounds at Q's size).  The base is thus read
+    // here and not carried, and Q(t-2), hD(t-1) and w(t-2) end here, before the viscous
+    // fluxes, where most values are live.
+    auto inv_xy = [&](int t, R Fxy[PX][5]) {
+        R mu0[PX], m0[PX], w[PX][5];
+        const R *U = sPr + pZ + bc, *V = sPr + pZ + NB + bc;
+        ldp<PX>(smu(mZ) + bc, mu0);
+        {
+            R x[PX + 4];
+            row(U, x);
+            ldp<PX>(sq(iZ, 1) + bc, m0);
+#pragma unroll
+            for (int a = 0; a < PX; a++) {
+                const bool q = (C.pex * fabs(m0[a])) > C.PexVal * mu0[a];
+                inv_weights(x[a], x[a + 1], x[a + 2], x[a + 3], x[a + 4], q, C.sx8, C.sx12, C.sx12, w[a]);
+            }
+#pragma unroll
+            for (int c = 0; c < 5; c++) {
+                row(sq(iZ, c) + bc, x);
+#pragma unroll
+                for (int a = 0; a < PX; a++) Fxy[a][c] = wsum(w[a], x[a], x[a + 1], x[a + 2], x[a + 3], x[a + 4]);
+            }
+        }
+        {
+            R y[5][PX];
+#pragma unroll
+            for (int m = 0; m < 5; m++) ldp<PX>(V + (m - 2) * BX, y[m]);
+            ldp<PX>(sq(iZ, 2) + bc, m0);
+            R wz[PX], cz = R(0);
+            if constexpr (FOLD) {
+                R w0[PX], m3[PX];
+                ldp<PX>(sPr + pZ + 2 * NB + bc, w0);
+                ldp<PX>(sq(iZ, 3) + bc, m3);
+                const R pez = ktab(kPez, t), s8 = ktab(kS8, t), s12o = ktab(kS12o, t);
+                cz = ktab(kCzh, t);
+#pragma unroll
+                for (int a = 0; a < PX; a++) {
+                    qz[a] = (pez * fabs(m3[a])) > C.pez_val * mu0[a];
+                    const R r2 = ((w0[a] + wm1[a]) * R(0.5)) * s8;   // weight of Q(t-2), as inv_weights has it
+                    wz[a] = qz[a] ? (r2 >= R(0) ? r2 : R(0)) : wm2[a] * s12o;
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < PX; a++) {
+                const bool q = (C.pey * fabs(m0[a])) > C.PeyVal * mu0[a];
+                inv_weights(y[0][a], y[1][a], y[2][a], y[3][a], y[4][a], q, C.sy8, C.sy12, C.sy12, w[a]);
+            }
+#pragma unroll
+            for (int c = 0; c < 5; c++) {
+                const R *Q = sq(iZ, c) + bc;
+#pragma unroll
+                for (int m = 0; m < 5; m++) ldp<PX>(Q + (m - 2) * BX, y[m]);
+#pragma unroll
+                for (int a = 0; a < PX; a++)
+                    Fxy[a][c] = Fxy[a][c] + wsum(w[a], y[0][a], y[1][a], y[2][a], y[3][a], y[4][a]);
+                if constexpr (FOLD) {
+                    R qb[PX];
+#pragma unroll
+                    for (int a = 0; a < PX; a++) {
+                        qb[a] = y[2][a];
+                        Fxy[a][c] = fmaR(wz[a], qm2[c][a], Fxy[a][c]);
+                        if (c > 0) Fxy[a][c] = fmaR(-h1[a][c > 0 ? c - 1 : 0], cz, Fxy[a][c]);
+                    }
+                    if (need_base) ldp<PX>(sQB + (c * TJ + ty) * TI + PX * tx, qb);
+#pragma unroll
+                    for (int a = 0; a < PX; a++)
+                        Fxy[a][c] = fmaR(-(R)P.rk_cdt, Fxy[a][c], fmaR((R)P.rk_eps, y[2][a], (R)P.rk_a * (qb[a] - y[2][a])));
+                }
+            }
         }
     };
 
-    // primitives (and mu, p on R1) of plane m over the box, from its Q box in
-    // slot s (with per-thread loads, Q is first loaded into the slot).  A wall
-    // plane's box holds, at periodic duplicates and ghosts, the values of their
-    // image points: the viscous fluxes next to a wall read the wall only there,
-    // and the reference's flux at a duplicate column or row is the exchanged
-    // flux of its image (whose wall values may differ from the duplicate's own
-    // under a non-periodic wall BC).  hD on a wall plane reads the wall's own
-    // values from memory instead (hflux_wall).
-    auto no_extra = []() {};
-    // FP64 rings: mu (and p) formed and stored at every box point, not only on R1,
-    // where they are read (the other cells of the slot are never read): the
-    // conversion's block then has no branch on R1, and the 1.31 -> 1.69 powers per
-    // output cost less than the divergent branch did (2.9% of the FP64 stage time;
-    // the float kernels, whose float mu is cheap, are 0.9% slower with it).
-    // CHAN_MU_R1 keeps the branch, for measurement.
-#ifdef CHAN_MU_R1
-    constexpr bool mu_all = false;
-#else
-    constexpr bool mu_all = sizeof(R) == 8;
-#endif
-    auto convert = [&](int m, int s, int po, int mo, bool with_xy, auto &&extra) {
+    // primitives, mu and p of plane m over the box, from its Q box in slot s (with
+    // per-thread loads, Q is first loaded into the slot).  A wall plane's box
+    // holds, at periodic duplicates and ghosts, the values of their image points:
+    // the viscous fluxes next to a wall read the wall only there, and the
+    // reference's flux at a duplicate column or row is the exchanged flux of its
+    // image (whose wall values may differ from the duplicate's own under a
+    // non-periodic wall BC).  hD on a wall plane reads the wall's own values from
+    // memory instead (hflux_wall).
+    auto convert = [&](int m, int s, int po, int mo, bool with_xy, R (*Fxy)[PX][5] = nullptr) {
         const Slot sl = slot(po);
-        R *MU = smu(mo), *PR = sMP + mo + NB;
+        R *MU = smu(mo);
         const bool wall = (m == 1 || m == n3);
         const double *W = P.wp + (size_t)(m == 1 ? 0 : 8) * plane;
         auto one = [&](int l, bool wall_plane) {
             if (lp[l] < 0) return;
-            const int p = lp[l] & 0xffff;
-            const bool r1 = (lp[l] & 0x10000) != 0;
-            double q[5];
+            const int p = lp[l];
+            double q[5][PX];
             if (!TMA) {
                 const long long off = (long long)m * plane + lo[l];
 #pragma unroll
                 for (int v = 0; v < 5; v++) {
-                    q[v] = ldq_c<PERSIST>(qin() + v * vol + off);
-                    sq(s, v)[p] = (R)q[v];
+                    ldgp<PX, PERSIST>(qin() + v * vol + off, q[v]);
+                    stp<PX>(sq(s, v) + p, q[v]);
                 }
             }
-            double u, vv, w, T, pr;
-            R mu;
+            double u[PX], vv[PX], w[PX], T[PX];
+            R mu[PX];
             if (wall_plane) {
                 const int bj = p / BX, bi = p - bj * BX;
-                const long long wo = (long long)wrap_idx(j0 - 2 + bj, n2) * P.px + wrap_idx(i0 - 2 + bi, n1);
-                u = W[1 * plane + wo];
-                vv = W[2 * plane + wo];
-                w = W[3 * plane + wo];
-                T = W[5 * plane + wo];
-                pr = W[6 * plane + wo];
-                mu = (R)W[7 * plane + wo];
+                const long long wj = (long long)wrap_idx(j0 - 2 + bj, n2) * P.px;
+#pragma unroll
+                for (int a = 0; a < PX; a++) {
+                    const long long wo = wj + wrap_idx(min(i0 - 2 + bi + a, n1 + 1), n1);
+                    u[a] = W[1 * plane + wo];
+                    vv[a] = W[2 * plane + wo];
+                    w[a] = W[3 * plane + wo];
+                    T[a] = W[5 * plane + wo];
+                    mu[a] = (R)W[7 * plane + wo];
+                }
             } else {
                 if (TMA) {
 #pragma unroll
-                    for (int v = 0; v < 5; v++) q[v] = (double)sq(s, v)[p];
+                    for (int v = 0; v < 5; v++) ldp<PX>(sq(s, v) + p, q[v]);
                 }
-                prims_from_q(P, q, u, vv, w, T);
-                pr = (q[0] * T) * P.inv_gM2;
-                mu = mu_all ? mu_of<R>(T) : (r1 ? mu_of<R>(T) : R(0));
+#pragma unroll
+                for (int a = 0; a < PX; a++) {
+                    const double qa[5] = {q[0][a], q[1][a], q[2][a], q[3][a], q[4][a]};
+                    prims_from_q(P, qa, u[a], vv[a], w[a], T[a]);
+                    mu[a] = mu_of<R>(T[a]);
+                }
             }
-            ((R *)sl.U)[p] = (R)u;
-            ((R *)sl.V)[p] = (R)vv;
-            ((R *)sl.W)[p] = (R)w;
-            ((R *)sl.T)[p] = (R)T;
-            if (mu_all || r1) {
-                MU[p] = mu;
-                if (S::p_ring) PR[p] = (R)pr;
-            }
+            stp<PX>((R *)sl.U + p, u);
+            stp<PX>((R *)sl.V + p, vv);
+            stp<PX>((R *)sl.W + p, w);
+            stp<PX>((R *)sl.T + p, T);
+            stp<PX>(MU + p, mu);
         };
         // the wall test taken once per plane, so that each loop's body is
-        // straight-line code (2.6% of the FP64 stage time against one loop with the
-        // test inside); the per-thread box loads one box point at a time, with fewer
-        // loads in flight (0.4% of the mean float stage time)
+        // straight-line code; the per-thread box loads one pair at a time, with
+        // fewer loads in flight
         auto loop = [&](bool wall_plane) {
             if (!TMA) {
 #pragma unroll 1
@@ -936,40 +1008,87 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
 #pragma unroll
                 for (int l = 0; l < NL; l++) one(l, wall_plane);
             }
-            if (xy_a && with_xy) inv_xy();
-            extra();
+            if (with_xy) inv_xy(m - 1, *Fxy);
         };
         if (wall) loop(true);
         else loop(false);
     };
 
-    // own-column Q and u,v,w,T of plane m read straight from memory
-    auto center = [&](int m, double q[5], double &u, double &v, double &w, double &T) {
+    // own columns' Q and u,v,w,T of plane m read straight from memory
+    auto center = [&](int m, double q[5][PX], double u[PX], double v[PX], double w[PX], double T[PX]) {
         const long long off = (long long)m * plane + colo;
 #pragma unroll
-        for (int c = 0; c < 5; c++) q[c] = ldq_c<PERSIST>(qin() + c * vol + off);
+        for (int c = 0; c < 5; c++) ldgp<PX, PERSIST>(qin() + c * vol + off, q[c]);
         if (m == 1 || m == n3) {
             const double *W = P.wp + (size_t)(m == 1 ? 0 : 8) * plane + colo;
-            u = W[1 * plane]; v = W[2 * plane]; w = W[3 * plane]; T = W[5 * plane];
+            ldgp<PX, true>(W + 1 * plane, u);
+            ldgp<PX, true>(W + 2 * plane, v);
+            ldgp<PX, true>(W + 3 * plane, w);
+            ldgp<PX, true>(W + 5 * plane, T);
         } else {
-            prims_from_q(P, q, u, v, w, T);
+#pragma unroll
+            for (int a = 0; a < PX; a++) {
+                const double qa[5] = {q[0][a], q[1][a], q[2][a], q[3][a], q[4][a]};
+                prims_from_q(P, qa, u[a], v[a], w[a], T[a]);
+            }
         }
     };
 
-    // hD at the own column of interior plane m (prims at po, (mu,p) at mo, Q
-    // slot s); dz from (m-1, m+1) values
-    auto hflux = [&](int m, int po, int mo, int s, R um, R vm, R wm, R Tm, R up, R vp, R wp_, R Tp, R h[4]) {
-        const Slot sl = slot(po);
-        const R sc = ktab<R>(P, 0, m);
-        visc_fz<BX>(C, sl, smu(mo)[bc], pres_at<R, S::p_ring>(C, sl, spr(mo, s), bc), bc, (up - um) * sc, (vp - vm) * sc,
-                    (wp_ - wm) * sc, (Tp - Tm) * sc, h);
+    // x and y gradients of a ring field at the own points (and its own values)
+    auto grad_x = [&](const R *f, R g[PX], R f0[PX]) {
+        if constexpr (PX == 2) {
+            R x[6];
+            row(f + bc, x);
+            g[0] = (x[3] - x[1]) * C.hdx;
+            g[1] = (x[4] - x[2]) * C.hdx;
+            f0[0] = x[2];
+            f0[1] = x[3];
+        } else {
+            g[0] = (f[bc + 1] - f[bc - 1]) * C.hdx;
+            f0[0] = f[bc];
+        }
     };
-    // hD at the own column of wall plane m, from the wall's own values in
+    auto grad_y = [&](const R *f, R g[PX]) {
+        R a[PX], b[PX];
+        ldp<PX>(f + bc + BX, a);
+        ldp<PX>(f + bc - BX, b);
+#pragma unroll
+        for (int k = 0; k < PX; k++) g[k] = (a[k] - b[k]) * C.hdy;
+    };
+    auto own = [&](const R *f, R f0[PX]) { ldp<PX>(f + bc, f0); };
+    // mu and p = rho T / (gama Ma^2) at the own points: mu at mo, Q slot s, T
+    auto mu_p = [&](int mo, int s, const R T0[PX], R mu[PX], R pr[PX]) {
+        own(smu(mo), mu);
+        own(sq(s, 0), pr);
+#pragma unroll
+        for (int k = 0; k < PX; k++) pr[k] = (pr[k] * T0[k]) * C.inv_gM2;
+    };
+
+    // hD at the own columns of interior plane m (prims at po, mu at mo, Q
+    // slot s); dz from (m-1, m+1) values
+    auto hflux = [&](int m, int po, int mo, int s, const R um[PX], const R vm[PX], const R wm[PX], const R Tm[PX],
+                     const R up[PX], const R vp[PX], const R wp_[PX], const R Tp[PX], R h[PX][4]) {
+        const Slot sl = slot(po);
+        const R sc = ktab(kCzh, m);
+        R ux[PX], vy[PX], wx[PX], wy[PX], u0[PX], v0[PX], w0[PX], T0[PX], mu[PX], pr[PX];
+        grad_x(sl.U, ux, u0);
+        grad_y(sl.V, vy);
+        own(sl.V, v0);
+        grad_x(sl.W, wx, w0);
+        grad_y(sl.W, wy);
+        own(sl.T, T0);
+        mu_p(mo, s, T0, mu, pr);
+#pragma unroll
+        for (int a = 0; a < PX; a++)
+            visc_fz_vals(C, ux[a], vy[a], wx[a], wy[a], u0[a], v0[a], w0[a], mu[a], pr[a], (up[a] - um[a]) * sc,
+                         (vp[a] - vm[a]) * sc, (wp_[a] - wm[a]) * sc, (Tp[a] - Tm[a]) * sc, h[a]);
+    };
+    // hD at column `colo + a` of wall plane m, from the wall's own values in
     // memory, in double; one-sided dz against the interior neighbour values
     // (ui..Ti): (q(2)-q(1))/dz1 at the bottom, (q(nP3)-q(nP3-1))/dzN at the
     // top.  The pressure is the pressure-BC state.
-    auto hflux_wall = [&](int m, double ui, double vi, double wi, double Ti, double h[4]) {
-        const double *W = P.wp + (size_t)(m == 1 ? 0 : 8) * plane + colo;
+    auto hflux_wall = [&](int m, int a, double ui, double vi, double wi, double Ti, double h[4]) {
+        const double *W = P.wp + (size_t)(m == 1 ? 0 : 8) * plane + colo + a;
         const long long px = P.px;
         const double u0 = W[plane], v0 = W[2 * plane], w0 = W[3 * plane], T0 = W[5 * plane];
         const double sc = m == 1 ? P.inv_dz1 : P.inv_dzN;
@@ -982,580 +1101,381 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
         visc_fz_vals(P.cd, ux, vy, wx, wy, u0, v0, w0, W[7 * plane], W[6 * plane], uz, vz, wz, Tz, h);
     };
 
-    // halo-flux lanes: fD of the two x-halo columns on lanes 0..2TJ-1 of warp
-    // 0, gD of the two y-halo rows on lanes 32..32+2TI-1.  Each owns one halo
-    // point for the whole march and keeps that point's plane t-1 values (u or
-    // v, and w) in sH[.][tid].  hbox: the point's box index.
-    const bool hx_lane = tid < 2 * TJ;
-    const bool hy_lane = tid >= 32 && tid < 32 + 2 * TI;
-    auto hbox = [&]() -> int {
-        if (hx_lane) {
-            const int side = tid / TJ, r = tid - side * TJ;
+    // halo-flux points h: fD of the two x-halo columns at h < 2*TJ, gD of the two
+    // y-halo rows from there on.  The x ones are taken by the first warp, the y ones
+    // by the next ones, one point per thread (a second one where the CTA has fewer
+    // threads).  plane t-1's values (u or v, and w) of point h are kept in sH[.][h].
+    auto hbox = [&](int h) -> int {
+        if (h < 2 * TJ) {
+            const int side = h / TJ, r = h - side * TJ;
             return (r + 2) * BX + (side ? TI + 2 : 1);
         }
-        const int h = tid - 32, side = h / TI, cc = h - side * TI;
+        const int side = (h - 2 * TJ) / TI, cc = h - 2 * TJ - side * TI;
         return (side ? TJ + 2 : 1) * BX + cc + 2;
     };
-    // the halo lane's values (u or v, w) in ring slot sl, kept as plane t-1
-    auto keep_halo = [&](const Slot &sl) {
-        if (hx_lane || hy_lane) {
-            const int b = hbox();
-            sH[tid] = hx_lane ? sl.U[b] : sl.V[b];
-            sH[S::NHL + tid] = sl.W[b];
+    auto each_halo = [&](auto &&f) {
+#pragma unroll
+        for (int h0 = 0; h0 < 32 + 2 * TI; h0 += NT) {
+            const int l = tid + h0;
+            if (l < 2 * TJ) f(l);
+            else if (l >= 32 && l < 32 + 2 * TI) f(l - 32 + 2 * TJ);
         }
+    };
+    // the halo points' values (u or v, w) in ring slot sl, kept as plane t-1
+    auto keep_halo = [&](const Slot &sl) {
+        each_halo([&](int h) {
+            const int b = hbox(h);
+            sH[h] = h < 2 * TJ ? sl.U[b] : sl.V[b];
+            sH[NHL + h] = sl.W[b];
+        });
     };
 
     // ---------------- prologue: planes kb-1 (Q slot 0, prims at pP) and kb
-    // (Q slot 1, prims at pZ); hD(kb-1), hD(kb); plane kb+1 starts its way in
+    // (Q slot 1, prims at pZ); hD(kb-1); plane kb+1 starts its way in
     issue(kb - 1, 0);
     issue(kb, 1);
     issue(kb + 1, 2);   // kb+1 <= ke+1 <= nP3
+    issue_base(kb);
     bool bad = !wait_slot(0);
-    convert(kb - 1, 0, pP, mP, false, no_extra);
+    convert(kb - 1, 0, pP, mP, false);
     bad = !wait_slot(1) || bad;
-    convert(kb, 1, pZ, mZ, false, no_extra);
+    convert(kb, 1, pZ, mZ, false);
     if (__syncthreads_or(bad)) { give_up(); return; }
 
-    R qm2[5] = {0, 0, 0, 0, 0}, qm1[5], hm1[4] = {0, 0, 0, 0}, h0[4] = {0, 0, 0, 0};
-    R wm2 = R(0), um1 = R(0), vm1 = R(0), wm1 = R(0);   // own column: w at t-2; u, v, w at t-1
     {
         const Slot sA = slot(pP), sB = slot(pZ);
         if (col_ok) {
+            R uA[PX], vA[PX], wA[PX], uB[PX], vB[PX], wB[PX], TB[PX];
+            own(sA.U, uA); own(sA.V, vA); own(sA.W, wA);
+            own(sB.U, uB); own(sB.V, vB); own(sB.W, wB); own(sB.T, TB);
             // hD(kb-1)
             if (kb - 1 == 1) {
-                double h[4];
-                hflux_wall(1, sB.U[bc], sB.V[bc], sB.W[bc], sB.T[bc], h);
 #pragma unroll
-                for (int c = 0; c < 4; c++) hm1[c] = (R)h[c];
+                for (int a = 0; a < PX; a++) {
+                    double h[4];
+                    if (a == 0 || i + a <= n1) {
+                        hflux_wall(1, a, uB[a], vB[a], wB[a], TB[a], h);
+#pragma unroll
+                        for (int c = 0; c < 4; c++) h1[a][c] = (R)h[c];
+                    }
+                }
             } else {
-                double q[5], u, v, w, T;
+                double q[5][PX], u[PX], v[PX], w[PX], T[PX];
                 center(kb - 2, q, u, v, w, T);
-                hflux(kb - 1, pP, mP, 0, (R)u, (R)v, (R)w, (R)T, sB.U[bc], sB.V[bc], sB.W[bc], sB.T[bc], hm1);
-            }
-            // hD(kb)
-            {
-                double q[5], u, v, w, T;
-                center(kb + 1, q, u, v, w, T);
-                hflux(kb, pZ, mZ, 1, sA.U[bc], sA.V[bc], sA.W[bc], sA.T[bc], (R)u, (R)v, (R)w, (R)T, h0);
-            }
-            if (kb - 2 >= 1) {
-                double q[5], u, v, w, T;
-                center(kb - 2, q, u, v, w, T);
+                R ur[PX], vr[PX], wr[PX], Tr[PX];
 #pragma unroll
-                for (int c = 0; c < 5; c++) qm2[c] = (R)q[c];
-                wm2 = (R)w;
-            }
-            // the last chunk stages hD of the top wall plane for its last plane
-            if (ke == n3 - 1) {
-                double q[5], u, v, w, T, h[4];
-                center(n3 - 1, q, u, v, w, T);
-                hflux_wall(n3, u, v, w, T, h);
+                for (int a = 0; a < PX; a++) {
+                    ur[a] = (R)u[a]; vr[a] = (R)v[a]; wr[a] = (R)w[a]; Tr[a] = (R)T[a];
+                    wm2[a] = wr[a];
 #pragma unroll
-                for (int c = 0; c < 4; c++) P.hwt[c * plane + colo] = h[c];
+                    for (int c = 0; c < 5; c++) qm2[c][a] = (R)q[c][a];
+                }
+                hflux(kb - 1, pP, mP, 0, ur, vr, wr, Tr, uB, vB, wB, TB, h1);
             }
 #pragma unroll
-            for (int c = 0; c < 5; c++) qm1[c] = sq(0, c)[bc];
-            um1 = sA.U[bc]; vm1 = sA.V[bc]; wm1 = sA.W[bc];
-        } else {
+            for (int c = 0; c < 5; c++) own(sq(0, c), qm1[c]);
 #pragma unroll
-            for (int c = 0; c < 5; c++) qm1[c] = R(0);
+            for (int a = 0; a < PX; a++) { um1[a] = uA[a]; vm1[a] = vA[a]; wm1[a] = wA[a]; }
+            own(sA.T, Tm1);
         }
         keep_halo(sA);
     }
     __syncthreads();
 
-    for (int t = kb; t <= ke; t++) {
-        // ---------- A: own column of t+2; (float rings: the own point's RK base
-        // starts its way into shared memory); plane t+1's box is converted, beside
-        // the inviscid x/y sums of plane t; after the barrier, plane t+2's box
-        // starts its way in (converted at the next plane)
-        // No barrier ends the plane (neb), so a warp that has finished plane t's
-        // update goes on to plane t+1's loads, box wait and conversion while others
-        // still run phase E.  What makes that safe: plane t+2's box goes into the
-        // slot of plane t-1 only after phase A's barrier, which every thread passes
-        // after its phase-E reads of that slot; and what phases E and F read of
-        // plane t's primitive and (mu, p) slots, which the next plane's conversion
-        // overwrites, is read before barrier C.  FP64 stage time 3.5% lower together
-        // with the split own-column conversion below (alone 1% higher); float 1%
-        // lower.  CHAN_END_BAR restores the barrier, for measurement.
-#ifndef CHAN_END_BAR
-        constexpr bool neb = !S::tma_base;
-#else
-        constexpr bool neb = false;
-#endif
-        if (t < ke && !neb) issue(t + 2, iN);
-        const bool need_base = P.rk_mode != 0;
-        if (S::tma_base && need_base) issue_base(t);
-        if (S::prefetch_base) {
-            if (P.rk_mode != 0 && out_ok) {
-                const double *src = P.qbase + (long long)t * plane + colo;
+    // source of plane m: lagged wall-shear forcing (main_v1.9.f90:565-571), formed on
+    // every launch (the statistics array always holds these entries) and selected by
+    // the flag; buoyancy on the wall-normal momentum and its work on the energy
+    auto source = [&](int m, const R u[PX], const R w[PX], const R T[PX], const R r[PX], double s2[PX], double s4[PX],
+                      double s5[PX]) {
+        const double tau = *stau, rb = rbar(m);
+        const double f2 = (0.5 * tau) * rb;
 #pragma unroll
-                for (int c = 0; c < 5; c++) cp_async8(sQB + c * NT + tid, src + c * vol);
-            }
-            cp_async_commit();
-        }
-#ifndef CHAN_NO_PREFETCH_BASE_L1
-        // the own point's RK base into L1 now; the update reads it at the end of
-        // the plane (2.7% of the FP64 stage time against loading it there cold)
-        if (!S::prefetch_base && !S::tma_base && P.rk_mode != 0 && out_ok) {
-            const double *src = P.qbase + (long long)t * plane + colo;
-#pragma unroll
-            for (int c = 0; c < 5; c++) asm volatile("prefetch.global.L1 [%0];" ::"l"(src + c * vol));
-        }
-#endif
-        // FP64: plane t+3's own column into L1 a plane before it is loaded (1.8% of the
-        // FP64 stage time; the float kernels, which load plane t+2 in phase C, are
-        // slower with it)
-        if (sizeof(R) == 8 && col_ok && t + 3 <= n3) {
-            const QI *src = qin() + (long long)(t + 3) * plane + colo;
-#pragma unroll
-            for (int c = 0; c < 5; c++) asm volatile("prefetch.global.L1 [%0];" ::"l"(src + c * vol));
-        }
-        R qp2[5] = {0, 0, 0, 0, 0}, up2 = 0, vp2 = 0, wp2 = 0, Tp2 = 0;
-        // FP64: plane t+2's own column is loaded before the box wait and converted
-        // after it, in the straight-line block of the box conversion (1.9% of the
-        // stage time alone, 3.5% with neb); CHAN_T2_JOINED converts it at its load
-#ifndef CHAN_T2_JOINED
-        constexpr bool t2_split = !late_t2;
-#else
-        constexpr bool t2_split = false;
-#endif
-        const bool own2 = col_ok && t + 2 < n3;   // plane t+2's own column is an interior one
-        double cq[5] = {0, 0, 0, 0, 0};
-        // plane t+2's own column: the float kernels prefetch it into L1 here and
-        // load and convert it in phase C, where its values start to be used; the
-        // FP64 kernel loads and converts it here but reads its Q again in phase E
-        // (an L1 hit) instead of keeping it in registers across the plane
-        if (late_t2) {
-            if (col_ok && t + 2 <= n3) {
-                const QI *src = qin() + (long long)(t + 2) * plane + colo;
-#pragma unroll
-                for (int c = 0; c < 5; c++) asm volatile("prefetch.global.L1 [%0];" ::"l"(src + c * vol));
-            }
-        } else if (t2_split && own2) {
-            // interior plane t+2: its own column's Q now, its primitives after the box wait
-            const long long off = (long long)(t + 2) * plane + colo;
-#pragma unroll
-            for (int c = 0; c < 5; c++) cq[c] = ldq_c<PERSIST>(qin() + c * vol + off);
-        } else if (col_ok && t + 2 <= n3) {
-            double q[5], u, v, w, T;
-            center(t + 2, q, u, v, w, T);
-            if (!late_qp2) {
-#pragma unroll
-                for (int c = 0; c < 5; c++) qp2[c] = (R)q[c];
-            }
-            up2 = (R)u; vp2 = (R)v; wp2 = (R)w; Tp2 = (R)T;
-        }
-        // the primitives of plane t+2's own column formed in the same straight-line
-        // block as the box conversion (selects keep the other cases' values)
-        auto t2_prims = [&]() {
-            if (t2_split) {
-                double u, v, w, T;
-                prims_from_q(P, cq, u, v, w, T);
-                up2 = own2 ? (R)u : up2;
-                vp2 = own2 ? (R)v : vp2;
-                wp2 = own2 ? (R)w : wp2;
-                Tp2 = own2 ? (R)T : Tp2;
-                if (!late_qp2) {
-#pragma unroll
-                    for (int c = 0; c < 5; c++) qp2[c] = own2 ? (R)cq[c] : qp2[c];
-                }
-            }
-        };
-        bad = !wait_slot(iP);
-        convert(t + 1, iP, pP, mP, true, t2_prims);
-        if (__syncthreads_or(bad)) { give_up(); return; }
-        if (t < ke && neb) issue(t + 2, iN);
-
-        // ---------- C: viscous flux vectors
-        const Slot s0 = slot(pZ), sp = slot(pP);
-        R hp1[4] = {0, 0, 0, 0};
-        R fown[4] = {0, 0, 0, 0};   // fD at the own column (exchanged by shuffles when fx_shfl)
-        {
-            const R czt = ktab<R>(P, 0, t);
-            const R *MU = smu(mZ), *PR = spr(mZ, iZ);
-            if (col_ok) {
-                if (late_t2 && t + 2 <= n3) {
-                    double q[5], u, v, w, T;
-                    center(t + 2, q, u, v, w, T);
-#pragma unroll
-                    for (int c = 0; c < 5; c++) qp2[c] = (R)q[c];
-                    up2 = (R)u; vp2 = (R)v; wp2 = (R)w; Tp2 = (R)T;
-                }
-                // FP64 rings: hD(t+1) on every plane (on the top wall plane it reads the
-                // wall's valid ring values and is not used), so that it shares one
-                // straight-line block with fD and gD (0.9% of the FP64 stage time; the
-                // float kernels keep the uniform branch, 0.2% faster).  CHAN_HFLUX_GUARD
-                // keeps the branch in the FP64 kernel too, for measurement.
-#ifdef CHAN_HFLUX_GUARD
-                constexpr bool hflux_all = false;
-#else
-                constexpr bool hflux_all = sizeof(R) == 8;
-#endif
-                if (hflux_all) {
-                    R h[4];
-                    hflux(t + 1, pP, mP, iP, s0.U[bc], s0.V[bc], s0.W[bc], s0.T[bc], up2, vp2, wp2, Tp2, h);
-                    const bool hok = t + 1 != n3;
-#pragma unroll
-                    for (int c = 0; c < 4; c++) hp1[c] = hok ? h[c] : R(0);
-                } else if (t + 1 != n3) {
-                    hflux(t + 1, pP, mP, iP, s0.U[bc], s0.V[bc], s0.W[bc], s0.T[bc], up2, vp2, wp2, Tp2, hp1);
-                }
-                R g[4];
-                visc_fxy<BX, R, S::p_ring>(C, s0, um1, vm1, wm1, sp, MU, PR, bc, czt, fown, g);
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    if (!S::fx_shfl) sF[(c * TJ + ty) * (TI + 2) + tx + 1] = fown[c];
-                    sG[(c * (TJ + 2) + ty + 1) * TI + tx] = g[c];
-                }
-            }
-            if (hx_lane) {
-                const int side = tid / TJ, r = tid - side * TJ;
-                const int ci = side ? i0 + TI : i0 - 1, cj = j0 + r;
-                if (ci <= n1 && cj <= n2) {
-                    R f[4];
-                    visc_fx<BX, R, S::p_ring>(C, s0, sH[tid], sH[S::NHL + tid], sp, MU, PR,
-                                              (r + 2) * BX + (side ? TI + 2 : 1), czt, f);
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        if (S::fx_shfl) sF[c * S::NFX + r * 2 + side] = f[c];
-                        else sF[c * S::NFX + r * (TI + 2) + (side ? TI + 1 : 0)] = f[c];
-                    }
-                }
-            } else if (hy_lane) {
-                const int h = tid - 32, side = h / TI, cc = h - side * TI;
-                const int ci = i0 + cc, cj = side ? j0 + TJ : j0 - 1;
-                if (ci <= n1 && cj <= n2) {
-                    R g[4];
-                    visc_fy<BX, R, S::p_ring>(C, s0, sH[tid], sH[S::NHL + tid], sp, MU, PR,
-                                              (side ? TJ + 2 : 1) * BX + cc + 2, czt, g);
-#pragma unroll
-                    for (int c = 0; c < 4; c++) sG[c * S::NGY + (side ? TJ + 1 : 0) * TI + cc] = g[c];
-                }
-            }
-        }
-        // without the end-of-plane barrier, the next plane's conversion overwrites
-        // plane t's primitive and (mu, p) slots while this plane's phase E may still
-        // run: what phases E and F read of them is read here, before barrier C
-        R w0n = R(0), mu0n = R(0), T0n = R(0);
-        if (neb) {
-            um1 = s0.U[bc]; vm1 = s0.V[bc];   // plane t-1's u, v are not read after phase C
-            w0n = s0.W[bc];
-            mu0n = smu(mZ)[bc];
-            if (buoy) T0n = s0.T[bc];
-            keep_halo(s0);
-        }
-        if (S::tma_base && need_base) {
-            bad = !wait_slot(3);
-            if (__syncthreads_or(bad)) { give_up(); return; }
-        } else {
-            __syncthreads();
-        }
-
-        // ---------- E: fluxes, source, RK update
-        // fD at the x neighbours: lanes tx+-1 of the row's warp, the halo columns
-        // at the row's ends (every lane takes part in the shuffles)
-        R fxp[4], fxm[4];
-        if (S::fx_shfl) {
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                fxp[c] = __shfl_down_sync(0xffffffffu, fown[c], 1);
-                fxm[c] = __shfl_up_sync(0xffffffffu, fown[c], 1);
-                if (tx == TI - 1) fxp[c] = sF[c * S::NFX + ty * 2 + 1];
-                if (tx == 0) fxm[c] = sF[c * S::NFX + ty * 2 + 0];
-            }
-        }
-        R q0[5];
-#pragma unroll
-        for (int c = 0; c < 5; c++) q0[c] = sq(iZ, c)[bc];
-        if (out_ok) {
-#ifdef CHAN_EARLY_BASE
-            // the RK base of the own point, loaded before the flux sums so that
-            // its latency overlaps them (FP64 rings)
-            double qbe[5] = {0, 0, 0, 0, 0};
-            if (!S::prefetch_base && P.rk_mode != 0) {
-                const long long off = (long long)t * plane + colo;
-#pragma unroll
-                for (int c = 0; c < 5; c++) qbe[c] = ldq_c<PERSIST>(P.qbase + c * vol + off);
-            }
-#endif
-            R Fs[5];   // sum of the flux derivatives
-            const R mu0 = neb ? mu0n : smu(mZ)[bc];
-            if (xy_a) {
-                // (F1 + G1) from phase A, then the viscous x and y terms
-                Fs[0] = Fxy[0];
-#pragma unroll
-                for (int c = 1; c < 5; c++) {
-                    R F2;
-                    if (S::fx_shfl) {
-                        F2 = (fxp[c - 1] - fxm[c - 1]) * C.hdx;
-                    } else {
-                        const int r = (c - 1) * TJ + ty;
-                        F2 = (sF[r * (TI + 2) + tx + 2] - sF[r * (TI + 2) + tx]) * C.hdx;
-                    }
-                    const R G2 = (sG[((c - 1) * (TJ + 2) + ty + 2) * TI + tx] -
-                                  sG[((c - 1) * (TJ + 2) + ty) * TI + tx]) * C.hdy;
-                    Fs[c] = (Fxy[c] + F2) + G2;
-                }
-            }
-            // x
-            if (!xy_a) {
-                const R *U = s0.U;
-                const bool qk = (C.pex * fabs(q0[1])) > C.PexVal * mu0;
-                R w[5];
-                inv_weights(U[bc - 2], U[bc - 1], U[bc], U[bc + 1], U[bc + 2], qk, C.sx8, C.sx12, w);
-                R F1[5];
-#pragma unroll
-                for (int c = 0; c < 5; c++) {
-                    const R *Q = sq(iZ, c);
-                    F1[c] = wsum(w, Q[bc - 2], Q[bc - 1], Q[bc], Q[bc + 1], Q[bc + 2]);
-                }
-                Fs[0] = F1[0];  // F2 of continuity is zero
-#pragma unroll
-                for (int c = 1; c < 5; c++) {
-                    R F2;
-                    if (S::fx_shfl) {
-                        F2 = (fxp[c - 1] - fxm[c - 1]) * C.hdx;
-                    } else {
-                        const int r = (c - 1) * TJ + ty;
-                        F2 = (sF[r * (TI + 2) + tx + 2] - sF[r * (TI + 2) + tx]) * C.hdx;
-                    }
-                    Fs[c] = F1[c] + F2;
-                }
-            }
-            // y
-            if (!xy_a) {
-                const R *V = s0.V;
-                const bool qk = (C.pey * fabs(q0[2])) > C.PeyVal * mu0;
-                R w[5];
-                inv_weights(V[bc - 2 * BX], V[bc - BX], V[bc], V[bc + BX], V[bc + 2 * BX], qk, C.sy8, C.sy12, w);
-                R G1[5];
-#pragma unroll
-                for (int c = 0; c < 5; c++) {
-                    const R *Q = sq(iZ, c);
-                    G1[c] = wsum(w, Q[bc - 2 * BX], Q[bc - BX], Q[bc], Q[bc + BX], Q[bc + 2 * BX]);
-                }
-                Fs[0] = Fs[0] + G1[0];
-#pragma unroll
-                for (int c = 1; c < 5; c++) {
-                    const R G2 = (sG[((c - 1) * (TJ + 2) + ty + 2) * TI + tx] -
-                                  sG[((c - 1) * (TJ + 2) + ty) * TI + tx]) * C.hdy;
-                    Fs[c] = (Fs[c] + G1[c]) + G2;
-                }
-            }
-            // z
-            {
-                const R w0 = neb ? w0n : s0.W[bc], wp1 = sp.W[bc];
-                R w[5];
-                // FP64 rings: the second-order weights of the planes next to the walls
-                // and the hybrid ones both formed and selected by the (uniform) plane
-                // test, so that the update's block has no branch (0.7% of the FP64 stage
-                // time); CHAN_ZW_BRANCH keeps the branch, for measurement
-#ifdef CHAN_ZW_BRANCH
-                constexpr bool zw_sel = false;
-#else
-                constexpr bool zw_sel = sizeof(R) == 8;
-#endif
-                if (zw_sel) {
-                    // both weight sets, selected by the (uniform) plane test: no branch
-                    // in the update's block (the tables hold nP3+2 entries, so the
-                    // interior set's reads stay in range on every plane)
-                    const bool near = t < 3 || t > n3 - 2;
-                    const R c2 = ktab<R>(P, 0, t);
-                    const bool qk = (ktab<R>(P, 3, t) * fabs(q0[3])) > C.pez_val * mu0;
-                    R wi[5];
-                    inv_weights(wm2, wm1, w0, wp1, wp2, qk, ktab<R>(P, 1, t), ktab<R>(P, 2, t), wi);
-                    w[0] = near ? R(0) : wi[0];
-                    w[1] = near ? -(wm1 * c2) : wi[1];
-                    w[2] = near ? R(0) : wi[2];
-                    w[3] = near ? wp1 * c2 : wi[3];
-                    w[4] = near ? R(0) : wi[4];
-                } else if (t < 3 || t > n3 - 2) {
-                    const R c2 = ktab<R>(P, 0, t);
-                    w[0] = R(0); w[1] = -(wm1 * c2); w[2] = R(0); w[3] = wp1 * c2; w[4] = R(0);
-                } else {
-                    const bool qk = (ktab<R>(P, 3, t) * fabs(q0[3])) > C.pez_val * mu0;
-                    inv_weights(wm2, wm1, w0, wp1, wp2, qk, ktab<R>(P, 1, t), ktab<R>(P, 2, t), w);
-                }
-                const R czt = ktab<R>(P, 0, t);
-                // plane t+2's own-column Q again (in L1 since phase A)
-                if (late_qp2 && t + 2 <= n3) {
-                    const long long off = (long long)(t + 2) * plane + colo;
-#pragma unroll
-                    for (int c = 0; c < 5; c++) qp2[c] = (R)ldq_c<PERSIST>(qin() + c * vol + off);
-                }
-                Fs[0] = Fs[0] + wsum(w, qm2[0], qm1[0], q0[0], sq(iP, 0)[bc], qp2[0]);
-                const bool top = t + 1 == n3;   // hD of the top wall plane was staged in the prologue
-                // float rings: the top plane's hD from the prologue's staging, under one
-                // uniform branch (hp1 is not formed on the top plane, and the march ends
-                // there).  Measured with the select weights: 1% faster in the float
-                // kernels, 1% slower in the FP64 one (register allocation), which keeps
-                // the select inside the flux loop.
-#ifdef CHAN_TOP_HOIST_D
-                constexpr bool hoist_d = true;
-#else
-                constexpr bool hoist_d = false;
-#endif
-#ifdef CHAN_NO_TOP_HOIST_F
-                constexpr bool hoist_f = false;
-#else
-                constexpr bool hoist_f = true;
-#endif
-                constexpr bool hoist = sizeof(R) == 8 ? hoist_d : hoist_f;
-                if (hoist && top) {
-#pragma unroll
-                    for (int c = 0; c < 4; c++) hp1[c] = (R)P.hwt[c * plane + colo];
-                }
-#pragma unroll
-                for (int c = 1; c < 5; c++) {
-                    const R H1 = wsum(w, qm2[c], qm1[c], q0[c], sq(iP, c)[bc], qp2[c]);
-                    const R hp = hoist ? hp1[c - 1] : (top ? (R)P.hwt[(c - 1) * plane + colo] : hp1[c - 1]);
-                    const R H2 = (hp - hm1[c - 1]) * czt;
-                    Fs[c] = (Fs[c] + H1) + H2;
-                }
-            }
-            // source: lagged wall-shear forcing (main_v1.9.f90:565-571), in double
-            double src2 = 0.0, src5 = 0.0;
-            // FP64 rings: the forcing terms formed on every launch (the statistics
-            // array always holds these entries) and selected by the flag, so that the
-            // update's block has no branch on it (1.1% of the FP64 stage time);
-            // CHAN_FORCE_BRANCH keeps the branch, for measurement
-#if defined(CHAN_FORCE_BRANCH)
-            constexpr bool force_sel = false;
-#elif defined(CHAN_FORCE_SEL_F)
-            constexpr bool force_sel = true;
-#else
-            constexpr bool force_sel = sizeof(R) == 8;
-#endif
-            if (force_sel) {
-                const double tau = P.stat[23 * n3 + 0] - P.stat[23 * n3 + 1];
-                const double rb = P.stat[t - 1];
-                const double s2 = (0.5 * tau) * rb;
-                const double s5 = (((P.ggM * (double)(neb ? um1 : s0.U[bc])) * 0.5) * tau) * rb;
-                src2 = P.force_on ? s2 : 0.0;
-                src5 = P.force_on ? s5 : 0.0;
-            } else if (P.force_on) {
-                const double tau = P.stat[23 * n3 + 0] - P.stat[23 * n3 + 1];
-                const double rb = P.stat[t - 1];
-                src2 = (0.5 * tau) * rb;
-                src5 = (((P.ggM * (double)(neb ? um1 : s0.U[bc])) * 0.5) * tau) * rb;
-            }
-            double Rd[5];
-            Rd[0] = -(double)Fs[0];
-            Rd[1] = src2 - (double)Fs[1];
-            Rd[2] = -(double)Fs[2];
-            Rd[3] = -(double)Fs[3];
+        for (int a = 0; a < PX; a++) {
+            const double f5 = (((P.ggM * (double)u[a]) * 0.5) * tau) * rb;
+            s2[a] = P.force_on ? f2 : 0.0;
+            s4[a] = 0.0;
+            s5[a] = P.force_on ? f5 : 0.0;
             if (buoy) {
-                // buoyancy on the wall-normal momentum and its work on the energy
-                const double bq = P.ri * ((double)q0[0] * ((double)(neb ? T0n : s0.T[bc]) - P.tref));
-                Rd[3] = bq - (double)Fs[3];
-                src5 = src5 + (P.ggM * (double)(neb ? w0n : s0.W[bc])) * bq;
-            }
-            Rd[4] = src5 - (double)Fs[4];
-            // RK update in double, on the stage input at its stored precision
-            double qs[5];
-            if (std::is_same<QI, R>::value) {
-#pragma unroll
-                for (int c = 0; c < 5; c++) qs[c] = (double)q0[c];
-            } else {
-                const long long off = (long long)t * plane + colo;
-#pragma unroll
-                for (int c = 0; c < 5; c++) qs[c] = ldq_c<PERSIST>(qin() + c * vol + off);
-            }
-            double qn[5];
-            double qb[5] = {0, 0, 0, 0, 0};
-            if (P.rk_mode != 0) {
-                if (S::tma_base) {
-#pragma unroll
-                    for (int c = 0; c < 5; c++) qb[c] = sQB[c * NT + tid];
-                } else if (S::prefetch_base) {
-                    cp_async_wait<0>();
-#pragma unroll
-                    for (int c = 0; c < 5; c++) qb[c] = sQB[c * NT + tid];
-                } else {
-#ifdef CHAN_EARLY_BASE
-#pragma unroll
-                    for (int c = 0; c < 5; c++) qb[c] = qbe[c];
-#else
-                    const long long off = (long long)t * plane + colo;
-#pragma unroll
-                    for (int c = 0; c < 5; c++) qb[c] = ldq_c<PERSIST>(P.qbase + c * vol + off);
-#endif
-                }
-            }
-            if (P.rk_mode == 0) {
-#pragma unroll
-                for (int c = 0; c < 5; c++) qn[c] = qs[c] + P.rk_cdt * Rd[c];
-            } else if (P.rk_mode == 1) {
-#pragma unroll
-                for (int c = 0; c < 5; c++) qn[c] = qb[c] + P.rk_cdt * Rd[c];
-            } else {
-#pragma unroll
-                for (int c = 0; c < 5; c++) qn[c] = (P.rk_a * qb[c] + P.rk_b * qs[c]) + P.rk_cdt * Rd[c];
-            }
-            // store + periodic images (the ghosts the reference's halo exchange fills)
-            const int im = (i <= 3) ? i + (n1 - 2) : ((i >= n1 - 2) ? i - (n1 - 2) : -1);
-            const int jm = (j <= 3) ? j + (n2 - 2) : ((j >= n2 - 2) ? j - (n2 - 2) : -1);
-            const long long pk = (long long)t * plane;
-            // FP64 rings: the periodic images under one branch that only points within 2
-            // of a periodic edge take (0.7% of the stage time); the float rings keep
-            // predicated stores (the branch costs them spills)
-#ifndef CHAN_NO_IMAGE_BRANCH
-            constexpr bool img_branch = sizeof(R) == 8;
-#else
-            constexpr bool img_branch = false;
-#endif
-            if (img_branch) {
-                // own point; then, only at points within 2 of a periodic edge, the images
-#pragma unroll
-                for (int c = 0; c < 5; c++) qout()[c * vol + pk + colo] = (QO)qn[c];
-                if (im >= 0 || jm >= 0) {
-#pragma unroll
-                    for (int c = 0; c < 5; c++) {
-                        QO *O = qout() + c * vol + pk;
-                        const QO v = (QO)qn[c];
-                        if (im >= 0) O[(long long)j * P.px + im] = v;
-                        if (jm >= 0) O[(long long)jm * P.px + i] = v;
-                        if (im >= 0 && jm >= 0) O[(long long)jm * P.px + im] = v;
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < 5; c++) {
-                    QO *O = qout() + c * vol + pk;
-                    const QO v = (QO)qn[c];
-                    O[(long long)j * P.px + i] = v;
-                    if (im >= 0) O[(long long)j * P.px + im] = v;
-                    if (jm >= 0) O[(long long)jm * P.px + i] = v;
-                    if (im >= 0 && jm >= 0) O[(long long)jm * P.px + im] = v;
-                }
-            }
-            if (P.check) {
-                const double tr = qn[0] * qn[4] - P.ggMh * ((qn[1] * qn[1] + qn[2] * qn[2]) + qn[3] * qn[3]);
-                if (qn[0] < 0.0 || (qn[0] > 0.0 && tr < 0.0)) flag_blown(P.status, i, j, t, kstep(P));
-                bool fin = true;
-#pragma unroll
-                for (int c = 0; c < 5; c++) fin = fin && isfinite(qn[c]);
-                if (!fin) flag_nonfinite(P.status, i, j, t);
+                const double bq = P.ri * ((double)r[a] * ((double)T[a] - P.tref));
+                s4[a] = bq;
+                s5[a] = s5[a] + (P.ggM * (double)w[a]) * bq;
             }
         }
-        // ---------- F: plane t becomes t-1; rotate the rings (no barrier: see neb)
+    };
+    // Plane tz completed from what plane tz+2 brings: w and Q of plane tz+2 (wn, getq)
+    // and hD(tz+1) (h).  Of the periodic images (the ghosts the reference's halo exchange
+    // fills) those in x are stored here, by one predicated store; those in y are whole
+    // rows, which the kernel that follows copies (image_body).  With all of them
+    // stored here the CTAs at the periodic edges, a third of all, took 10% longer than
+    // the others, and the whole launch with them.
+    auto complete = [&](int tz, const R wn[PX], const R h[PX][4], bool staged, auto &&getq) {
+        const R s12p = ktab(kS12o, tz), czp = ktab(kCzh, tz);
+        const long long off = (long long)tz * plane + colo;
+        R wq[PX];
+        double qu[5][PX];
+        [[maybe_unused]] double s2[PX], s4[PX], s5[PX];
+#pragma unroll
+        for (int a = 0; a < PX; a++) wq[a] = qk[a] ? w4[a] : -(wn[a] * s12p);
+        if constexpr (!FOLD) {
+            source(tz, um1, wm1, Tm1, qm1[0], s2, s4, s5);
+            if (need_base && staged) cp_async_wait<0>();
+        }
 #pragma unroll
         for (int c = 0; c < 5; c++) {
-            qm2[c] = qm1[c];
-            qm1[c] = q0[c];
-        }
-        wm2 = wm1;
-        if (neb) {
-            wm1 = w0n;
-        } else {
-            um1 = s0.U[bc]; vm1 = s0.V[bc]; wm1 = s0.W[bc];
-            keep_halo(s0);
+            const int d = c > 0 ? c - 1 : 0;
+            R qn[PX];
+            getq(c, qn);
+            if constexpr (FOLD) {
+#pragma unroll
+                for (int a = 0; a < PX; a++) {
+                    R x = wq[a] * qn[a];
+                    if (c > 0) x = fmaR(h[a][d], czp, x);
+                    qu[c][a] = qm1[c][a] + fmaR(-(R)P.rk_cdt, x, Fs[a][c]);
+                }
+            } else {
+                // in double, on the stage input at its stored precision
+                double qs[PX], qb[PX];
+                if (TMA) {
+#pragma unroll
+                    for (int a = 0; a < PX; a++) qs[a] = (double)qm1[c][a];
+                } else {
+                    ldgp<PX, PERSIST>(qin() + c * vol + off, qs);
+                }
+                if (need_base) {
+                    if (staged) ldp<PX>(sQB + (c * NT + tid) * PX, qb);
+                    else ldgp<PX, PERSIST>(P.qbase + c * vol + off, qb);
+                }
+#pragma unroll
+                for (int a = 0; a < PX; a++) {
+                    R F = addR(Fs[a][c], fmaR(wq[a], qn[a], H1p[a][c]));
+                    if (c > 0) F = fmaR(h[a][d] - hm[a][d], czp, F);
+                    double Rd = -(double)F;
+                    if (c == 1) Rd = s2[a] - (double)F;
+                    if (c == 3 && buoy) Rd = s4[a] - (double)F;
+                    if (c == 4) Rd = s5[a] - (double)F;
+                    if (need_base) qu[c][a] = (P.rk_a * qb[a] + P.rk_b * qs[a]) + P.rk_cdt * Rd;
+                    else qu[c][a] = qs[a] + P.rk_cdt * Rd;
+                }
+            }
         }
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            hm1[c] = h0[c];
-            h0[c] = hp1[c];
+        for (int c = 0; c < 5; c++) {
+            QO *O = qout() + c * vol + off;
+            if (PX == 1 || out1) stp<PX>(O, qu[c]);
+            else *O = (QO)qu[c][0];
+        }
+        if (xim != 0) {
+#pragma unroll
+            for (int a = 0; a < PX; a++) {
+                const int ia = i + a;
+                if (PX > 1 && !(ia <= 3 || (ia >= n1 - 2 && ia <= n1 - 1))) continue;
+                QO *O = qout() + off + a + xim;
+#pragma unroll
+                for (int c = 0; c < 5; c++) O[c * vol] = (QO)qu[c][a];
+            }
+        }
+        // the blow-up test: rho, rho*rhoE - ggM/2 |rho u|^2 (the sign of T), all finite
+        if constexpr (CHK) {
+            if (P.check) {
+#pragma unroll
+                for (int a = 0; a < PX; a++) {
+                    if (a == 1 && !out1) break;
+                    const double tr = qu[0][a] * qu[4][a] -
+                                      P.ggMh * ((qu[1][a] * qu[1][a] + qu[2][a] * qu[2][a]) + qu[3][a] * qu[3][a]);
+                    if (qu[0][a] < 0.0 || (qu[0][a] > 0.0 && tr < 0.0)) flag_blown(P.status, i + a, j, tz, kstep(P));
+                    bool fin = true;
+#pragma unroll
+                    for (int c = 0; c < 5; c++) fin = fin && isfinite(qu[c][a]);
+                    if (!fin) flag_nonfinite(P.status, i + a, j, tz);
+                }
+            }
+        }
+    };
+    // float rings: the own points' RK base of plane m starts its way into shared memory
+    auto fetch_base = [&](int m) {
+        if (!FOLD && need_base && out0) {
+            const double *src = P.qbase + (long long)m * plane + colo;
+#pragma unroll
+            for (int c = 0; c < 5; c++) cp_async_d<PX>(sQB + (c * NT + tid) * PX, src + c * vol);
+        }
+        if (!FOLD && need_base) cp_async_commit();
+    };
+
+    // Iteration t forms the fluxes of plane t and completes plane t-1, whose
+    // wall-normal derivatives need hD(t) and Q, w of plane t+1.  So plane t+1 is
+    // the furthest plane read, each point is converted once, hD shares the
+    // gradients of fD and gD, and no own column is read from memory on the way.
+    // Plane ke is completed after the loop, from its own columns alone.
+    for (int t = kb; t <= ke; t++) {
+        // ---------- A: plane t+1's box is converted, beside the inviscid x/y sums of
+        // plane t; after the barrier, plane t+2's box starts its way in (converted
+        // at the next plane).
+        // No barrier ends the plane, so a warp that has finished plane t goes on to
+        // plane t+1's box wait and conversion while others still run phase E.  What
+        // makes that safe: plane t+2's box goes into the slot of plane t-1, and plane
+        // t-1's RK base over plane t-2's, only after
+        // phase A's barrier, which every thread passes after its phase-E reads of that
+        // slot; and phase E reads no primitive or mu slot, which the next conversion
+        // overwrites.
+        R Fxy[PX][5];
+        if (t > kb) fetch_base(t - 1);
+        bad = !wait_slot(iP) || bad;
+        if (FOLD && need_base) bad = !wait_slot(3) || bad;
+        convert(t + 1, iP, pP, mP, true, &Fxy);
+        if (__syncthreads_or(bad)) { give_up(); return; }
+        if (t < ke) {
+            issue(t + 2, iN);
+            issue_base(t + 1);
+        }
+
+        // ---------- C: viscous flux vectors
+        const R czt = ktab(kCzh, t);
+        const Slot s0 = slot(pZ), sp = slot(pP);
+        R h[PX][4], wn[PX], w0[PX], u0[PX], v0[PX], T0[PX];
+        if (col_ok) {
+            R ux[PX], uy[PX], vx[PX], vy[PX], wx[PX], wy[PX], Tx[PX], Ty[PX], pr[PX], un[PX], vn[PX], Tn[PX], mu[PX], m3[PX];
+            own(sp.U, un); own(sp.V, vn); own(sp.W, wn); own(sp.T, Tn);
+            grad_x(s0.U, ux, u0); grad_y(s0.U, uy);
+            grad_x(s0.V, vx, v0); grad_y(s0.V, vy);
+            grad_x(s0.W, wx, w0); grad_y(s0.W, wy);
+            grad_x(s0.T, Tx, T0); grad_y(s0.T, Ty);
+            mu_p(mZ, iZ, T0, mu, pr);
+            if constexpr (!FOLD) {
+                own(sq(iZ, 3), m3);
+                const R pez = ktab(kPez, t);
+#pragma unroll
+                for (int a = 0; a < PX; a++) qz[a] = (pez * fabs(m3[a])) > C.pez_val * mu[a];
+            }
+            R f[PX][4], g[PX][4];
+#pragma unroll
+            for (int a = 0; a < PX; a++) {
+                const R uz = (un[a] - um1[a]) * czt, vz = (vn[a] - vm1[a]) * czt, wz = (wn[a] - wm1[a]) * czt;
+                const R Tz = (Tn[a] - Tm1[a]) * czt;
+                fd_point(C, mu[a], pr[a], u0[a], v0[a], w0[a], ux[a], vy[a], wz, vx[a], uy[a], wx[a], uz, Tx[a], f[a]);
+                gd_point(C, mu[a], pr[a], u0[a], v0[a], w0[a], ux[a], vy[a], wz, vx[a], uy[a], wy[a], vz, Ty[a], g[a]);
+                visc_fz_vals(C, ux[a], vy[a], wx[a], wy[a], u0[a], v0[a], w0[a], mu[a], pr[a], uz, vz, wz, Tz, h[a]);
+            }
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                R x[PX], y[PX];
+#pragma unroll
+                for (int a = 0; a < PX; a++) { x[a] = f[a][c]; y[a] = g[a][c]; }
+                // fD3 and gD2 are one stress
+                if (c == 1) stp<PX>(sX + (ty + 1) * FP + PX * tx + FO, x);
+                else stp<PX>(sF + ((c > 1 ? c - 1 : c) * TJ + ty) * FP + PX * tx + FO, x);
+                if (c > 0) stp<PX>(sG + ((c - 1) * (TJ + 2) + ty + 1) * TI + PX * tx, y);
+            }
+        }
+        {
+            const R *MU = smu(mZ), *RHO = sq(iZ, 0);
+            each_halo([&](int hp) {
+                if (hp < 2 * TJ) {
+                    const int side = hp / TJ, r = hp - side * TJ;
+                    const int ci = side ? i0 + TI : i0 - 1, cj = j0 + r;
+                    if (ci <= n1 && cj <= n2) {
+                        R f[4];
+                        visc_fx<BX, R>(C, s0, sH[hp], sH[NHL + hp], sp, MU, RHO, hbox(hp), czt, f);
+#pragma unroll
+                        for (int c = 0; c < 4; c++) {
+                            const int o = side ? FO + TI : FO - 1;
+                            if (c == 1) sX[(r + 1) * FP + o] = f[c];
+                            else sF[((c > 1 ? c - 1 : c) * TJ + r) * FP + o] = f[c];
+                        }
+                    }
+                } else {
+                    const int side = (hp - 2 * TJ) / TI, cc = hp - 2 * TJ - side * TI;
+                    const int ci = i0 + cc, cj = side ? j0 + TJ : j0 - 1;
+                    if (ci <= n1 && cj <= n2) {
+                        R g[4];
+                        visc_fy<BX, R>(C, s0, sH[hp], sH[NHL + hp], sp, MU, RHO, hbox(hp), czt, g);
+#pragma unroll
+                        for (int c = 1; c < 4; c++) sG[(c - 1) * S::NGY + (side ? TJ + 1 : 0) * TI + cc] = g[c];
+                        sX[(side ? TJ + 1 : 0) * FP + FO + cc] = g[0];
+                    }
+                }
+            });
+            keep_halo(s0);
+        }
+        __syncthreads();
+        // ---------- E: (FP64: plane t-1 completed;) the flux derivatives of plane t known
+        // so far.  In FP64 the three loops below stay apart: merged, their live values
+        // spill, and with two CTAs' shared memory the L1 has no room for spills.
+        if (t > kb && out0) complete(t - 1, wn, h, true, [&](int c, R qn[PX]) { own(sq(iP, c), qn); });
+        if (col_ok) {
+#pragma unroll
+            for (int a = 0; a < PX; a++) { um1[a] = u0[a]; vm1[a] = v0[a]; Tm1[a] = T0[a]; }
+        }
+        if (out0) {
+            const R s12 = ktab(kS12, t), s12o = ktab(kS12o, t), s8 = ktab(kS8, t);
+            R w[PX][5];
+#pragma unroll
+            for (int a = 0; a < PX; a++) {
+                qk[a] = qz[a];
+                inv_weights(wm2[a], wm1[a], w0[a], wn[a], R(0), qk[a], s8, s12, s12o, w[a]);
+                w4[a] = w[a][4];   // of the QUICK set; the central one needs w(t+2)
+                wm2[a] = wm1[a];
+                wm1[a] = w0[a];
+            }
+            double s2[PX], s4[PX], s5[PX];
+            if constexpr (FOLD) {
+                R r0[PX];
+                own(sq(iZ, 0), r0);
+                source(t, um1, w0, Tm1, r0, s2, s4, s5);
+            }
+#pragma unroll
+            for (int c = 0; c < 5; c++) {
+                const int d = c > 0 ? c - 1 : 0;
+                R qn[PX], q0[PX];
+                own(sq(iP, c), qn);
+                own(sq(iZ, c), q0);
+#pragma unroll
+                for (int a = 0; a < PX; a++) {
+                    R H;
+                    if constexpr (FOLD) {
+                        H = fmaR(w[a][3], qn[a], fmaR(w[a][2], q0[a], w[a][1] * qm1[c][a]));
+                        if (c == 1) H = H - s2[a];
+                        if (c == 3 && buoy) H = H - s4[a];
+                        if (c == 4) H = H - s5[a];
+                        Fs[a][c] = fmaR(-P.rk_cdt, H, Fxy[a][c]);
+                    } else {
+                        H1p[a][c] = H = wsum4(w[a], qm2[c][a], qm1[c][a], q0[a], qn[a]);
+                        Fs[a][c] = Fxy[a][c];
+                        if (c > 0) hm[a][d] = h1[a][d];
+                    }
+                    if (c > 0) h1[a][d] = h[a][d];
+                    qm2[c][a] = qm1[c][a];
+                    qm1[c][a] = q0[a];
+                }
+            }
+#pragma unroll
+            for (int c = 1; c < 5; c++) {
+                // fD2, fD3, fD4, fD5 and gD2, gD3, gD4, gD5
+                const R *F = (c == 2 ? sX + (ty + 1) * FP : sF + ((c > 2 ? c - 2 : c - 1) * TJ + ty) * FP) + PX * tx + FO;
+                const R *G = c == 1 ? sX + ty * FP + PX * tx + FO : sG + ((c - 2) * (TJ + 2) + ty) * TI + PX * tx;
+                const int gs = 2 * (c == 1 ? FP : TI);
+                R F2[PX], gm[PX], gp[PX];
+                if constexpr (PX == 2) {
+                    R x[6];
+                    row(F, x);
+                    F2[0] = x[3] - x[1];
+                    F2[1] = x[4] - x[2];
+                } else {
+                    F2[0] = F[1] - F[-1];
+                }
+                ldp<PX>(G, gm);
+                ldp<PX>(G + gs, gp);
+#pragma unroll
+                for (int a = 0; a < PX; a++) {
+                    if constexpr (FOLD)
+                        Fs[a][c] = fmaR(-P.rk_cdt, fmaR(gp[a] - gm[a], C.hdy, F2[a] * C.hdx), Fs[a][c]);
+                    else
+                        Fs[a][c] = fmaR(gp[a] - gm[a], C.hdy, fmaR(F2[a], C.hdx, Fs[a][c]));
+                }
+            }
+        } else if (col_ok) {
+            // a column whose fD or gD a neighbour reads
+#pragma unroll
+            for (int a = 0; a < PX; a++) wm1[a] = w0[a];
         }
         {
             const int o = iZ;
@@ -1563,18 +1483,48 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
             int x = pZ; pZ = pP; pP = x;
             x = mZ; mZ = mP; mP = x;
         }
-        if (!neb) __syncthreads();
     }
-    if (S::prefetch_base) cp_async_wait<0>();
+    if (!out0) return;
+    // ---------- plane ke completed: hD(ke+1) from the converted plane ke+1 and plane
+    // ke+2 in memory, or the top wall's (its own values in memory, against plane
+    // nP3-1's)
+    R h[PX][4], qn[5][PX], wn[PX] = {};
+    double q[5][PX], u[PX], v[PX], w[PX], T[PX];
+    if (ke + 1 == n3) {
+        center(n3 - 1, q, u, v, w, T);
+#pragma unroll
+        for (int a = 0; a < PX; a++) {
+            double hw[4];
+            hflux_wall(n3, a, u[a], v[a], w[a], T[a], hw);
+#pragma unroll
+            for (int c = 0; c < 4; c++) h[a][c] = (R)hw[c];
+#pragma unroll
+            for (int c = 0; c < 5; c++) qn[c][a] = R(0);
+        }
+    } else {
+        center(ke + 2, q, u, v, w, T);
+        R un[PX], vn[PX], Tn[PX];
+#pragma unroll
+        for (int a = 0; a < PX; a++) {
+            un[a] = (R)u[a]; vn[a] = (R)v[a]; wn[a] = (R)w[a]; Tn[a] = (R)T[a];
+#pragma unroll
+            for (int c = 0; c < 5; c++) qn[c][a] = (R)q[c][a];
+        }
+        hflux(ke + 1, pZ, mZ, iZ, um1, vm1, wm1, Tm1, un, vn, wn, Tn, h);
+    }
+    complete(ke, wn, h, false, [&](int c, R x[PX]) {
+#pragma unroll
+        for (int a = 0; a < PX; a++) x[a] = qn[c][a];
+    });
 }
 
 template <int TI, int TJ, typename QI, typename QO, typename R, bool BUOY>
-__global__ void __launch_bounds__(TI *TJ, StageShape<TI, TJ, R>::minb)
+__global__ void __launch_bounds__(StageShape<TI, TJ, R>::NT, StageShape<TI, TJ, R>::minb)
     k_stage(const KParams P, const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUtensorMap tmb)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    stage_body<TI, TJ, QI, QO, R, BUOY ? 1 : 0, false>(P, &tmq, &tmb, blockIdx.x, blockIdx.y, blockIdx.z,
-                                                          threadIdx.x, threadIdx.y, smem_raw);
+    stage_body<TI, TJ, QI, QO, R, BUOY ? 1 : 0, false>(P, &tmq, &tmb, blockIdx.x, blockIdx.y, blockIdx.z, threadIdx.x,
+                                                       threadIdx.y, smem_raw);
 }
 
 // ---------------------------------------------------------------------------
@@ -1593,7 +1543,8 @@ __device__ __forceinline__ void inner_uvT(const KParams &P, int i, int j, int k,
         u = C[1]; v = C[2]; T = C[5];
         return;
     }
-    const long long o = (long long)k * P.plane + (long long)j * P.px + i;
+    // a periodic duplicate row: its source (the row itself is being written by image blocks)
+    const long long o = (long long)k * P.plane + (long long)wrap_idx(j, n2) * P.px + i;
     const double q0 = qo[o];
 #ifndef CHAN_TRUE_DIV
     const double r = rcp_fast(q0);
@@ -1647,14 +1598,12 @@ constexpr int kWallBX = 32, kWallBY = 8;
 constexpr int kWallHX = kWallBX + 2, kWallHY = kWallBY + 2;
 using WallStage = double[2][6][kWallHY][kWallHX];
 
-// One block's work of the wall kernel: block (bx, by) of wall `wall`,
-// thread (tx, ty), near-wall staging area sp.
-template <typename QT>
-__device__ __forceinline__ void wall_body(const KParams &P, int bx_, int by_, int wall, int tx, int ty, WallStage &sp)
+// One block's work of the wall kernel: block (bx, by) of wall `wall`, by NTH
+// threads, near-wall staging area sp.
+template <typename QT, int NTH>
+__device__ __forceinline__ void wall_body(const KParams &P, int bx_, int by_, int wall, int tid, WallStage &sp)
 {
     const QT *qo = static_cast<const QT *>(P.qout);
-    const int i = bx_ * kWallBX + tx;
-    const int j = by_ * kWallBY + ty;
     const int n1 = P.n1, n2 = P.n2, n3 = P.n3;
     const long long plane = P.plane, vol = P.vol;
     // primitives of the two planes next to the wall on the block's (i,j) tile
@@ -1663,11 +1612,13 @@ __device__ __forceinline__ void wall_body(const KParams &P, int bx_, int by_, in
     {
         const int k2 = wall == 0 ? 2 : n3 - 1, k3 = wall == 0 ? 3 : n3 - 2;
         const int i0 = bx_ * kWallBX - 1, j0 = by_ * kWallBY - 1;
-        for (int e = ty * kWallBX + tx; e < 2 * HX * HY; e += kWallBX * kWallBY) {
+        for (int e = tid; e < 2 * HX * HY; e += NTH) {
             const int pl = e / (HX * HY), r0 = e - pl * HX * HY, by = r0 / HX, bx = r0 - by * HX;
             const int ii = i0 + bx, jj = j0 + by;
             if (ii < 1 || ii > n1 || jj < 1 || jj > n2) continue;
-            const long long o = (long long)(pl == 0 ? k2 : k3) * plane + (long long)jj * P.px + ii;
+            // a periodic duplicate row: its source (the row itself is being written by
+            // the image blocks)
+            const long long o = (long long)(pl == 0 ? k2 : k3) * plane + (long long)wrap_idx(jj, n2) * P.px + ii;
             const double q0 = qo[o], q1 = qo[vol + o], q2 = qo[2 * vol + o];
             const double q3 = qo[3 * vol + o], q4 = qo[4 * vol + o];
 #ifndef CHAN_TRUE_DIV
@@ -1692,95 +1643,147 @@ __device__ __forceinline__ void wall_body(const KParams &P, int bx_, int by_, in
         }
     }
     __syncthreads();
-    if (i > n1 + 1 || j > n2 + 1) return;
     if (frozen(P.status, kstep(P))) return;
     double *W = P.wp + (size_t)wall * 8 * plane;
-    const long long idx = (long long)j * P.px + i;
-    const bool custom = P.wall_custom != 0;
-    double uw = 0.0, vw = 0.0, Tw = wall == 0 ? P.Twb : P.Twt;
-    double muw = wall == 0 ? P.muwb : P.muwt;
-    if (custom) {
-        wall_point<QT>(P, wall, i, j, uw, vw, Tw);
-        if (P.wbc[wall].therm == 1) muw = pow07(Tw);
-    }
-    const double pold = W[6 * plane + idx];
-    const double rho = (P.gM2 * pold) / Tw;   // gama*Mac**2*p/T with the previous p
-    double pnew = pold;
-    if (i >= 2 && i <= n1 - 1 && j >= 2 && j <= n2 - 1) {
-        // neighbours at the two planes next to the wall: k2 (adjacent) and k3
-        const int k2 = wall == 0 ? 2 : n3 - 1, k3 = wall == 0 ? 3 : n3 - 2;
-        const double *c1 = wall == 0 ? P.f1 : P.b1;
-        const double *c2 = wall == 0 ? P.f2 : P.b2;
-        // primitive + mu of one interior point, as calcPrim/calcBC produce them
-        // (staged above); kk selects the plane k2 or k3
-        auto prim = [&](int ii, int jj, int kk, double &r, double &u, double &v, double &w, double &T,
-                        double &p, double &mu) {
-            const int pl = kk == k2 ? 0 : 1;
-            const int bx = ii - bx_ * kWallBX + 1, by = jj - by_ * kWallBY + 1;
-            r = sp[pl][0][by][bx];
-            u = sp[pl][1][by][bx];
-            v = sp[pl][2][by][bx];
-            w = sp[pl][3][by][bx];
-            p = sp[pl][4][by][bx];
-            mu = sp[pl][5][by][bx];
-            T = 0.0;
-        };
-        // wall-point terms c0*mu_w*u_w of the neighbours (zero for a no-slip wall)
-        double t_ip = 0.0, t_im = 0.0, t_jp = 0.0, t_jm = 0.0;
+#pragma unroll 1
+    for (int e = tid; e < kWallBX * kWallBY; e += NTH) {
+        const int i = bx_ * kWallBX + e % kWallBX;
+        const int j = by_ * kWallBY + e / kWallBX;
+        if (i > n1 + 1 || j > n2 + 1) continue;
+        const long long idx = (long long)j * P.px + i;
+        const bool custom = P.wall_custom != 0;
+        double uw = 0.0, vw = 0.0, Tw = wall == 0 ? P.Twb : P.Twt;
+        double muw = wall == 0 ? P.muwb : P.muwt;
         if (custom) {
-            double u, v, T;
-            wall_point<QT>(P, wall, i + 1, j, u, v, T);
-            t_ip = c1[0] * (P.wbc[wall].therm == 1 ? pow07(T) : muw) * u;
-            wall_point<QT>(P, wall, i - 1, j, u, v, T);
-            t_im = c1[0] * (P.wbc[wall].therm == 1 ? pow07(T) : muw) * u;
-            wall_point<QT>(P, wall, i, j + 1, u, v, T);
-            t_jp = c1[0] * (P.wbc[wall].therm == 1 ? pow07(T) : muw) * v;
-            wall_point<QT>(P, wall, i, j - 1, u, v, T);
-            t_jm = c1[0] * (P.wbc[wall].therm == 1 ? pow07(T) : muw) * v;
+            wall_point<QT>(P, wall, i, j, uw, vw, Tw);
+            if (P.wbc[wall].therm == 1) muw = pow07(Tw);
         }
-        double r, u, v, w, T, p, mu;
-        double a2, a3, b2, b3;
-        // d/dx of mu*du/dz
-        prim(i + 1, j, k2, r, u, v, w, T, p, mu); a2 = c1[1] * mu * u;
-        prim(i + 1, j, k3, r, u, v, w, T, p, mu); a3 = c1[2] * mu * u;
-        prim(i - 1, j, k2, r, u, v, w, T, p, mu); b2 = c1[1] * mu * u;
-        prim(i - 1, j, k3, r, u, v, w, T, p, mu); b3 = c1[2] * mu * u;
-        const double dudxdz = (((t_ip + a2) + a3) - ((t_im + b2) + b3)) * P.hdx;
-        prim(i, j + 1, k2, r, u, v, w, T, p, mu); a2 = c1[1] * mu * v;
-        prim(i, j + 1, k3, r, u, v, w, T, p, mu); a3 = c1[2] * mu * v;
-        prim(i, j - 1, k2, r, u, v, w, T, p, mu); b2 = c1[1] * mu * v;
-        prim(i, j - 1, k3, r, u, v, w, T, p, mu); b3 = c1[2] * mu * v;
-        const double dvdydz = (((t_jp + a2) + a3) - ((t_jm + b2) + b3)) * P.hdy;
-        double p2, p3, d2, d3, e2, e3;
-        prim(i, j, k2, r, u, v, w, T, p, mu);
-        d2 = c2[1] * mu * w; e2 = c1[1] * r * (w * w); p2 = p;
-        prim(i, j, k3, r, u, v, w, T, p, mu);
-        d3 = c2[2] * mu * w; e3 = c1[2] * r * (w * w); p3 = p;
-        // the wall-point w terms vanish: w = 0 on every wall
-        const double d2wdz2 = d2 + d3;
-        const double drhow2dz = e2 + e3;
-        const double lhs = P.invRe * ((-dudxdz - dvdydz) + P.two3rd * ((dudxdz + dvdydz) - 2.0 * d2wdz2)) + drhow2dz;
-        pnew = -((lhs + c1[1] * p2) + c1[2] * p3) / c1[0];
+        const double pold = W[6 * plane + idx];
+        const double rho = (P.gM2 * pold) / Tw;   // gama*Mac**2*p/T with the previous p
+        double pnew = pold;
+        if (i >= 2 && i <= n1 - 1 && j >= 2 && j <= n2 - 1) {
+            // neighbours at the two planes next to the wall: k2 (adjacent) and k3
+            const int k2 = wall == 0 ? 2 : n3 - 1, k3 = wall == 0 ? 3 : n3 - 2;
+            const double *c1 = wall == 0 ? P.f1 : P.b1;
+            const double *c2 = wall == 0 ? P.f2 : P.b2;
+            // primitive + mu of one interior point, as calcPrim/calcBC produce them
+            // (staged above); kk selects the plane k2 or k3
+            auto prim = [&](int ii, int jj, int kk, double &r, double &u, double &v, double &w, double &T,
+                            double &p, double &mu) {
+                const int pl = kk == k2 ? 0 : 1;
+                const int bx = ii - bx_ * kWallBX + 1, by = jj - by_ * kWallBY + 1;
+                r = sp[pl][0][by][bx];
+                u = sp[pl][1][by][bx];
+                v = sp[pl][2][by][bx];
+                w = sp[pl][3][by][bx];
+                p = sp[pl][4][by][bx];
+                mu = sp[pl][5][by][bx];
+                T = 0.0;
+            };
+            // wall-point terms c0*mu_w*u_w of the neighbours (zero for a no-slip wall)
+            double t_ip = 0.0, t_im = 0.0, t_jp = 0.0, t_jm = 0.0;
+            if (custom) {
+                double u, v, T;
+                wall_point<QT>(P, wall, i + 1, j, u, v, T);
+                t_ip = c1[0] * (P.wbc[wall].therm == 1 ? pow07(T) : muw) * u;
+                wall_point<QT>(P, wall, i - 1, j, u, v, T);
+                t_im = c1[0] * (P.wbc[wall].therm == 1 ? pow07(T) : muw) * u;
+                wall_point<QT>(P, wall, i, j + 1, u, v, T);
+                t_jp = c1[0] * (P.wbc[wall].therm == 1 ? pow07(T) : muw) * v;
+                wall_point<QT>(P, wall, i, j - 1, u, v, T);
+                t_jm = c1[0] * (P.wbc[wall].therm == 1 ? pow07(T) : muw) * v;
+            }
+            double r, u, v, w, T, p, mu;
+            double a2, a3, b2, b3;
+            // d/dx of mu*du/dz
+            prim(i + 1, j, k2, r, u, v, w, T, p, mu); a2 = c1[1] * mu * u;
+            prim(i + 1, j, k3, r, u, v, w, T, p, mu); a3 = c1[2] * mu * u;
+            prim(i - 1, j, k2, r, u, v, w, T, p, mu); b2 = c1[1] * mu * u;
+            prim(i - 1, j, k3, r, u, v, w, T, p, mu); b3 = c1[2] * mu * u;
+            const double dudxdz = (((t_ip + a2) + a3) - ((t_im + b2) + b3)) * P.hdx;
+            prim(i, j + 1, k2, r, u, v, w, T, p, mu); a2 = c1[1] * mu * v;
+            prim(i, j + 1, k3, r, u, v, w, T, p, mu); a3 = c1[2] * mu * v;
+            prim(i, j - 1, k2, r, u, v, w, T, p, mu); b2 = c1[1] * mu * v;
+            prim(i, j - 1, k3, r, u, v, w, T, p, mu); b3 = c1[2] * mu * v;
+            const double dvdydz = (((t_jp + a2) + a3) - ((t_jm + b2) + b3)) * P.hdy;
+            double p2, p3, d2, d3, e2, e3;
+            prim(i, j, k2, r, u, v, w, T, p, mu);
+            d2 = c2[1] * mu * w; e2 = c1[1] * r * (w * w); p2 = p;
+            prim(i, j, k3, r, u, v, w, T, p, mu);
+            d3 = c2[2] * mu * w; e3 = c1[2] * r * (w * w); p3 = p;
+            // the wall-point w terms vanish: w = 0 on every wall
+            const double d2wdz2 = d2 + d3;
+            const double drhow2dz = e2 + e3;
+            const double lhs = P.invRe * ((-dudxdz - dvdydz) + P.two3rd * ((dudxdz + dvdydz) - 2.0 * d2wdz2)) + drhow2dz;
+            pnew = -((lhs + c1[1] * p2) + c1[2] * p3) / c1[0];
+        }
+        W[0 * plane + idx] = rho;
+        W[1 * plane + idx] = uw;
+        W[2 * plane + idx] = vw;
+        W[3 * plane + idx] = 0.0;
+        W[4 * plane + idx] = custom ? Tw + P.ggMh * ((uw * uw + vw * vw) + 0.0) : Tw;
+        W[5 * plane + idx] = Tw;
+        W[6 * plane + idx] = pnew;
+        W[7 * plane + idx] = muw;
+        if (P.check && i >= 1 && i <= n1 && j >= 1 && j <= n2) {
+            if (rho < 0.0 || Tw < 0.0) flag_blown(P.status, i, j, wall == 0 ? 1 : n3, kstep(P));
+            if (!isfinite(rho) || !isfinite(pnew)) flag_nonfinite(P.status, i, j, wall == 0 ? 1 : n3);
+        }
     }
-    W[0 * plane + idx] = rho;
-    W[1 * plane + idx] = uw;
-    W[2 * plane + idx] = vw;
-    W[3 * plane + idx] = 0.0;
-    W[4 * plane + idx] = custom ? Tw + P.ggMh * ((uw * uw + vw * vw) + 0.0) : Tw;
-    W[5 * plane + idx] = Tw;
-    W[6 * plane + idx] = pnew;
-    W[7 * plane + idx] = muw;
-    if (P.check && i >= 1 && i <= n1 && j >= 1 && j <= n2) {
-        if (rho < 0.0 || Tw < 0.0) flag_blown(P.status, i, j, wall == 0 ? 1 : n3, kstep(P));
-        if (!isfinite(rho) || !isfinite(pnew)) flag_nonfinite(P.status, i, j, wall == 0 ? 1 : n3);
+}
+
+// Periodic images of the stage output in y: the ghost rows 0, 1, nP2, nP2+1 of
+// interior plane k, whole rows (their x images came with the stage), by one block of
+// NTH threads; b < image_blocks splits the row points.  The five variables of a point
+// at once, so that their loads are in flight together.
+constexpr int kImgItems = 512;
+__host__ __device__ __forceinline__ int image_blocks(int n1) { return (4 * (n1 + 2) + kImgItems - 1) / kImgItems; }
+template <typename QT, int NTH>
+__device__ __forceinline__ void image_body(const KParams &P, int k, int b, int tid)
+{
+    if (frozen(P.status, kstep(P))) return;
+    const int n1 = P.n1, n2 = P.n2, px = P.px, n = 4 * (n1 + 2);
+    QT *q = static_cast<QT *>(P.qout) + (long long)k * P.plane;
+#pragma unroll 2
+    for (int e = b * kImgItems + tid; e < min(n, (b + 1) * kImgItems); e += NTH) {
+        const int g = e / (n1 + 2), i = e - g * (n1 + 2);
+        const int j = g < 2 ? g : n2 + g - 2;
+        const QT *r = q + (long long)wrap_idx(j, n2) * px + i;
+        QT *o = q + (long long)j * px + i;
+        QT x[5];
+#pragma unroll
+        for (int c = 0; c < 5; c++) x[c] = r[c * P.vol];
+#pragma unroll
+        for (int c = 0; c < 5; c++) o[c * P.vol] = x[c];
+    }
+}
+
+// Blocks of the launch that follows a stage: first the wall blocks (x, y, wall), then
+// the image blocks of each interior plane.
+__host__ __device__ __forceinline__ int wall_blocks_x(int n1) { return (n1 + 2 + kWallBX - 1) / kWallBX; }
+__host__ __device__ __forceinline__ int wall_blocks_y(int n2) { return (n2 + 2 + kWallBY - 1) / kWallBY; }
+__host__ __device__ __forceinline__ int edge_blocks(int n1, int n2, int n3)
+{
+    return 2 * wall_blocks_x(n1) * wall_blocks_y(n2) + image_blocks(n1) * (n3 - 2);
+}
+template <typename QT, int NTH>
+__device__ __forceinline__ void edge_body(const KParams &P, int b, int tid, WallStage &sp)
+{
+    const int nx = wall_blocks_x(P.n1), ny = wall_blocks_y(P.n2), nw = 2 * nx * ny;
+    if (b < nw) {
+        const int bx = b % nx, r = b / nx;
+        wall_body<QT, NTH>(P, bx, r % ny, r / ny, tid, sp);
+    } else {
+        const int ni = image_blocks(P.n1);
+        image_body<QT, NTH>(P, 2 + (b - nw) / ni, (b - nw) % ni, tid);
     }
 }
 
 template <typename QT>
-__global__ void __launch_bounds__(kWallBX * kWallBY) k_wall(const KParams P)
+__global__ void __launch_bounds__(kWallBX * kWallBY, 4) k_wall(const KParams P)
 {
     __shared__ double sp[2][6][kWallHY][kWallHX];
-    wall_body<QT>(P, blockIdx.x, blockIdx.y, blockIdx.z, threadIdx.x, threadIdx.y, sp);
+    edge_body<QT, kWallBX * kWallBY>(P, blockIdx.x, threadIdx.x, sp);
 }
 
 // ---------------------------------------------------------------------------
@@ -1843,24 +1846,29 @@ __device__ __forceinline__ double warp_sum(double v)
 // pb = n3, n3+1: the wall-shear sum of the bottom, top wall) into
 // part[(pb*S + sub)*23 + c].  Pass 2 adds the S partial sums in a fixed
 // order: the result is deterministic.
+// NTH < kStatThreads threads take the points of kStatThreads in turn, each
+// group of 32 with the same points and the same sums.
 using StatRed = double[kStatThreads / 32][23];
+template <int NTH>
 __device__ __forceinline__ void stats_part_body(const KParams &P, const double *q, int do_moments, int do_tau, int S,
                                                 double *part, int blk, int tid, StatRed &red)
 {
     const int n1 = P.n1, n2 = P.n2, n3 = P.n3;
     const int pb = blk / S, sub = blk - pb * S;
-    const int lane = tid & 31, warp = tid >> 5;
+    const int lane = tid & 31;
     if (frozen(P.status, kstep(P) + 1)) return;
     double *out = part + ((size_t)pb * S + sub) * 23;
     if (pb < n3) {
         if (!do_moments) return;
         const int k = pb + 1;
+#pragma unroll 1
+        for (int v = tid; v < kStatThreads; v += NTH) {
         double acc[23];
 #pragma unroll
         for (int c = 0; c < 23; c++) acc[c] = 0.0;
         const int np = n1 * n2;
 #pragma unroll 2
-        for (int p = sub * kStatThreads + tid; p < np; p += S * kStatThreads) {
+        for (int p = sub * kStatThreads + v; p < np; p += S * kStatThreads) {
             const int jj = p / n1, ii = p - jj * n1;
             double x[7];
             ref_var(P, q, ii + 1, jj + 1, k, x);
@@ -1882,7 +1890,8 @@ __device__ __forceinline__ void stats_part_body(const KParams &P, const double *
 #pragma unroll
         for (int c = 0; c < 23; c++) {
             const double s = warp_sum(acc[c]);
-            if (lane == 0) red[warp][c] = s;
+            if (lane == 0) red[v >> 5][c] = s;
+        }
         }
         __syncthreads();
         if (tid < 23) {
@@ -1897,9 +1906,11 @@ __device__ __forceinline__ void stats_part_body(const KParams &P, const double *
     const double *W = P.wp + (size_t)wall * 8 * P.plane;
     const double *c = wall == 0 ? P.f1 : P.b1;
     const int k2 = wall == 0 ? 2 : n3 - 1, k3 = wall == 0 ? 3 : n3 - 2;
-    double acc = 0.0;
     const int ni = n1 - 2, np = (n1 - 2) * (n2 - 2);
-    for (int p = sub * kStatThreads + tid; p < np; p += S * kStatThreads) {
+#pragma unroll 1
+    for (int v = tid; v < kStatThreads; v += NTH) {
+    double acc = 0.0;
+    for (int p = sub * kStatThreads + v; p < np; p += S * kStatThreads) {
         const int jj = 2 + p / ni, ii = 2 + p % ni;
         const long long o = (long long)jj * P.px + ii;
         const double mu = W[7 * P.plane + o];
@@ -1911,7 +1922,8 @@ __device__ __forceinline__ void stats_part_body(const KParams &P, const double *
         acc += (dwdx + dudz) * P.invRe;
     }
     const double s = warp_sum(acc);
-    if (lane == 0) red[warp][0] = s;
+    if (lane == 0) red[v >> 5][0] = s;
+    }
     __syncthreads();
     if (tid == 0) {
         double t = 0.0;
@@ -1924,7 +1936,7 @@ __global__ void __launch_bounds__(kStatThreads, 3) k_stats_part(const KParams P,
                                                              int do_tau, int S, double *part)
 {
     __shared__ double red[kStatThreads / 32][23];
-    stats_part_body(P, q, do_moments, do_tau, S, part, blockIdx.x, threadIdx.x, red);
+    stats_part_body<kStatThreads>(P, q, do_moments, do_tau, S, part, blockIdx.x, threadIdx.x, red);
 }
 
 // Pass 2: one warp per plane / wall adds the S partial sums in order and
@@ -2401,17 +2413,16 @@ __global__ void k_sgs_div(const KParams P, const float *Y, double gama, double *
     }
 }
 
-// q_out += cdt * S at every stored point of the interior planes (periodic
-// duplicates and ghosts take their image's source)
+// q_out += cdt * S at the interior rows, their periodic images in x included (those
+// in y follow with the wall kernel's image blocks)
 __global__ void k_sgs_apply(const KParams P, double *qo, const double *S, double cdt)
 {
-    const int n1 = P.n1, n2 = P.n2, n3 = P.n3, m1 = n1 - 2, m2 = n2 - 2;
-    const long long n = (long long)m1 * m2 * (n3 - 2);
-    const long long tot = (long long)(n1 + 2) * (n2 + 2) * (n3 - 2);
+    const int n1 = P.n1, m1 = n1 - 2, m2 = P.n2 - 2, w = n1 + 2;
+    const long long n = (long long)m1 * m2 * (P.n3 - 2), tot = (long long)w * m2 * (P.n3 - 2);
     for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < tot; s += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(s % (n1 + 2)), j = (int)((s / (n1 + 2)) % (n2 + 2)), k = 2 + (int)(s / ((long long)(n1 + 2) * (n2 + 2)));
-        const int iu = wrap_any(i, n1), ju = wrap_any(j, n2);
-        const long long src = (((long long)(k - 2) * m2) + (ju - 2)) * m1 + (iu - 2);
+        const int i = (int)(s % w), r = (int)(s / w);       // r: row of S
+        const int j = 2 + r % m2, k = 2 + r / m2;
+        const long long src = (long long)r * m1 + (wrap_any(i, n1) - 2);
         const long long o = (long long)k * P.plane + (long long)j * P.px + i;
         // S rows: rho*u, rho*v, rho*w, rho*E (state variables 1..4)
 #pragma unroll
@@ -2476,7 +2487,7 @@ struct PPhase {
     unsigned long long need;    // member's completed units before this phase may start
     double dt;                  // clock advance
     const CUtensorMap *tm;      // stage: tensor map of the input buffer
-    const CUtensorMap *tmb;     // stage: tensor map of the RK base (tiles that stage it by bulk copy)
+    const CUtensorMap *tmb;     // stage: tensor map of the RK base by tile
     const double *q;            // statistics: the state buffer
     double *part;               // statistics: partial sums
 };
@@ -2518,15 +2529,17 @@ constexpr unsigned long long kDepWaitNs = 1000000000ull;
 template <int TI, int TJ, typename QI, typename QO, typename R>
 __device__ __forceinline__ void pstage(const PPhase &F, const KParams &P, int unit, int tid, unsigned char *smem)
 {
+    using S = StageShape<TI, TJ, R>;
     const int bx = unit % F.nx, r = unit / F.nx, by = r % F.ny, bz = r / F.ny;
-    stage_body<TI, TJ, QI, QO, R, 2, true>(P, F.tm, F.tmb, bx, by, bz, tid % TI, tid / TI, smem);
+    stage_body<TI, TJ, QI, QO, R, 2, true>(P, F.tm, F.tmb, bx, by, bz, tid % S::TX, tid / S::TX, smem);
 }
 
-#ifndef CHAN_PMINB_MIXED
-#define CHAN_PMINB_MIXED 2   // resident CTAs per SM of the mixed-precision persistent kernel (3 spills ~1.3 KB per thread)
-#endif
 template <bool MIXED>
 struct PersistShape {
+    // threads of a persistent CTA: those of the stage units on the 32x8 and 16x16 tiles
+    using R = typename std::conditional<MIXED, float, double>::type;
+    static constexpr int NT = StageShape<32, 8, R>::NT;
+    static_assert(StageShape<16, 16, R>::NT == NT, "both tiles' units have the same threads");
     // dynamic shared memory: the largest unit's, plus the work-item slot
     static constexpr size_t st = MIXED ? (StageShape<32, 8, float>::bytes > StageShape<16, 16, float>::bytes
                                                ? StageShape<32, 8, float>::bytes
@@ -2537,11 +2550,11 @@ struct PersistShape {
     static constexpr size_t wall = sizeof(double) * 2 * 6 * kWallHY * kWallHX;
     static constexpr size_t body = ((st > wall ? st : wall) + 127) / 128 * 128;
     static constexpr size_t bytes = body + 128;
-    static constexpr int minb = MIXED ? CHAN_PMINB_MIXED : 2;
+    static constexpr int minb = 2;
 };
 
 template <bool MIXED>
-__global__ void __launch_bounds__(256, PersistShape<MIXED>::minb) k_ensemble(const PPlan plan)
+__global__ void __launch_bounds__(PersistShape<MIXED>::NT, PersistShape<MIXED>::minb) k_ensemble(const PPlan plan)
 {
     using PS = PersistShape<MIXED>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -2606,21 +2619,22 @@ __global__ void __launch_bounds__(256, PersistShape<MIXED>::minb) k_ensemble(con
             break;
         case kPWall: {
             WallStage &sp = *reinterpret_cast<WallStage *>(smem_raw);
-            const int nb = F.nx * F.ny * 2, b0 = I.unit * F.group, b1 = min(b0 + F.group, nb);
+            const int nb = edge_blocks(P.n1, P.n2, P.n3), b0 = I.unit * F.group, b1 = min(b0 + F.group, nb);
             for (int b = b0; b < b1; b++) {
                 if (b > b0) __syncthreads();   // the staging area is reused
-                const int bx = b % F.nx, r = b / F.nx, by = r % F.ny, wall = r / F.ny;
-                if (F.variant == 0) wall_body<double>(P, bx, by, wall, tid % kWallBX, tid / kWallBX, sp);
-                else wall_body<float>(P, bx, by, wall, tid % kWallBX, tid / kWallBX, sp);
+                if (F.variant == 0) edge_body<double, PS::NT>(P, b, tid, sp);
+                else edge_body<float, PS::NT>(P, b, tid, sp);
             }
             break;
         }
         case kPStatsPart:
-            stats_part_body(P, F.q, 1, 1, F.nx, F.part, I.unit, tid, *reinterpret_cast<StatRed *>(smem_raw));
+            stats_part_body<PS::NT>(P, F.q, 1, 1, F.nx, F.part, I.unit, tid, *reinterpret_cast<StatRed *>(smem_raw));
             break;
         case kPStatsFin: {
-            const int pb = I.unit * 8 + (tid >> 5);
-            if (pb < P.n3 + 2) stats_fin_body(P, 1, 1, F.nx, F.part, pb, tid & 31);
+            for (int w = tid >> 5; w < 8; w += PS::NT / 32) {
+                const int pb = I.unit * 8 + w;
+                if (pb < P.n3 + 2) stats_fin_body(P, 1, 1, F.nx, F.part, pb, tid & 31);
+            }
             break;
         }
         default:

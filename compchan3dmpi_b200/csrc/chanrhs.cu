@@ -24,6 +24,7 @@ namespace {
 using StageFn = void (*)(const chan::KParams, const CUtensorMap, const CUtensorMap);
 struct StageSet {
     int ti, tj;
+    dim3 block[2];     // [FP64, float rings]
     StageFn k[2][4];   // [buoyancy][0 FP64, 1 mixed first stage, 2 mixed middle, 3 mixed last]
     size_t smem, smemf;
 };
@@ -41,6 +42,8 @@ StageSet make_stage_set()
     StageSet s{};
     s.ti = TI_;
     s.tj = TJ_;
+    s.block[0] = dim3(chan::StageShape<TI_, TJ_, double>::TX, TJ_);
+    s.block[1] = dim3(chan::StageShape<TI_, TJ_, float>::TX, TJ_);
     fill_stage_set<TI_, TJ_, false>(s);
     fill_stage_set<TI_, TJ_, true>(s);
     s.smem = chan::StageShape<TI_, TJ_, double>::bytes;
@@ -69,9 +72,7 @@ struct chan_ctx {
     double *q[3] = {nullptr, nullptr, nullptr};   // plain FP64: state and two stage buffers
     float *qf[2] = {nullptr, nullptr};            // mixed precision: the two stage buffers in float
     bool mixed = false;
-    float *tabf = nullptr;                        // per-k tables in float (mixed)
-    double *wp = nullptr, *cs = nullptr, *tabs = nullptr, *stat = nullptr, *dvar = nullptr, *tacc = nullptr;
-    double *hwt = nullptr;   // hD of the top wall plane, staged inside a stage
+    double *wp = nullptr, *cs = nullptr, *tabs = nullptr, *ktab = nullptr, *stat = nullptr, *dvar = nullptr, *tacc = nullptr;
     double *spart = nullptr; // statistics partial sums [(nP3+2)*nsplit][23]
     int nsplit = 1;          // blocks per plane in the statistics pass
     unsigned char *wmask[2] = {nullptr, nullptr};  // wall-BC plug-in arrays (allocated on first use)
@@ -287,6 +288,7 @@ void set_stage(chan_ctx *c, int iter)
             k.rk_mode = 1; k.rk_a = 1.0; k.rk_b = 0.0; k.rk_cdt = dt;
         }
     }
+    k.rk_eps = k.rk_a + (k.rk_b - 1.0);   // exact: both sums are
 }
 
 // stage-kernel launch shape: tile shape and number of k-chunks (0: the
@@ -303,7 +305,7 @@ int set_launch(chan_ctx *c, int tile, int nchunks)
         int sms = 148, occ = 1;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
         const int v = c->mixed ? 2 : 0;
-        CK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ss.k[0][v], ss.ti * ss.tj,
+        CK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ss.k[0][v], ss.block[v != 0].x * ss.tj,
                                                             v == 0 ? ss.smem : ss.smemf));
         if (occ < 1) occ = 1;
         const long long slots = (long long)sms * occ, tiles = (long long)ntx * nty;
@@ -379,9 +381,9 @@ int launch_stage(chan_ctx *c, int iter, bool check, long long step, double time)
     {
         ProfScope ps(c, 0);
         const StageSet &ss = kStageSets[c->tile];
-        dim3 grid(c->ntx, c->nty, c->nchunks), block(ss.ti, ss.tj);
+        dim3 grid(c->ntx, c->nty, c->nchunks);
         const int v = !c->mixed ? 0 : (iter == 1 ? 1 : (last ? 3 : 2));
-        ss.k[c->kp.buoy_on ? 1 : 0][v]<<<grid, block, v == 0 ? ss.smem : ss.smemf, c->stream>>>(
+        ss.k[c->kp.buoy_on ? 1 : 0][v]<<<grid, ss.block[v != 0], v == 0 ? ss.smem : ss.smemf, c->stream>>>(
             c->kp, stage_map(c), c->tmb[c->tile]);
     }
     if (c->closure_on) {
@@ -391,7 +393,7 @@ int launch_stage(chan_ctx *c, int iter, bool check, long long step, double time)
     CK(c, cudaGetLastError());
     {
         ProfScope ps(c, 1);
-        dim3 block(32, 8), grid((c->n1 + 2 + 31) / 32, (c->n2 + 2 + 7) / 8, 2);
+        const int block = chan::kWallBX * chan::kWallBY, grid = chan::edge_blocks(c->n1, c->n2, c->n3);
         if (c->mixed && !last)
             chan::k_wall<float><<<grid, block, 0, c->stream>>>(c->kp);
         else
@@ -686,13 +688,11 @@ int chan_init(const chan_params *p, const double *x3, const double *jac, const d
             if ((r = dalloc(c, &t, (5 * (size_t)c->vol + 1) / 2))) { g_init_error = c->err; chan_free(c); return r; }
             c->qf[b] = reinterpret_cast<float *>(t);
         }
-        double *t = nullptr;
-        if ((r = dalloc(c, &t, (4 * (size_t)(n3 + 2) + 1) / 2))) { g_init_error = c->err; chan_free(c); return r; }
-        c->tabf = reinterpret_cast<float *>(t);
     }
     if ((r = dalloc(c, &c->wp, 2 * 8 * (size_t)c->plane)) || (r = dalloc(c, &c->cs, (size_t)(n3 + 2) * 28)) ||
-        (r = dalloc(c, &c->tabs, 4 * (size_t)(n3 + 2))) || (r = dalloc(c, &c->stat, 23 * (size_t)n3 + 2)) ||
-        (r = dalloc(c, &c->tacc, 23 * (size_t)n3 + 2)) || (r = dalloc(c, &c->hwt, 4 * (size_t)c->plane)) ||
+        (r = dalloc(c, &c->tabs, (size_t)(n3 + 2))) ||
+        (r = dalloc(c, &c->ktab, chan::kTabWords * (size_t)(n3 + 2))) || (r = dalloc(c, &c->stat, 23 * (size_t)n3 + 2)) ||
+        (r = dalloc(c, &c->tacc, 23 * (size_t)n3 + 2)) ||
         (r = dalloc(c, &c->spart, 23 * (size_t)(n3 + 2) * kMaxSplit)) ||
         (r = dalloc(c, &c->dvar, 7 * (size_t)n1 * n2 * n3))) {
         g_init_error = c->err;
@@ -713,17 +713,24 @@ int chan_init(const chan_params *p, const double *x3, const double *jac, const d
     const double Re = p->Re, Mac = p->Mac, gama = p->gama;
     const double dx = p->Lx / (double)(n1 - 1), dy = p->Ly / (double)(n2 - 1), dXi = 2.0 / (double)(n3 - 1);
     const double invdx = 1.0 / dx, invdy = 1.0 / dy, invdXi = 1.0 / dXi;
-    std::vector<double> tab(4 * (size_t)(n3 + 2), 0.0);
+    // the stage kernel's constants per plane (chan::KTab), in its ring type
+    const int kw = chan::kTabWords;
+    std::vector<double> czh((size_t)(n3 + 2), 0.0), kt(kw * (size_t)(n3 + 2), 0.0);
     for (int k = 1; k <= n3; k++) {
-        tab[0 * (n3 + 2) + k] = 0.5 * invdXi * INV[k];
-        tab[1 * (n3 + 2) + k] = (invdXi * INV[k]) / 8.0;
-        tab[2 * (n3 + 2) + k] = (invdXi * INV[k]) * (1.0 / 12.0);
-        tab[3 * (n3 + 2) + k] = (Re * dXi) * JAC[k];
+        czh[k] = 0.5 * invdXi * INV[k];
+        const bool near = k < 3 || k > n3 - 2;
+        double *o = &kt[(size_t)kw * k];
+        o[chan::kCzh] = czh[k];
+        o[chan::kS8] = (invdXi * INV[k]) / 8.0;
+        o[chan::kS12] = near ? czh[k] * 0.125 : (invdXi * INV[k]) * (1.0 / 12.0);
+        o[chan::kS12o] = near ? 0.0 : (invdXi * INV[k]) * (1.0 / 12.0);
+        o[chan::kPez] = near ? -INFINITY : (Re * dXi) * JAC[k];
     }
-    e = cudaMemcpyAsync(c->tabs, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream);
-    std::vector<float> tabf(tab.begin(), tab.end());
-    if (e == cudaSuccess && c->mixed)
-        e = cudaMemcpyAsync(c->tabf, tabf.data(), tabf.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream);
+    const std::vector<float> ktf(kt.begin(), kt.end());
+    e = cudaMemcpyAsync(c->tabs, czh.data(), czh.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(c->ktab, c->mixed ? (const void *)ktf.data() : (const void *)kt.data(),
+                            kt.size() * (c->mixed ? sizeof(float) : sizeof(double)), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) { fail(nullptr, "table upload", e); chan_free(c); return CHAN_ECUDA; }
 
@@ -731,8 +738,8 @@ int chan_init(const chan_params *p, const double *x3, const double *jac, const d
     k.n1 = n1; k.n2 = n2; k.n3 = n3; k.px = c->px; k.NJ = c->NJ;
     k.plane = c->plane; k.vol = c->vol;
     k.wp = c->wp; k.cs = c->cs;
-    k.czh = c->tabs; k.cz8 = c->tabs + (n3 + 2); k.cz12 = c->tabs + 2 * (n3 + 2); k.pez = c->tabs + 3 * (n3 + 2);
-    k.stat = c->stat; k.status = c->status; k.tacc = c->tacc; k.acc_on = 0; k.hwt = c->hwt;
+    k.czh = c->tabs; k.ktab = c->ktab;
+    k.stat = c->stat; k.status = c->status; k.tacc = c->tacc; k.acc_on = 0;
     k.invRe = 1.0 / Re;
     k.ggM = gama * (gama - 1) * (Mac * Mac);
     k.ggMh = k.ggM * 0.5;
@@ -747,7 +754,6 @@ int chan_init(const chan_params *p, const double *x3, const double *jac, const d
     k.pex = Re * dx; k.pey = Re * dy;
     k.PexVal = p->Pe[0]; k.PeyVal = p->Pe[1]; k.pez_val = p->Pe[2];
     k.inv_dz1 = 1.0 / co[12]; k.inv_dzN = 1.0 / co[13];
-    k.tabf = c->tabf;
     k.cd = chan::FluxC<double>{k.invRe, k.ggM, k.two3rd, k.kq, k.inv_gM2, k.hdx, k.hdy, k.sx8, k.sx12, k.sy8,
                                k.sy12, k.pex, k.pey, k.PexVal, k.PeyVal, k.pez_val};
     k.cf = chan::FluxC<float>{(float)k.invRe, (float)k.ggM, (float)k.two3rd, (float)k.kq, (float)k.inv_gM2,
@@ -1674,7 +1680,7 @@ std::string persistent_blocker(const chan_ensemble *e)
     for (chan_ctx *c : e->m) {
         if (c->mixed != mixed) return "members of both precisions";
         if (c->closure_on) return "a member runs with the learned closure";
-        if (c->tile != CHAN_TILE_32x8 && c->tile != CHAN_TILE_16x16) return "a member uses a tile of other than 256 threads";
+        if (c->tile != CHAN_TILE_32x8 && c->tile != CHAN_TILE_16x16) return "a member uses a tile other than 32x8 and 16x16";
     }
     long long recs = 0;
     for (chan_ctx *c : e->m) recs += c->nstage;
@@ -1728,10 +1734,8 @@ int build_persistent(chan_ensemble *e)
                 chan::PPhase w{};
                 w.kind = chan::kPWall;
                 w.variant = (c->mixed && !last) ? 1 : 0;
-                w.nx = (c->n1 + 2 + chan::kWallBX - 1) / chan::kWallBX;
-                w.ny = (c->n2 + 2 + chan::kWallBY - 1) / chan::kWallBY;
                 w.group = 8;
-                w.units = (w.nx * w.ny * 2 + w.group - 1) / w.group;
+                w.units = (chan::edge_blocks(c->n1, c->n2, c->n3) + w.group - 1) / w.group;
                 w.kp = kp0 + it - 1;
                 add(w);
             }
@@ -1789,10 +1793,11 @@ int build_persistent(chan_ensemble *e)
     e->nitems = (long long)items.size();
 
     const void *fn = mixed ? (const void *)chan::k_ensemble<true> : (const void *)chan::k_ensemble<false>;
+    const int nth = mixed ? chan::PersistShape<true>::NT : chan::PersistShape<false>::NT;
     const size_t smem = mixed ? chan::PersistShape<true>::bytes : chan::PersistShape<false>::bytes;
     EK(e, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int occ = 0, sms = 148;
-    EK(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 256, smem));
+    EK(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, nth, smem));
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev);
     e->pgrid = std::max(1, occ) * sms;
 
@@ -1810,9 +1815,9 @@ int build_persistent(chan_ensemble *e)
     if (r == cudaSuccess) r = cudaMemsetAsync(e->dcnt, 0, (n + 1) * sizeof(unsigned long long), e->origin);
     if (r == cudaSuccess) {
         if (mixed)
-            chan::k_ensemble<true><<<e->pgrid, 256, smem, e->origin>>>(plan);
+            chan::k_ensemble<true><<<e->pgrid, nth, smem, e->origin>>>(plan);
         else
-            chan::k_ensemble<false><<<e->pgrid, 256, smem, e->origin>>>(plan);
+            chan::k_ensemble<false><<<e->pgrid, nth, smem, e->origin>>>(plan);
         r = cudaGetLastError();
     }
     cudaGraph_t g = nullptr;
@@ -2080,7 +2085,7 @@ int chan_ensemble_tune(chan_ensemble *e, int32_t reps, double *best_ms)
         for (int t = 0; t < CHAN_NTILES && rc == CHAN_OK; t++)
             for (int d : depth) {
                 if (e->mode == CHAN_ENSEMBLE_PERSISTENT && (t == CHAN_TILE_32x4 || t == CHAN_TILE_32x16))
-                    continue;   // the persistent kernel runs 256-thread CTAs
+                    continue;   // the persistent kernel runs the 32x8 and 16x16 tiles
                 std::vector<int> tt(n, t), cc(n);
                 for (size_t i = 0; i < n; i++) {
                     const int nz = e->m[i]->n3 - 2, dd = std::min(d, nz);
