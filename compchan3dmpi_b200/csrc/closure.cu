@@ -145,78 +145,370 @@ __device__ __forceinline__ void st_bf16x8(unsigned char *base, uint32_t off, con
     *(uint4 *)(base + off) = *(uint4 *)h;
 }
 
-// Shared memory of the MLP kernel (bytes)
-struct MlpSmem {
-    static constexpr int w = 0;                                      // weight images
-    static constexpr int x = w + WImages::bytes;                     // X   [128][16]
-    static constexpr int h1 = x + kTile * kInP * 2;                  // H1  [128][64]
+// ---------------------------------------------------------------------------
+// Training kernel: forward and backward pass over the batch rows, 128 per tile.
+//
+// A tile is a chain of five dependent tensor-core steps with an epilogue between
+// each two, far too little work to fill the tensor cores: the chain's latency and the
+// epilogues' GELUs bound it.  So a CTA (one per SM) runs two tiles at a time, each by
+// a group of 128 threads (thread = row), and a ninth warp issues every MMA, the two
+// groups' steps in turn; one group's epilogue covers the other's products.  Groups
+// and issuer meet on mbarriers (ready: the group's operands are written; done: the
+// step's MMAs are complete), never on a CTA barrier.
+//   step 0: dW1 += dZ1^T X of the previous tile; Z1 = X W1^T
+//   step 1: Z2 = H1 W2^T        step 2: Y = H2 W3^T
+//   step 3: dH2 = dY W3;  dW3^T += H2^T dY
+//   step 4: dH1 = dZ2 W2; dW2 += dZ2^T H1
+// Tensor memory: Z1, Z2 and dH (Y, dH2, dH1 in turn) per group, the weight-gradient
+// sums shared: the one issuing thread's MMAs on them run in order.  The weight
+// gradients read the tiles MN-major, so there are no transposed copies; bias
+// gradients are reduced across the warp by halving exchanges, 31 shuffles for 32
+// columns, into one register per 32.  The sample of a row needs no division: the
+// permutation is affine, so a group's next tile is a fixed step further.
+// 65,536 rows: 197 us in the earlier form (one tile per CTA, transposed copies, 128-bit
+// sample indices, a five-shuffle sum and an atomic per bias column).
+constexpr int kGroups = 2, kTrainThreads = kGroups * kTile + 32;
+struct TrainSmem {
+    static constexpr int x = 0;                                      // X   [2][128][16], alternating by tile
+    static constexpr int h1 = x + 2 * kTile * kInP * 2;              // H1  [128][64]
     static constexpr int h2 = h1 + kTile * kHid * 2;                 // H2  [128][64]
-    static constexpr int dy = h2 + kTile * kHid * 2;                 // dY  [128][16]
-    static constexpr int dz2 = dy + kTile * kOutP * 2;               // dZ2 [128][64]
-    static constexpr int xt = dz2 + kTile * kHid * 2;                // X^T  [16][128]
-    static constexpr int h1t = xt + kInP * kTile * 2;                // H1^T [64][128]
-    static constexpr int h2t = h1t + kHid * kTile * 2;               // H2^T [64][128]
-    static constexpr int gt = h2t + kHid * kTile * 2;                // dY^T / dZ2^T / dZ1^T [128][128]
-    static constexpr int fl = gt + kTile * kTile * 2;                // floats: b1 b2 b3 db1 db2 db3 loss
-    static constexpr int bytes = fl + (64 + 64 + 16 + 64 + 64 + 16 + 4) * 4;
+    static constexpr int dz = h2 + kTile * kHid * 2;                 // dZ2, then dZ1 [128][64]
+    static constexpr int dy = dz + kTile * kHid * 2;                 // dY  [128][16]
+    static constexpr int group = dy + kTile * kOutP * 2;             // bytes of one group's tiles
+    static constexpr int w = kGroups * group;                        // weight images
+    static constexpr int fl = w + WImages::bytes;                    // floats: b1 b2 b3, norm, db1 db2 db3, loss
+    static constexpr int bytes = fl + (64 + 64 + 16 + 44 + 64 + 64 + 16 + 4) * 4;
 };
+constexpr int cZ1 = 0, cZ2 = 64, cdH = 128, cGroup = 192, cdW2 = kGroups * cGroup, cdW1 = cdW2 + 64, cdW3 = cdW1 + 16;
 
-// Shared memory of the inference-only kernel: the forward weight images, X, H1, H2
+// v[i] of every lane summed over the warp; lane l gets the sum of v[l]
+__device__ __forceinline__ float warp_colsum32(float v[32], int lane)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < o; i++) {
+            const float keep = up ? v[i + o] : v[i], give = up ? v[i] : v[i + o];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    return v[0];
+}
+
+__device__ __forceinline__ void red_add4(float *p, float a, float b, float c, float d)
+{
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+__global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams P)
+{
+    using S = TrainSmem;
+    extern __shared__ __align__(128) unsigned char sm[];
+    __shared__ __align__(8) uint64_t ready[kGroups], done[kGroups];
+    __shared__ uint32_t tbase;
+    __shared__ int sfail;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float *fb1 = (float *)(sm + S::fl), *fb2 = fb1 + 64, *fb3 = fb2 + 64, *nrm = fb3 + 16;
+    float *db1 = nrm + 44, *db2 = db1 + 64, *db3 = db2 + 64, *sloss = db3 + 16;
+    unsigned char *sW = sm + S::w;
+    {   // weight images, biases, normalisation
+        const uint4 *src = (const uint4 *)P.wimg;
+        uint4 *dst = (uint4 *)sW;
+        for (int e = tid; e < WImages::bytes / 16; e += kTrainThreads) dst[e] = src[e];
+        if (tid < 64) { fb1[tid] = P.b1[tid]; fb2[tid] = P.b2[tid]; db1[tid] = 0.f; db2[tid] = 0.f; }
+        if (tid < 16) { fb3[tid] = tid < kOut ? P.b3[tid] : 0.f; db3[tid] = 0.f; }
+        if (tid < 44) nrm[tid] = P.xmu[tid];   // xmu, xsd, ymu, ysd in one array
+        if (tid == 0) { sloss[0] = 0.f; sfail = 0; }
+    }
+    if (warp == 0) umma::tmem_alloc(&tbase, 512);
+    if (tid == 0)
+        for (int g = 0; g < kGroups; g++) { umma::mbar_init(&ready[g], kTile); umma::mbar_init(&done[g], 1); }
+    umma::fence_async_smem();
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    const uint32_t tb = tbase;
+    const int ntiles = (int)((P.rows + kTile - 1) / kTile), grid = (int)gridDim.x;
+    // tiles of group g: blockIdx.x + grid * (g + kGroups * it)
+    auto count = [&](int g) {
+        const int t0 = (int)blockIdx.x + grid * g;
+        return t0 < ntiles ? (ntiles - t0 + grid * kGroups - 1) / (grid * kGroups) : 0;
+    };
+    if (warp == kGroups * 4) {
+        // ---- the issuing warp: the groups' steps in turn, group 0 first (it has as many
+        // tiles as group 1 or one more); a group's last step 0 only ends its last tile
+        if (lane == 0) {
+            const int n0 = count(0), n1 = count(1);
+            uint32_t ph[kGroups] = {0, 0};
+            bool acc2 = false, acc1 = false, acc3 = false, ok = true;
+            for (int it = 0; it <= n0 && ok; it++)
+                for (int step = 0; step < 5 && ok; step++)
+                    for (int g = 0; g < kGroups && ok; g++) {
+                        const int n = g == 0 ? n0 : n1;
+                        if (it > n || n == 0 || (it == n && step > 0)) continue;
+                        ok = umma::mbar_wait(&ready[g], ph[g], kWaitLimit);
+                        if (!ok) break;
+                        ph[g] ^= 1u;
+                        umma::fence_after_sync();
+                        unsigned char *T = sm + g * S::group;
+                        unsigned char *X = T + S::x, *H1 = T + S::h1, *H2 = T + S::h2, *dZ = T + S::dz, *dY = T + S::dy;
+                        const uint32_t tz = tb + g * cGroup;
+                        constexpr int xb = kTile * kInP * 2;
+                        if (step == 0) {
+                            if (it > 0) {
+                                umma::gemm_mnmajor(tb + cdW1, dZ, kHid, X + ((it - 1) & 1) * xb, kInP, kTile, acc1);
+                                acc1 = true;
+                            }
+                            if (it < n) umma::gemm_kmajor(tz + cZ1, X + (it & 1) * xb, sW + WImages::w1, kInP, kHid, false);
+                        } else if (step == 1) {
+                            umma::gemm_kmajor(tz + cZ2, H1, sW + WImages::w2, kHid, kHid, false);
+                        } else if (step == 2) {
+                            umma::gemm_kmajor(tz + cdH, H2, sW + WImages::w3, kHid, kOutP, false);
+                        } else if (step == 3) {
+                            umma::gemm_kmajor(tz + cdH, dY, sW + WImages::w3t, kOutP, kHid, false);
+                            umma::gemm_mnmajor(tb + cdW3, H2, kHid, dY, kOutP, kTile, acc3);
+                            acc3 = true;
+                        } else {
+                            umma::gemm_kmajor(tz + cdH, dZ, sW + WImages::w2t, kHid, kHid, false);
+                            umma::gemm_mnmajor(tb + cdW2, dZ, kHid, H1, kHid, kTile, acc2);
+                            acc2 = true;
+                        }
+                        umma::commit(&done[g]);
+                    }
+            if (!ok) atomicExch(&sfail, 1);
+        }
+    } else {
+        const int g = warp >> 2, r = tid & (kTile - 1), wq = warp & 3;
+        unsigned char *T = sm + g * S::group;
+        unsigned char *sH1 = T + S::h1, *sH2 = T + S::h2, *sdZ = T + S::dz, *sdY = T + S::dy;
+        const uint32_t tz = tb + g * cGroup;
+        const int n = count(g);
+        uint32_t ph = 0;
+        bool ok = true;
+        float sb1[2] = {0.f, 0.f}, sb2[2] = {0.f, 0.f}, sb3 = 0.f, loss = 0.f;
+        auto signal = [&]() {   // this thread's operands of the next step are written, its reads of TMEM done
+            umma::fence_async_smem();
+            umma::fence_before_sync();
+            umma::mbar_arrive(&ready[g]);
+        };
+        auto wait = [&]() {   // one verdict per warp, which meets again for the loads from TMEM
+            ok = __all_sync(0xffffffffu, ok && umma::mbar_wait(&done[g], ph, kWaitLimit));
+            ph ^= 1u;
+            umma::fence_after_sync();
+        };
+        // sample of this thread's row, and the step to the group's next tile (mod n samples;
+        // all factors are below 2^32, the products below 2^64)
+        const unsigned long long ns = (unsigned long long)P.n, pa = (unsigned long long)P.perm_a;
+        const long long row0 = ((long long)blockIdx.x + (long long)grid * g) * kTile + r;
+        unsigned long long smp = (pa * ((unsigned long long)(P.row0 + row0) % ns) + (unsigned long long)P.perm_b) % ns;
+        const unsigned long long sstep = (pa * ((unsigned long long)grid * kGroups * kTile % ns)) % ns;
+        long long row = row0;
+        float xr[kIn], tr[kOut];   // raw inputs and targets of the coming tile
+        auto fetch = [&]() {
+            if (row < P.rows) {
+                const float *X = P.X + smp * kIn, *Tg = P.T + smp * kOut;
+#pragma unroll
+                for (int f = 0; f < kIn; f++) xr[f] = X[f];
+#pragma unroll
+                for (int o = 0; o < kOut; o++) tr[o] = Tg[o];
+            } else {
+#pragma unroll
+                for (int f = 0; f < kIn; f++) xr[f] = 0.f;
+#pragma unroll
+                for (int o = 0; o < kOut; o++) tr[o] = 0.f;
+            }
+        };
+        if (n > 0) fetch();
+        for (int it = 0; it < n; it++) {
+            const bool live = row < P.rows;
+            float tgt[kOut];
+            {
+                float xin[kInP];
+#pragma unroll
+                for (int f = 0; f < kInP; f++) xin[f] = (live && f < kIn) ? (xr[f < kIn ? f : 0] - nrm[f < kIn ? f : 0]) / nrm[13 + (f < kIn ? f : 0)] : 0.f;
+                unsigned char *sX = T + S::x + (it & 1) * (kTile * kInP * 2);
+                st_bf16x8(sX, umma::kmaj_off(r, 0, kInP), xin);
+                st_bf16x8(sX, umma::kmaj_off(r, 8, kInP), xin + 8);
+            }
+            signal();
+#pragma unroll
+            for (int o = 0; o < kOut; o++) tgt[o] = live ? (tr[o] - nrm[26 + o]) / nrm[35 + o] : 0.f;
+            row += (long long)grid * kGroups * kTile;
+            smp += sstep;
+            if (smp >= ns) smp -= ns;
+            if (it + 1 < n) fetch();
+            // ---- H1 = gelu(Z1 + b1)
+            wait();
+#pragma unroll 1
+            for (int c = 0; c < kHid; c += 16) {
+                float z[16], h[16];
+                umma::tmem_ld16(umma::lane_addr(tz, wq, cZ1 + c), z);
+#pragma unroll
+                for (int i = 0; i < 16; i++) h[i] = gelu(z[i] + fb1[c + i]);
+                st_bf16x8(sH1, umma::kmaj_off(r, c, kHid), h);
+                st_bf16x8(sH1, umma::kmaj_off(r, c + 8, kHid), h + 8);
+            }
+            signal();
+            // ---- H2 = gelu(Z2 + b2)
+            wait();
+#pragma unroll 1
+            for (int c = 0; c < kHid; c += 16) {
+                float z[16], h[16];
+                umma::tmem_ld16(umma::lane_addr(tz, wq, cZ2 + c), z);
+#pragma unroll
+                for (int i = 0; i < 16; i++) h[i] = gelu(z[i] + fb2[c + i]);
+                st_bf16x8(sH2, umma::kmaj_off(r, c, kHid), h);
+                st_bf16x8(sH2, umma::kmaj_off(r, c + 8, kHid), h + 8);
+            }
+            signal();
+            // ---- loss and dY = 2 (y - t) / (9 rows)
+            wait();
+            {
+                float y[16], dy[32];
+                umma::tmem_ld16(umma::lane_addr(tz, wq, cdH), y);
+#pragma unroll
+                for (int o = 0; o < 32; o++) dy[o] = 0.f;
+#pragma unroll
+                for (int o = 0; o < kOut; o++) {
+                    const float e = live ? (y[o] + fb3[o]) - tgt[o] : 0.f;
+                    loss += e * e;
+                    dy[o] = e * P.inv_count;
+                }
+                st_bf16x8(sdY, umma::kmaj_off(r, 0, kOutP), dy);
+                st_bf16x8(sdY, umma::kmaj_off(r, 8, kOutP), dy + 8);
+                signal();
+                sb3 += warp_colsum32(dy, lane);
+            }
+            // ---- dZ2 = dH2 gelu'(Z2 + b2)
+            wait();
+#pragma unroll
+            for (int hc = 0; hc < 2; hc++) {
+                float d[32];
+#pragma unroll
+                for (int c = 0; c < 32; c += 16) {
+                    float gq[16], z[16];
+                    umma::tmem_ld16(umma::lane_addr(tz, wq, cdH + 32 * hc + c), gq);
+                    umma::tmem_ld16(umma::lane_addr(tz, wq, cZ2 + 32 * hc + c), z);
+#pragma unroll
+                    for (int i = 0; i < 16; i++) d[c + i] = live ? gq[i] * gelu_d(z[i] + fb2[32 * hc + c + i]) : 0.f;
+                    st_bf16x8(sdZ, umma::kmaj_off(r, 32 * hc + c, kHid), d + c);
+                    st_bf16x8(sdZ, umma::kmaj_off(r, 32 * hc + c + 8, kHid), d + c + 8);
+                }
+                if (hc == 1) signal();
+                sb2[hc] += warp_colsum32(d, lane);
+            }
+            // ---- dZ1 = dH1 gelu'(Z1 + b1), over dZ2; its product joins the next step 0
+            wait();
+#pragma unroll
+            for (int hc = 0; hc < 2; hc++) {
+                float d[32];
+#pragma unroll
+                for (int c = 0; c < 32; c += 16) {
+                    float gq[16], z[16];
+                    umma::tmem_ld16(umma::lane_addr(tz, wq, cdH + 32 * hc + c), gq);
+                    umma::tmem_ld16(umma::lane_addr(tz, wq, cZ1 + 32 * hc + c), z);
+#pragma unroll
+                    for (int i = 0; i < 16; i++) d[c + i] = live ? gq[i] * gelu_d(z[i] + fb1[32 * hc + c + i]) : 0.f;
+                    st_bf16x8(sdZ, umma::kmaj_off(r, 32 * hc + c, kHid), d + c);
+                    st_bf16x8(sdZ, umma::kmaj_off(r, 32 * hc + c + 8, kHid), d + c + 8);
+                }
+                sb1[hc] += warp_colsum32(d, lane);
+            }
+            if (!ok) break;
+        }
+        if (n > 0 && ok) {
+            signal();
+            wait();
+        }
+        if (!ok) atomicExch(&sfail, 1);
+        // bias gradients and loss of the CTA
+#pragma unroll
+        for (int hc = 0; hc < 2; hc++) {
+            atomicAdd(&db1[32 * hc + lane], sb1[hc]);
+            atomicAdd(&db2[32 * hc + lane], sb2[hc]);
+        }
+        if (lane < kOut) atomicAdd(&db3[lane], sb3);
+        const float ls = warp_sum(loss);
+        if (lane == 0) atomicAdd(sloss, ls);
+    }
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    if (!sfail && count(0) > 0) {
+        // weight-gradient sums out of tensor memory (lanes 0..63 hold rows): dW2 row o, the
+        // columns split between the groups; dW1 row o; dW3^T row = feature
+        const int g = warp >> 2, wq = warp & 3, o = wq * 32 + lane;
+        if (g < kGroups && wq < 2) {
+            for (int c = 32 * g; c < 32 * g + 32; c += 16) {
+                float v[16];
+                umma::tmem_ld16(umma::lane_addr(tb, wq, cdW2 + c), v);
+#pragma unroll
+                for (int i = 0; i < 16; i += 4) red_add4(&P.gW2[o * kHid + c + i], v[i], v[i + 1], v[i + 2], v[i + 3]);
+            }
+            float v[16];
+            umma::tmem_ld16(umma::lane_addr(tb, wq, g == 0 ? cdW1 : cdW3), v);
+            if (g == 0) {
+#pragma unroll
+                for (int i = 0; i < kIn; i++) atomicAdd(&P.gW1[o * kIn + i], v[i]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < kOut; i++) atomicAdd(&P.gW3[i * kHid + o], v[i]);
+            }
+        }
+        if (tid < 64) { atomicAdd(&P.gb1[tid], db1[tid]); atomicAdd(&P.gb2[tid], db2[tid]); }
+        else if (tid < 64 + kOut) atomicAdd(&P.gb3[tid - 64], db3[tid - 64]);
+        else if (tid == 96) atomicAdd(P.loss, sloss[0]);
+    }
+    if (sfail && tid == 0) {
+        // an MMA did not signal completion: give the groups' barriers one more bounded
+        // wait each before the tensor memory they write is released
+        for (int g = 0; g < kGroups; g++) umma::mbar_wait(&done[g], 0, kWaitLimit);
+        atomicExch(P.err, 1);
+    }
+    umma::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) umma::tmem_free(tb, 512);
+}
+
+// ---------------------------------------------------------------------------
+// Inference: forward only, 128 rows per tile, one CTA of 128 threads per tile in turn.
+// Three dependent products and two GELU epilogues per tile; what hides their latency
+// is other CTAs, so everything is sized for six per SM: 64 tensor-memory columns (Z1,
+// Z2 and Y in turn) and 34 KB of shared memory (H2 over H1).
 struct InferSmem {
     static constexpr int wbytes = WImages::w2t;                      // W1, W2, W3 images
     static constexpr int x = wbytes;
-    static constexpr int h1 = x + kTile * kInP * 2;
-    static constexpr int h2 = h1 + kTile * kHid * 2;
-    static constexpr int fl = h2 + kTile * kHid * 2;
-    static constexpr int bytes = fl + (64 + 64 + 16 + 64 + 64 + 16 + 4) * 4;
+    static constexpr int h = x + kTile * kInP * 2;                   // H1, then H2 [128][64]
+    static constexpr int fl = h + kTile * kHid * 2;                  // floats: b1 b2 b3, norm
+    static constexpr int bytes = fl + (64 + 64 + 16 + 44) * 4;
 };
+constexpr int kInferCtas = 6;
 
-// tensor-memory columns: training holds all 512 (one CTA per SM); inference
-// needs Z1, Z2 and Y, with Y over Z1's columns (128, four CTAs per SM)
-constexpr int cZ1 = 0, cZ2 = 64, cdH2 = 192, cdH1 = 256, cdW3 = 320, cdW2 = 384, cdW1 = 448;
-template <bool TRAIN>
-struct MlpCfg {
-    static constexpr int cY = TRAIN ? 128 : 0, tmem = TRAIN ? 512 : 128, minb = TRAIN ? 1 : 4;
-    static constexpr int wbytes = TRAIN ? WImages::bytes : InferSmem::wbytes;
-    static constexpr int x = TRAIN ? MlpSmem::x : InferSmem::x, h1 = TRAIN ? MlpSmem::h1 : InferSmem::h1,
-                         h2 = TRAIN ? MlpSmem::h2 : InferSmem::h2, fl = TRAIN ? MlpSmem::fl : InferSmem::fl,
-                         bytes = TRAIN ? MlpSmem::bytes : InferSmem::bytes;
-};
-
-// Forward (and for TRAIN the backward) pass over the batch rows, 128 per
-// tile, tiles strided over the grid; one CTA of 128 threads per SM (the CTA
-// holds all 512 tensor-memory columns).  Thread t owns row t of each tile.
-template <bool TRAIN>
-__global__ void __launch_bounds__(128, MlpCfg<TRAIN>::minb) k_mlp(const MlpParams P)
+__global__ void __launch_bounds__(kTile, kInferCtas) k_mlp_infer(const MlpParams P)
 {
-    using G = MlpCfg<TRAIN>;
-    constexpr int cY = G::cY;
+    using S = InferSmem;
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tbase;
     const int tid = threadIdx.x, warp = tid >> 5;
-    float *fb1 = (float *)(sm + G::fl), *fb2 = fb1 + 64, *fb3 = fb2 + 64;
-    float *db1 = fb3 + 16, *db2 = db1 + 64, *db3 = db2 + 64, *sloss = db3 + 16;
-    {   // weight images and biases
+    float *fb1 = (float *)(sm + S::fl), *fb2 = fb1 + 64, *fb3 = fb2 + 64, *nrm = fb3 + 16;
+    {   // weight images, biases, normalisation
         const uint4 *src = (const uint4 *)P.wimg;
-        uint4 *dst = (uint4 *)(sm + MlpSmem::w);
-        for (int e = tid; e < G::wbytes / 16; e += 128) dst[e] = src[e];
-        if (tid < 64) { fb1[tid] = P.b1[tid]; fb2[tid] = P.b2[tid]; db1[tid] = 0.f; db2[tid] = 0.f; }
-        if (tid < 16) { fb3[tid] = tid < kOut ? P.b3[tid] : 0.f; db3[tid] = 0.f; }
-        if (tid == 0) sloss[0] = 0.f;
+        uint4 *dst = (uint4 *)sm;
+        for (int e = tid; e < S::wbytes / 16; e += kTile) dst[e] = src[e];
+        if (tid < 64) { fb1[tid] = P.b1[tid]; fb2[tid] = P.b2[tid]; }
+        if (tid < 16) fb3[tid] = tid < kOut ? P.b3[tid] : 0.f;
+        if (tid < 44) nrm[tid] = P.xmu[tid];   // xmu, xsd, ymu, ysd in one array
     }
-    if (warp == 0) umma::tmem_alloc(&tbase, G::tmem);
+    if (warp == 0) umma::tmem_alloc(&tbase, 64);
     if (tid == 0) umma::mbar_init(&mbar, 1);
     umma::fence_async_smem();
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tb = tbase;
-    unsigned char *sW = sm + MlpSmem::w;
-    unsigned char *sX = sm + G::x, *sH1 = sm + G::h1, *sH2 = sm + G::h2;
-    unsigned char *sdY = sm + MlpSmem::dy, *sdZ2 = sm + MlpSmem::dz2;
-    unsigned char *sXt = sm + MlpSmem::xt, *sH1t = sm + MlpSmem::h1t, *sH2t = sm + MlpSmem::h2t;
-    unsigned char *sGt = sm + MlpSmem::gt;
+    unsigned char *sX = sm + S::x, *sH = sm + S::h;
     uint32_t phase = 0;
     bool ok = true;
     // issue by thread 0 after the smem writes of every thread; then wait
@@ -237,171 +529,49 @@ __global__ void __launch_bounds__(128, MlpCfg<TRAIN>::minb) k_mlp(const MlpParam
         umma::fence_after_sync();
     };
     const long long ntiles = (P.rows + kTile - 1) / kTile;
-    bool first = true;
+    auto layer = [&](const float *b) {
+#pragma unroll 1
+        for (int c = 0; c < kHid; c += 16) {
+            float z[16], h[16];
+            umma::tmem_ld16(umma::lane_addr(tb, warp, c), z);
+#pragma unroll
+            for (int i = 0; i < 16; i++) h[i] = gelu(z[i] + b[c + i]);
+            st_bf16x8(sH, umma::kmaj_off(tid, c, kHid), h);
+            st_bf16x8(sH, umma::kmaj_off(tid, c + 8, kHid), h + 8);
+        }
+    };
     for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
         const long long row = tile * kTile + tid;
         const bool live = row < P.rows;
-        long long sample = 0;
-        if (live) sample = (long long)(((__int128)P.perm_a * (P.row0 + row) + P.perm_b) % P.n);
-        // ---- inputs, normalised, as X and X^T
-        float xin[kInP], tgt[kOut];
+        float xin[kInP];
 #pragma unroll
         for (int f = 0; f < kInP; f++)
-            xin[f] = (live && f < kIn) ? (P.X[sample * P.xr + f * P.xc] - P.xmu[f]) / P.xsd[f] : 0.f;
-        if (TRAIN) {
-#pragma unroll
-            for (int o = 0; o < kOut; o++) tgt[o] = live ? (P.T[sample * kOut + o] - P.ymu[o]) / P.ysd[o] : 0.f;
-        }
+            xin[f] = (live && f < kIn) ? (P.X[row * P.xr + f * P.xc] - nrm[f < kIn ? f : 0]) / nrm[13 + (f < kIn ? f : 0)] : 0.f;
         st_bf16x8(sX, umma::kmaj_off(tid, 0, kInP), xin);
         st_bf16x8(sX, umma::kmaj_off(tid, 8, kInP), xin + 8);
-        if (TRAIN) {
-#pragma unroll
-            for (int f = 0; f < kInP; f++) st_bf16(sXt, umma::kmaj_off(f, tid, kTile), xin[f]);
-        }
-        // ---- F1: Z1 = X W1^T
-        sync_issue_wait([&] { umma::gemm_kmajor(tb + cZ1, sX, sW + WImages::w1, kInP, kHid, false); });
+        sync_issue_wait([&] { umma::gemm_kmajor(tb, sX, sm + WImages::w1, kInP, kHid, false); });
         if (!ok) break;
-        for (int c = 0; c < kHid; c += 16) {
-            float z[16], h[16];
-            umma::tmem_ld16(umma::lane_addr(tb, warp, cZ1 + c), z);
-#pragma unroll
-            for (int i = 0; i < 16; i++) h[i] = gelu(z[i] + fb1[c + i]);
-            st_bf16x8(sH1, umma::kmaj_off(tid, c, kHid), h);
-            st_bf16x8(sH1, umma::kmaj_off(tid, c + 8, kHid), h + 8);
-            if (TRAIN) {
-#pragma unroll
-                for (int i = 0; i < 16; i++) st_bf16(sH1t, umma::kmaj_off(c + i, tid, kTile), h[i]);
-            }
-        }
-        // ---- F2: Z2 = H1 W2^T
-        sync_issue_wait([&] { umma::gemm_kmajor(tb + cZ2, sH1, sW + WImages::w2, kHid, kHid, false); });
+        layer(fb1);
+        sync_issue_wait([&] { umma::gemm_kmajor(tb, sH, sm + WImages::w2, kHid, kHid, false); });
         if (!ok) break;
-        for (int c = 0; c < kHid; c += 16) {
-            float z[16], h[16];
-            umma::tmem_ld16(umma::lane_addr(tb, warp, cZ2 + c), z);
-#pragma unroll
-            for (int i = 0; i < 16; i++) h[i] = gelu(z[i] + fb2[c + i]);
-            st_bf16x8(sH2, umma::kmaj_off(tid, c, kHid), h);
-            st_bf16x8(sH2, umma::kmaj_off(tid, c + 8, kHid), h + 8);
-            if (TRAIN) {
-#pragma unroll
-                for (int i = 0; i < 16; i++) st_bf16(sH2t, umma::kmaj_off(c + i, tid, kTile), h[i]);
-            }
-        }
-        // ---- F3: Y = H2 W3^T
-        sync_issue_wait([&] { umma::gemm_kmajor(tb + cY, sH2, sW + WImages::w3, kHid, kOutP, false); });
+        layer(fb2);
+        sync_issue_wait([&] { umma::gemm_kmajor(tb, sH, sm + WImages::w3, kHid, kOutP, false); });
         if (!ok) break;
         float y[16];
-        umma::tmem_ld16(umma::lane_addr(tb, warp, cY), y);
-#pragma unroll
-        for (int o = 0; o < kOutP; o++) y[o] += fb3[o];
-        if (!TRAIN) {
-            if (live) {
-                bool big = false;
-#pragma unroll
-                for (int o = 0; o < kOut; o++) {
-                    big = big || !(fabsf(y[o]) <= P.out_limit);
-                    P.Y[row * P.yr + o * P.yc] = y[o] * P.ysd[o] + P.ymu[o];
-                }
-                if (big && P.flag) atomicOr(P.flag, 1);
-            }
-            continue;
-        }
-        // ---- loss and dY = 2 (y - t) / (9 rows)
-        float dy[16], l = 0.f;
-#pragma unroll
-        for (int o = 0; o < kOutP; o++) {
-            const float e = (live && o < kOut) ? y[o] - tgt[o] : 0.f;
-            l += e * e;
-            dy[o] = e * P.inv_count;
-        }
-        st_bf16x8(sdY, umma::kmaj_off(tid, 0, kOutP), dy);
-        st_bf16x8(sdY, umma::kmaj_off(tid, 8, kOutP), dy + 8);
-#pragma unroll
-        for (int o = 0; o < kOutP; o++) st_bf16(sGt, umma::kmaj_off(o, tid, kTile), dy[o]);
-        {
-            const float ls = warp_sum(l);
-            if ((tid & 31) == 0) atomicAdd(sloss, ls);
+        umma::tmem_ld16(umma::lane_addr(tb, warp, 0), y);
+        if (live) {
+            bool big = false;
 #pragma unroll
             for (int o = 0; o < kOut; o++) {
-                const float s3 = warp_sum(dy[o]);
-                if ((tid & 31) == 0) atomicAdd(&db3[o], s3);
+                const float v = y[o] + fb3[o];
+                big = big || !(fabsf(v) <= P.out_limit);
+                P.Y[row * P.yr + o * P.yc] = v * nrm[35 + o] + nrm[26 + o];
             }
-        }
-        // ---- B3: dH2 = dY W3 ; G3: dW3 += dY^T H2
-        const bool acc = !first;
-        sync_issue_wait([&] {
-            umma::gemm_kmajor(tb + cdH2, sdY, sW + WImages::w3t, kOutP, kHid, false);
-            umma::gemm_kmajor(tb + cdW3, sGt, sH2t, kTile, kHid, acc);
-        });
-        if (!ok) break;
-        for (int c = 0; c < kHid; c += 16) {
-            float g[16], z[16], d[16];
-            umma::tmem_ld16(umma::lane_addr(tb, warp, cdH2 + c), g);
-            umma::tmem_ld16(umma::lane_addr(tb, warp, cZ2 + c), z);
-#pragma unroll
-            for (int i = 0; i < 16; i++) d[i] = live ? g[i] * gelu_d(z[i] + fb2[c + i]) : 0.f;
-            st_bf16x8(sdZ2, umma::kmaj_off(tid, c, kHid), d);
-            st_bf16x8(sdZ2, umma::kmaj_off(tid, c + 8, kHid), d + 8);
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                st_bf16(sGt, umma::kmaj_off(c + i, tid, kTile), d[i]);
-                const float s2 = warp_sum(d[i]);
-                if ((tid & 31) == 0) atomicAdd(&db2[c + i], s2);
-            }
-        }
-        // ---- B2: dH1 = dZ2 W2 ; G2: dW2 += dZ2^T H1
-        sync_issue_wait([&] {
-            umma::gemm_kmajor(tb + cdH1, sdZ2, sW + WImages::w2t, kHid, kHid, false);
-            umma::gemm_kmajor(tb + cdW2, sGt, sH1t, kTile, kHid, acc);
-        });
-        if (!ok) break;
-        for (int c = 0; c < kHid; c += 16) {
-            float g[16], z[16];
-            umma::tmem_ld16(umma::lane_addr(tb, warp, cdH1 + c), g);
-            umma::tmem_ld16(umma::lane_addr(tb, warp, cZ1 + c), z);
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const float d = live ? g[i] * gelu_d(z[i] + fb1[c + i]) : 0.f;
-                st_bf16(sGt, umma::kmaj_off(c + i, tid, kTile), d);
-                const float s1 = warp_sum(d);
-                if ((tid & 31) == 0) atomicAdd(&db1[c + i], s1);
-            }
-        }
-        // ---- G1: dW1 += dZ1^T X
-        sync_issue_wait([&] { umma::gemm_kmajor(tb + cdW1, sGt, sXt, kTile, kInP, acc); });
-        first = false;
-    }
-    if (TRAIN && ok && !first) {
-        // weight-gradient sums out of tensor memory: lane = output feature
-        const int o = tid;
-        for (int c = 0; c < kHid; c += 16) {
-            float v[16];
-            umma::tmem_ld16(umma::lane_addr(tb, warp, cdW3 + c), v);
-            if (o < kOut) {
-#pragma unroll
-                for (int i = 0; i < 16; i++) atomicAdd(&P.gW3[o * kHid + c + i], v[i]);
-            }
-            umma::tmem_ld16(umma::lane_addr(tb, warp, cdW2 + c), v);
-            if (o < kHid) {
-#pragma unroll
-                for (int i = 0; i < 16; i++) atomicAdd(&P.gW2[o * kHid + c + i], v[i]);
-            }
-        }
-        float v[16];
-        umma::tmem_ld16(umma::lane_addr(tb, warp, cdW1), v);
-        if (o < kHid) {
-#pragma unroll
-            for (int i = 0; i < kIn; i++) atomicAdd(&P.gW1[o * kIn + i], v[i]);
+            if (big && P.flag) atomicOr(P.flag, 1);
         }
     }
     umma::fence_before_sync();
     __syncthreads();
-    if (TRAIN) {
-        if (tid < 64) { atomicAdd(&P.gb1[tid], db1[tid]); atomicAdd(&P.gb2[tid], db2[tid]); }
-        if (tid < kOut) atomicAdd(&P.gb3[tid], db3[tid]);
-        if (tid == 0) atomicAdd(P.loss, sloss[0]);
-    }
     if (!ok) {
         // an MMA did not signal completion: give it one more bounded wait
         // before the tensor memory it writes is released
@@ -411,46 +581,54 @@ __global__ void __launch_bounds__(128, MlpCfg<TRAIN>::minb) k_mlp(const MlpParam
         }
         __syncthreads();
     }
-    if (warp == 0) umma::tmem_free(tb, G::tmem);
+    if (warp == 0) umma::tmem_free(tb, 64);
 }
 
-// Adam on the F32 master parameters, then the BF16 weight images.
+// Adam on the F32 master parameters, with the BF16 weight images.
 // Parameter vector: W1[64][13] b1[64] W2[64][64] b2[64] W3[9][64] b3[9].
 constexpr int kNW1 = kHid * kIn, kNW2 = kHid * kHid, kNW3 = kOut * kHid;
 constexpr int kOffB1 = kNW1, kOffW2 = kOffB1 + kHid, kOffB2 = kOffW2 + kNW2, kOffW3 = kOffB2 + kHid,
-              kOffB3 = kOffW3 + kNW3, kNParam = kOffB3 + kOut;
+              kOffB3 = kOffW3 + kNW3, kNParam = kOffB3 + kOut,
+              kPStride = (kNParam + 31) / 32 * 32;   // each of w, m, v, g starts on a 128-byte boundary
 
-__global__ void k_adam(float *w, float *m, float *v, const float *g, int n, float lr, float b1, float b2, float eps,
-                       float c1, float c2)
+// BF16 images of parameter i of the F32 master weights (padding stays zero from the memset)
+__device__ __forceinline__ void put_images(int i, float x, unsigned char *img)
+{
+    if (i < kNW1) {
+        st_bf16(img + WImages::w1, umma::kmaj_off(i / kIn, i % kIn, kInP), x);
+    } else if (i >= kOffW2 && i < kOffW2 + kNW2) {
+        const int j = i - kOffW2, o = j / kHid, f = j % kHid;
+        st_bf16(img + WImages::w2, umma::kmaj_off(o, f, kHid), x);
+        st_bf16(img + WImages::w2t, umma::kmaj_off(f, o, kHid), x);
+    } else if (i >= kOffW3 && i < kOffW3 + kNW3) {
+        const int j = i - kOffW3, o = j / kHid, f = j % kHid;
+        st_bf16(img + WImages::w3, umma::kmaj_off(o, f, kHid), x);
+        st_bf16(img + WImages::w3t, umma::kmaj_off(f, o, kOutP), x);
+    }
+}
+
+// one Adam step of every parameter, its BF16 images, and its gradient sum back to zero
+// for the next step: one launch where a memset, the update and the images were three
+__global__ void k_adam(float *w, float *m, float *v, float *g, unsigned char *img, float lr, float b1, float b2,
+                       float eps, float c1, float c2)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= kNParam) return;
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.f - b1) * gi;
     const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    g[i] = 0.f;
+    const float x = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    w[i] = x;
+    put_images(i, x, img);
 }
 
-// BF16 images of the F32 master weights (padding stays zero from the memset)
 __global__ void k_weight_images(const float *w, unsigned char *img)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kNW1) {
-        const int o = i / kIn, f = i % kIn;
-        st_bf16(img + WImages::w1, umma::kmaj_off(o, f, kInP), w[i]);
-    } else if (i < kNW1 + kNW2) {
-        const int j = i - kNW1, o = j / kHid, f = j % kHid;
-        const float x = w[kOffW2 + j];
-        st_bf16(img + WImages::w2, umma::kmaj_off(o, f, kHid), x);
-        st_bf16(img + WImages::w2t, umma::kmaj_off(f, o, kHid), x);
-    } else if (i < kNW1 + kNW2 + kNW3) {
-        const int j = i - kNW1 - kNW2, o = j / kHid, f = j % kHid;
-        const float x = w[kOffW3 + j];
-        st_bf16(img + WImages::w3, umma::kmaj_off(o, f, kHid), x);
-        st_bf16(img + WImages::w3t, umma::kmaj_off(f, o, kOutP), x);
-    }
+    if (i < kNParam) put_images(i, w[i], img);
 }
 
 // column sums and sums of squares of an [n][ncol] array (double atomics)
@@ -543,7 +721,7 @@ MlpParams base_params(chan_closure *m)
 
 int refresh_images(chan_closure *m)
 {
-    k_weight_images<<<(kNW1 + kNW2 + kNW3 + 255) / 256, 256, 0, m->stream>>>(m->w, m->img);
+    k_weight_images<<<(kNParam + 255) / 256, 256, 0, m->stream>>>(m->w, m->img);
     CLK(m, cudaGetLastError());
     return CHAN_OK;
 }
@@ -551,11 +729,11 @@ int refresh_images(chan_closure *m)
 int launch_mlp(chan_closure *m, const MlpParams &P, bool train, cudaStream_t st)
 {
     const long long ntiles = (P.rows + kTile - 1) / kTile;
-    const long long slots = (long long)m->sms * (train ? MlpCfg<true>::minb : MlpCfg<false>::minb);
+    const long long slots = (long long)m->sms * (train ? 1 : kInferCtas);
     const int grid = (int)(ntiles < slots ? ntiles : slots);
     if (grid < 1) return CHAN_OK;
-    if (train) k_mlp<true><<<grid, 128, MlpCfg<true>::bytes, st>>>(P);
-    else k_mlp<false><<<grid, 128, MlpCfg<false>::bytes, st>>>(P);
+    if (train) k_mlp_train<<<grid, kTrainThreads, TrainSmem::bytes, st>>>(P);
+    else k_mlp_infer<<<grid, kTile, InferSmem::bytes, st>>>(P);
     CLK(m, cudaGetLastError());
     return CHAN_OK;
 }
@@ -629,27 +807,27 @@ int chan_closure_create(int32_t device, int64_t capacity, chan_closure **out)
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess && capacity > 0) e = cudaMalloc((void **)&m->X, (size_t)capacity * kIn * sizeof(float));
     if (e == cudaSuccess && capacity > 0) e = cudaMalloc((void **)&m->T, (size_t)capacity * kOut * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&m->w, 4 * (size_t)kNParam * sizeof(float));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&m->w, 4 * (size_t)kPStride * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&m->img, WImages::bytes);
     if (e == cudaSuccess) e = cudaMalloc((void **)&m->norm, 44 * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&m->loss, sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&m->err, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(m->w, 0, 4 * (size_t)kNParam * sizeof(float));
+    if (e == cudaSuccess) e = cudaMemset(m->w, 0, 4 * (size_t)kPStride * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(m->img, 0, WImages::bytes);
     if (e == cudaSuccess) e = cudaMemset(m->err, 0, sizeof(int));
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mlp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MlpSmem::bytes);
+        e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, TrainSmem::bytes);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mlp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MlpCfg<false>::bytes);
+        e = cudaFuncSetAttribute(k_mlp_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, InferSmem::bytes);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) {
         g_cl_error = std::string("chan_closure_create: ") + cudaGetErrorString(e);
         chan_closure_free(m);
         return CHAN_ECUDA;
     }
-    m->m = m->w + kNParam;
-    m->v = m->m + kNParam;
-    m->g = m->v + kNParam;
+    m->m = m->w + kPStride;
+    m->v = m->m + kPStride;
+    m->g = m->v + kPStride;
     // identity normalisation until one is fitted or set
     float nrm[44];
     for (int i = 0; i < 44; i++) nrm[i] = (i >= 13 && i < 26) || i >= 35 ? 1.f : 0.f;
@@ -764,7 +942,7 @@ int chan_closure_set_params(chan_closure *m, const float *params)
     if (!m || !params) return CHAN_EINVAL;
     CLK(m, cudaSetDevice(m->dev));
     CLK(m, cudaMemcpy(m->w, params, (size_t)kNParam * sizeof(float), cudaMemcpyHostToDevice));
-    CLK(m, cudaMemset(m->m, 0, 2 * (size_t)kNParam * sizeof(float)));
+    CLK(m, cudaMemset(m->m, 0, 2 * (size_t)kPStride * sizeof(float)));
     m->adam_t = 0;
     int r = refresh_images(m);
     if (r) return r;
@@ -786,6 +964,7 @@ int chan_closure_train(chan_closure *m, int32_t epochs, int32_t batch, double lr
     if (m->count < batch) { m->msg = "fewer samples than one batch"; return CHAN_EINVAL; }
     CLK(m, cudaSetDevice(m->dev));
     CLK(m, cudaMemsetAsync(m->err, 0, sizeof(int), m->stream));
+    CLK(m, cudaMemsetAsync(m->g, 0, (size_t)kNParam * sizeof(float), m->stream));   // k_adam leaves it zero
     const long long n = m->count, nb = n / batch;
     uint64_t st = seed;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
@@ -796,7 +975,6 @@ int chan_closure_train(chan_closure *m, int32_t epochs, int32_t batch, double lr
         const long long b = (long long)(splitmix(st) % (uint64_t)n);
         CLK(m, cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
         for (long long bi = 0; bi < nb; bi++) {
-            CLK(m, cudaMemsetAsync(m->g, 0, (size_t)kNParam * sizeof(float), m->stream));
             MlpParams P = base_params(m);
             P.X = m->X; P.T = m->T; P.n = n;
             P.perm_a = a; P.perm_b = b;
@@ -806,11 +984,9 @@ int chan_closure_train(chan_closure *m, int32_t epochs, int32_t batch, double lr
             if (r) return r;
             m->adam_t++;
             const float c1 = 1.f - std::pow(b1, (float)m->adam_t), c2 = 1.f - std::pow(b2, (float)m->adam_t);
-            k_adam<<<(kNParam + 255) / 256, 256, 0, m->stream>>>(m->w, m->m, m->v, m->g, kNParam, (float)lr, b1, b2,
-                                                                   eps, c1, c2);
+            k_adam<<<(kNParam + 255) / 256, 256, 0, m->stream>>>(m->w, m->m, m->v, m->g, m->img, (float)lr, b1, b2, eps,
+                                                                   c1, c2);
             CLK(m, cudaGetLastError());
-            r = refresh_images(m);
-            if (r) return r;
         }
         float l = 0.f;
         CLK(m, cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));

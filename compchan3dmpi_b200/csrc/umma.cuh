@@ -11,6 +11,13 @@
 // two 8-column core matrices along K) is 128 and its stride byte offset
 // (between 8-row groups) is K * 16; step s of the K loop starts 256 * s
 // bytes further in.
+//
+// The same tile read the other way round, as the operand whose K runs along its rows
+// (MN-major): its core matrices are then 8 K rows of 8 contiguous M (or N) elements;
+// the stride byte offset (between 8-element groups along M) is 128, the leading one
+// (between 8-row groups along K) columns * 16, and step s of the K loop starts
+// 2 * s row groups further in.  A weight gradient dW = dZ^T H thus reads dZ and H as
+// the forward and backward passes stored them, without transposed copies.
 #pragma once
 #include <cstdint>
 
@@ -66,6 +73,19 @@ __device__ __forceinline__ void gemm_kmajor(uint32_t d_tmem, const void *A, cons
                  (accumulate || s > 0) ? 1u : 0u);
 }
 
+// D[128][N] (+)= A^T B over K rows: A is K x Ma and B K x N, both row tiles as above
+// read MN-major (Ma = ca columns, of which 128 are read: the D rows beyond ca are
+// garbage, and up to 2 KB beyond the tile are read); issued by the calling thread
+__device__ __forceinline__ void gemm_mnmajor(uint32_t d_tmem, const void *A, int ca, const void *B, int N, int K,
+                                             bool accumulate)
+{
+    const uint32_t a0 = smem_u32(A), b0 = smem_u32(B), la = (uint32_t)ca * 16u, lb = (uint32_t)N * 16u;
+    const uint32_t id = idesc_bf16_f32(128, N) | (1u << 15) | (1u << 16);
+    for (int s = 0; s < K / 16; s++)
+        mma_bf16(d_tmem, sdesc(a0 + 2u * la * s, la, 128u), sdesc(b0 + 2u * lb * s, lb, 128u), id,
+                 (accumulate || s > 0) ? 1u : 0u);
+}
+
 __device__ __forceinline__ void commit(uint64_t *mbar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(mbar))
@@ -97,6 +117,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity, uint3
         if (done) return true;
     }
     return false;
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t *mbar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(mbar)) : "memory");
 }
 
 // generic-proxy shared-memory writes made visible to the tensor core
