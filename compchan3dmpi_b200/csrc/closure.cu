@@ -151,8 +151,8 @@ __device__ __forceinline__ void st_bf16x8(unsigned char *base, uint32_t off, con
 // A tile is a chain of five dependent tensor-core steps with an epilogue between
 // each two, far too little work to fill the tensor cores: the chain's latency and the
 // epilogues' GELUs bound it.  So a CTA (one per SM) runs two tiles at a time, each by
-// a group of 128 threads (thread = row), and a ninth warp issues every MMA, the two
-// groups' steps in turn; one group's epilogue covers the other's products.  Groups
+// a group of 256 threads (two per row, 32 columns each), and one more warp issues every
+// MMA, the two groups' steps in turn; one group's epilogue covers the other's products.  Groups
 // and issuer meet on mbarriers (ready: the group's operands are written; done: the
 // step's MMAs are complete), never on a CTA barrier.
 //   step 0: dW1 += dZ1^T X of the previous tile; Z1 = X W1^T
@@ -163,11 +163,11 @@ __device__ __forceinline__ void st_bf16x8(unsigned char *base, uint32_t off, con
 // sums shared: the one issuing thread's MMAs on them run in order.  The weight
 // gradients read the tiles MN-major, so there are no transposed copies; bias
 // gradients are reduced across the warp by halving exchanges, 31 shuffles for 32
-// columns, into one register per 32.  The sample of a row needs no division: the
+// columns, into one register per thread and layer.  The sample of a row needs no division: the
 // permutation is affine, so a group's next tile is a fixed step further.
 // 65,536 rows: 197 us in the earlier form (one tile per CTA, transposed copies, 128-bit
 // sample indices, a five-shuffle sum and an atomic per bias column).
-constexpr int kGroups = 2, kTrainThreads = kGroups * kTile + 32;
+constexpr int kGroups = 2, kGroupThreads = 2 * kTile, kTrainThreads = kGroups * kGroupThreads + 32;
 struct TrainSmem {
     static constexpr int x = 0;                                      // X   [2][128][16], alternating by tile
     static constexpr int h1 = x + 2 * kTile * kInP * 2;              // H1  [128][64]
@@ -208,6 +208,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
     __shared__ __align__(8) uint64_t ready[kGroups], done[kGroups];
     __shared__ uint32_t tbase;
     __shared__ int sfail;
+    __shared__ float wloss[2][kGroups][4];   // loss sums of a tile's warps, by tile parity and group
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     float *fb1 = (float *)(sm + S::fl), *fb2 = fb1 + 64, *fb3 = fb2 + 64, *nrm = fb3 + 16;
     float *db1 = nrm + 44, *db2 = db1 + 64, *db3 = db2 + 64, *sloss = db3 + 16;
@@ -223,7 +224,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
     }
     if (warp == 0) umma::tmem_alloc(&tbase, 512);
     if (tid == 0)
-        for (int g = 0; g < kGroups; g++) { umma::mbar_init(&ready[g], kTile); umma::mbar_init(&done[g], 1); }
+        for (int g = 0; g < kGroups; g++) { umma::mbar_init(&ready[g], kGroupThreads); umma::mbar_init(&done[g], 1); }
     umma::fence_async_smem();
     umma::fence_before_sync();
     __syncthreads();
@@ -235,13 +236,14 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
         const int t0 = (int)blockIdx.x + grid * g;
         return t0 < ntiles ? (ntiles - t0 + grid * kGroups - 1) / (grid * kGroups) : 0;
     };
-    if (warp == kGroups * 4) {
+    if (warp == kTrainThreads / 32 - 1) {
         // ---- the issuing warp: the groups' steps in turn, group 0 first (it has as many
         // tiles as group 1 or one more); a group's last step 0 only ends its last tile
         if (lane == 0) {
             const int n0 = count(0), n1 = count(1);
             uint32_t ph[kGroups] = {0, 0};
             bool acc2 = false, acc1 = false, acc3 = false, ok = true;
+            float loss = 0.f;   // the CTA's tiles and their warps added in order: reproducible
             for (int it = 0; it <= n0 && ok; it++)
                 for (int step = 0; step < 5 && ok; step++)
                     for (int g = 0; g < kGroups && ok; g++) {
@@ -257,6 +259,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
                         constexpr int xb = kTile * kInP * 2;
                         if (step == 0) {
                             if (it > 0) {
+#pragma unroll
+                                for (int q = 0; q < 4; q++) loss += wloss[(it - 1) & 1][g][q];
                                 umma::gemm_mnmajor(tb + cdW1, dZ, kHid, X + ((it - 1) & 1) * xb, kInP, kTile, acc1);
                                 acc1 = true;
                             }
@@ -277,16 +281,18 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
                         umma::commit(&done[g]);
                     }
             if (!ok) atomicExch(&sfail, 1);
+            sloss[0] = loss;
         }
     } else {
-        const int g = warp >> 2, r = tid & (kTile - 1), wq = warp & 3;
+        // thread: row r of the group's tile, columns 32*half .. 32*half + 31 of each layer
+        const int g = warp >> 3, half = (warp >> 2) & 1, wq = warp & 3, r = wq * 32 + lane, c0 = 32 * half;
         unsigned char *T = sm + g * S::group;
         unsigned char *sH1 = T + S::h1, *sH2 = T + S::h2, *sdZ = T + S::dz, *sdY = T + S::dy;
-        const uint32_t tz = tb + g * cGroup;
+        const uint32_t tz = umma::lane_addr(tb + g * cGroup, wq, 0);
         const int n = count(g);
         uint32_t ph = 0;
         bool ok = true;
-        float sb1[2] = {0.f, 0.f}, sb2[2] = {0.f, 0.f}, sb3 = 0.f, loss = 0.f;
+        float sb1 = 0.f, sb2 = 0.f, sb3 = 0.f;
         auto signal = [&]() {   // this thread's operands of the next step are written, its reads of TMEM done
             umma::fence_async_smem();
             umma::fence_before_sync();
@@ -297,6 +303,33 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
             ph ^= 1u;
             umma::fence_after_sync();
         };
+        // 32 values of this row as BF16 into columns c0.. of a [128][64] tile
+        auto put32 = [&](unsigned char *t, const float *v) {
+#pragma unroll
+            for (int c = 0; c < 32; c += 8) st_bf16x8(t, umma::kmaj_off(r, c0 + c, kHid), v + c);
+        };
+        // h = gelu(z + b) of this thread's columns of a layer
+        auto forward = [&](int cz, const float *b, unsigned char *t) {
+            uint32_t z[32];
+            float h[32];
+            umma::tmem_ld32(tz + cz + c0, z);
+            umma::tmem_wait(z);
+#pragma unroll
+            for (int i = 0; i < 32; i++) h[i] = gelu(__uint_as_float(z[i]) + b[c0 + i]);
+            put32(t, h);
+        };
+        // d = dH gelu'(z + b) of this thread's columns into dZ
+        auto backward = [&](int cz, const float *b, bool live, float d[32]) {
+            uint32_t q[32], z[32];
+            umma::tmem_ld32(tz + cdH + c0, q);
+            umma::tmem_ld32(tz + cz + c0, z);
+            umma::tmem_wait(q);
+            umma::tmem_wait(z);
+#pragma unroll
+            for (int i = 0; i < 32; i++)
+                d[i] = live ? __uint_as_float(q[i]) * gelu_d(__uint_as_float(z[i]) + b[c0 + i]) : 0.f;
+            put32(sdZ, d);
+        };
         // sample of this thread's row, and the step to the group's next tile (mod n samples;
         // all factors are below 2^32, the products below 2^64)
         const unsigned long long ns = (unsigned long long)P.n, pa = (unsigned long long)P.perm_a;
@@ -304,32 +337,26 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
         unsigned long long smp = (pa * ((unsigned long long)(P.row0 + row0) % ns) + (unsigned long long)P.perm_b) % ns;
         const unsigned long long sstep = (pa * ((unsigned long long)grid * kGroups * kTile % ns)) % ns;
         long long row = row0;
-        float xr[kIn], tr[kOut];   // raw inputs and targets of the coming tile
+        // raw inputs 8*half .. and (half 0) targets of the coming tile
+        float xr[8], tr[kOut];
         auto fetch = [&]() {
-            if (row < P.rows) {
-                const float *X = P.X + smp * kIn, *Tg = P.T + smp * kOut;
 #pragma unroll
-                for (int f = 0; f < kIn; f++) xr[f] = X[f];
+            for (int f = 0; f < 8; f++) xr[f] = row < P.rows && 8 * half + f < kIn ? P.X[smp * kIn + 8 * half + f] : 0.f;
 #pragma unroll
-                for (int o = 0; o < kOut; o++) tr[o] = Tg[o];
-            } else {
-#pragma unroll
-                for (int f = 0; f < kIn; f++) xr[f] = 0.f;
-#pragma unroll
-                for (int o = 0; o < kOut; o++) tr[o] = 0.f;
-            }
+            for (int o = 0; o < kOut; o++) tr[o] = row < P.rows && half == 0 ? P.T[smp * kOut + o] : 0.f;
         };
         if (n > 0) fetch();
         for (int it = 0; it < n; it++) {
             const bool live = row < P.rows;
             float tgt[kOut];
             {
-                float xin[kInP];
+                float xin[8];
 #pragma unroll
-                for (int f = 0; f < kInP; f++) xin[f] = (live && f < kIn) ? (xr[f < kIn ? f : 0] - nrm[f < kIn ? f : 0]) / nrm[13 + (f < kIn ? f : 0)] : 0.f;
-                unsigned char *sX = T + S::x + (it & 1) * (kTile * kInP * 2);
-                st_bf16x8(sX, umma::kmaj_off(r, 0, kInP), xin);
-                st_bf16x8(sX, umma::kmaj_off(r, 8, kInP), xin + 8);
+                for (int f = 0; f < 8; f++) {
+                    const int i = 8 * half + f;
+                    xin[f] = live && i < kIn ? (xr[f] - nrm[min(i, kIn - 1)]) / nrm[13 + min(i, kIn - 1)] : 0.f;
+                }
+                st_bf16x8(T + S::x + (it & 1) * (kTile * kInP * 2), umma::kmaj_off(r, 8 * half, kInP), xin);
             }
             signal();
 #pragma unroll
@@ -338,83 +365,43 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
             smp += sstep;
             if (smp >= ns) smp -= ns;
             if (it + 1 < n) fetch();
-            // ---- H1 = gelu(Z1 + b1)
             wait();
-#pragma unroll 1
-            for (int c = 0; c < kHid; c += 16) {
-                float z[16], h[16];
-                umma::tmem_ld16(umma::lane_addr(tz, wq, cZ1 + c), z);
-#pragma unroll
-                for (int i = 0; i < 16; i++) h[i] = gelu(z[i] + fb1[c + i]);
-                st_bf16x8(sH1, umma::kmaj_off(r, c, kHid), h);
-                st_bf16x8(sH1, umma::kmaj_off(r, c + 8, kHid), h + 8);
-            }
+            forward(cZ1, fb1, sH1);
             signal();
-            // ---- H2 = gelu(Z2 + b2)
             wait();
-#pragma unroll 1
-            for (int c = 0; c < kHid; c += 16) {
-                float z[16], h[16];
-                umma::tmem_ld16(umma::lane_addr(tz, wq, cZ2 + c), z);
-#pragma unroll
-                for (int i = 0; i < 16; i++) h[i] = gelu(z[i] + fb2[c + i]);
-                st_bf16x8(sH2, umma::kmaj_off(r, c, kHid), h);
-                st_bf16x8(sH2, umma::kmaj_off(r, c + 8, kHid), h + 8);
-            }
+            forward(cZ2, fb2, sH2);
             signal();
-            // ---- loss and dY = 2 (y - t) / (9 rows)
+            // ---- loss and dY = 2 (y - t) / (9 rows), by the first half
             wait();
-            {
-                float y[16], dy[32];
-                umma::tmem_ld16(umma::lane_addr(tz, wq, cdH), y);
+            if (half == 0) {
+                float y[16], dy[32], l = 0.f;
+                umma::tmem_ld16(tz + cdH, y);
 #pragma unroll
                 for (int o = 0; o < 32; o++) dy[o] = 0.f;
 #pragma unroll
                 for (int o = 0; o < kOut; o++) {
                     const float e = live ? (y[o] + fb3[o]) - tgt[o] : 0.f;
-                    loss += e * e;
+                    l += e * e;
                     dy[o] = e * P.inv_count;
                 }
+                l = warp_sum(l);
+                if (lane == 0) wloss[it & 1][g][wq] = l;
                 st_bf16x8(sdY, umma::kmaj_off(r, 0, kOutP), dy);
                 st_bf16x8(sdY, umma::kmaj_off(r, 8, kOutP), dy + 8);
                 signal();
                 sb3 += warp_colsum32(dy, lane);
+            } else {
+                signal();
             }
-            // ---- dZ2 = dH2 gelu'(Z2 + b2)
+            float d[32];
             wait();
-#pragma unroll
-            for (int hc = 0; hc < 2; hc++) {
-                float d[32];
-#pragma unroll
-                for (int c = 0; c < 32; c += 16) {
-                    float gq[16], z[16];
-                    umma::tmem_ld16(umma::lane_addr(tz, wq, cdH + 32 * hc + c), gq);
-                    umma::tmem_ld16(umma::lane_addr(tz, wq, cZ2 + 32 * hc + c), z);
-#pragma unroll
-                    for (int i = 0; i < 16; i++) d[c + i] = live ? gq[i] * gelu_d(z[i] + fb2[32 * hc + c + i]) : 0.f;
-                    st_bf16x8(sdZ, umma::kmaj_off(r, 32 * hc + c, kHid), d + c);
-                    st_bf16x8(sdZ, umma::kmaj_off(r, 32 * hc + c + 8, kHid), d + c + 8);
-                }
-                if (hc == 1) signal();
-                sb2[hc] += warp_colsum32(d, lane);
-            }
-            // ---- dZ1 = dH1 gelu'(Z1 + b1), over dZ2; its product joins the next step 0
+            backward(cZ2, fb2, live, d);
+            signal();
+            sb2 += warp_colsum32(d, lane);
+            // ---- dZ1 over dZ2; its product joins the next step 0
             wait();
-#pragma unroll
-            for (int hc = 0; hc < 2; hc++) {
-                float d[32];
-#pragma unroll
-                for (int c = 0; c < 32; c += 16) {
-                    float gq[16], z[16];
-                    umma::tmem_ld16(umma::lane_addr(tz, wq, cdH + 32 * hc + c), gq);
-                    umma::tmem_ld16(umma::lane_addr(tz, wq, cZ1 + 32 * hc + c), z);
-#pragma unroll
-                    for (int i = 0; i < 16; i++) d[c + i] = live ? gq[i] * gelu_d(z[i] + fb1[32 * hc + c + i]) : 0.f;
-                    st_bf16x8(sdZ, umma::kmaj_off(r, 32 * hc + c, kHid), d + c);
-                    st_bf16x8(sdZ, umma::kmaj_off(r, 32 * hc + c + 8, kHid), d + c + 8);
-                }
-                sb1[hc] += warp_colsum32(d, lane);
-            }
+            backward(cZ1, fb1, live, d);
+            sb1 += warp_colsum32(d, lane);
             if (!ok) break;
         }
         if (n > 0 && ok) {
@@ -423,37 +410,31 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
         }
         if (!ok) atomicExch(&sfail, 1);
         // bias gradients and loss of the CTA
-#pragma unroll
-        for (int hc = 0; hc < 2; hc++) {
-            atomicAdd(&db1[32 * hc + lane], sb1[hc]);
-            atomicAdd(&db2[32 * hc + lane], sb2[hc]);
-        }
-        if (lane < kOut) atomicAdd(&db3[lane], sb3);
-        const float ls = warp_sum(loss);
-        if (lane == 0) atomicAdd(sloss, ls);
+        atomicAdd(&db1[c0 + lane], sb1);
+        atomicAdd(&db2[c0 + lane], sb2);
+        if (half == 0 && lane < kOut) atomicAdd(&db3[lane], sb3);
     }
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
     if (!sfail && count(0) > 0) {
-        // weight-gradient sums out of tensor memory (lanes 0..63 hold rows): dW2 row o, the
-        // columns split between the groups; dW1 row o; dW3^T row = feature
-        const int g = warp >> 2, wq = warp & 3, o = wq * 32 + lane;
-        if (g < kGroups && wq < 2) {
-            for (int c = 32 * g; c < 32 * g + 32; c += 16) {
-                float v[16];
-                umma::tmem_ld16(umma::lane_addr(tb, wq, cdW2 + c), v);
-#pragma unroll
-                for (int i = 0; i < 16; i += 4) red_add4(&P.gW2[o * kHid + c + i], v[i], v[i + 1], v[i + 2], v[i + 3]);
-            }
+        // weight-gradient sums out of tensor memory (lanes 0..63 hold rows): dW2 row o, 16
+        // columns per four warps; dW1 row o; dW3^T row = feature
+        const int part = warp >> 2, wq = warp & 3, o = wq * 32 + lane;
+        if (part < 4 && wq < 2) {
             float v[16];
-            umma::tmem_ld16(umma::lane_addr(tb, wq, g == 0 ? cdW1 : cdW3), v);
-            if (g == 0) {
+            umma::tmem_ld16(umma::lane_addr(tb, wq, cdW2 + 16 * part), v);
 #pragma unroll
-                for (int i = 0; i < kIn; i++) atomicAdd(&P.gW1[o * kIn + i], v[i]);
-            } else {
+            for (int i = 0; i < 16; i += 4) red_add4(&P.gW2[o * kHid + 16 * part + i], v[i], v[i + 1], v[i + 2], v[i + 3]);
+            if (part < 2) {
+                umma::tmem_ld16(umma::lane_addr(tb, wq, part == 0 ? cdW1 : cdW3), v);
+                if (part == 0) {
 #pragma unroll
-                for (int i = 0; i < kOut; i++) atomicAdd(&P.gW3[i * kHid + o], v[i]);
+                    for (int i = 0; i < kIn; i++) atomicAdd(&P.gW1[o * kIn + i], v[i]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < kOut; i++) atomicAdd(&P.gW3[i * kHid + o], v[i]);
+                }
             }
         }
         if (tid < 64) { atomicAdd(&P.gb1[tid], db1[tid]); atomicAdd(&P.gb2[tid], db2[tid]); }
@@ -531,13 +512,15 @@ __global__ void __launch_bounds__(kTile, kInferCtas) k_mlp_infer(const MlpParams
     const long long ntiles = (P.rows + kTile - 1) / kTile;
     auto layer = [&](const float *b) {
 #pragma unroll 1
-        for (int c = 0; c < kHid; c += 16) {
-            float z[16], h[16];
-            umma::tmem_ld16(umma::lane_addr(tb, warp, c), z);
+        for (int c = 0; c < kHid; c += 32) {
+            uint32_t z[32];
+            float h[32];
+            umma::tmem_ld32(umma::lane_addr(tb, warp, c), z);
+            umma::tmem_wait(z);
 #pragma unroll
-            for (int i = 0; i < 16; i++) h[i] = gelu(z[i] + b[c + i]);
-            st_bf16x8(sH, umma::kmaj_off(tid, c, kHid), h);
-            st_bf16x8(sH, umma::kmaj_off(tid, c + 8, kHid), h + 8);
+            for (int i = 0; i < 32; i++) h[i] = gelu(__uint_as_float(z[i]) + b[c + i]);
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) st_bf16x8(sH, umma::kmaj_off(tid, c + i, kHid), h + i);
         }
     };
     for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
