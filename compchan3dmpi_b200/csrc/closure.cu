@@ -96,7 +96,7 @@ struct MlpParams {
     long long row0, rows;        // batch rows [row0, row0 + rows)
     float *Y;                    // outputs (raw units), inference only: Y[row * yr + o * yc]
     long long xr, xc, yr, yc;    // element strides of X and Y (rows, columns)
-    float *gW1, *gW2, *gW3, *gb1, *gb2, *gb3;   // gradient sums (training)
+    float *part;                 // gradient sums of each CTA, [CTA][kPartStride] (training)
     float *loss;                 // sum of squared normalised errors (training)
     float inv_count;             // 2 / (9 * rows): d loss / d y factor
     float out_limit;             // inference: |normalised output| above this sets *flag
@@ -181,6 +181,17 @@ struct TrainSmem {
 };
 constexpr int cZ1 = 0, cZ2 = 64, cdH = 128, cGroup = 192, cdW2 = kGroups * cGroup, cdW1 = cdW2 + 64, cdW3 = cdW1 + 16;
 
+// One CTA's gradient sums: W1 and W2 by input column, 64 outputs each (the lanes that
+// hold a column write it in one go), then W3, b1, b2, b3 as in the parameter vector.
+constexpr int kPartW2 = kIn * kHid, kPartW3 = kPartW2 + kHid * kHid, kPartB1 = kPartW3 + kOut * kHid,
+              kPartB2 = kPartB1 + kHid, kPartB3 = kPartB2 + kHid, kPartN = kPartB3 + kOut,
+              kPartStride = (kPartN + 31) / 32 * 32;
+
+// a kernel launched with programmatic serialisation: the kernels before it are complete
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// the next kernel of the stream may be launched (it still waits before it reads)
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // v[i] of every lane summed over the warp; lane l gets the sum of v[l]
 __device__ __forceinline__ float warp_colsum32(float v[32], int lane)
 {
@@ -196,11 +207,6 @@ __device__ __forceinline__ float warp_colsum32(float v[32], int lane)
     return v[0];
 }
 
-__device__ __forceinline__ void red_add4(float *p, float a, float b, float c, float d)
-{
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
 __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams P)
 {
     using S = TrainSmem;
@@ -213,18 +219,24 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
     float *fb1 = (float *)(sm + S::fl), *fb2 = fb1 + 64, *fb3 = fb2 + 64, *nrm = fb3 + 16;
     float *db1 = nrm + 44, *db2 = db1 + 64, *db3 = db2 + 64, *sloss = db3 + 16;
     unsigned char *sW = sm + S::w;
-    {   // weight images, biases, normalisation
+    grid_dep_launch();
+    if (warp == 0) umma::tmem_alloc(&tbase, 512);
+    if (tid == 0) {
+        for (int g = 0; g < kGroups; g++) { umma::mbar_init(&ready[g], kGroupThreads); umma::mbar_init(&done[g], 1); }
+        sloss[0] = 0.f;
+        sfail = 0;
+    }
+    if (tid < 44) nrm[tid] = P.xmu[tid];   // xmu, xsd, ymu, ysd in one array
+    if (tid < 64) { db1[tid] = 0.f; db2[tid] = 0.f; }
+    if (tid < 16) db3[tid] = 0.f;
+    grid_dep_wait();   // the optimiser step before: weight images and biases
+    {
         const uint4 *src = (const uint4 *)P.wimg;
         uint4 *dst = (uint4 *)sW;
         for (int e = tid; e < WImages::bytes / 16; e += kTrainThreads) dst[e] = src[e];
-        if (tid < 64) { fb1[tid] = P.b1[tid]; fb2[tid] = P.b2[tid]; db1[tid] = 0.f; db2[tid] = 0.f; }
-        if (tid < 16) { fb3[tid] = tid < kOut ? P.b3[tid] : 0.f; db3[tid] = 0.f; }
-        if (tid < 44) nrm[tid] = P.xmu[tid];   // xmu, xsd, ymu, ysd in one array
-        if (tid == 0) { sloss[0] = 0.f; sfail = 0; }
+        if (tid < 64) { fb1[tid] = P.b1[tid]; fb2[tid] = P.b2[tid]; }
+        if (tid < 16) fb3[tid] = tid < kOut ? P.b3[tid] : 0.f;
     }
-    if (warp == 0) umma::tmem_alloc(&tbase, 512);
-    if (tid == 0)
-        for (int g = 0; g < kGroups; g++) { umma::mbar_init(&ready[g], kGroupThreads); umma::mbar_init(&done[g], 1); }
     umma::fence_async_smem();
     umma::fence_before_sync();
     __syncthreads();
@@ -417,28 +429,31 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
-    if (!sfail && count(0) > 0) {
+    if (!sfail) {
         // weight-gradient sums out of tensor memory (lanes 0..63 hold rows): dW2 row o, 16
-        // columns per four warps; dW1 row o; dW3^T row = feature
+        // columns per four warps; dW1 row o; dW3^T row = feature.  Each CTA writes its own
+        // sums, which the optimiser adds up: as atomics on one array the CTAs' 835,000
+        // took 15 of 53 us
+        float *out = P.part + (size_t)blockIdx.x * kPartStride;
         const int part = warp >> 2, wq = warp & 3, o = wq * 32 + lane;
         if (part < 4 && wq < 2) {
             float v[16];
             umma::tmem_ld16(umma::lane_addr(tb, wq, cdW2 + 16 * part), v);
 #pragma unroll
-            for (int i = 0; i < 16; i += 4) red_add4(&P.gW2[o * kHid + 16 * part + i], v[i], v[i + 1], v[i + 2], v[i + 3]);
+            for (int i = 0; i < 16; i++) out[kPartW2 + (16 * part + i) * kHid + o] = v[i];
             if (part < 2) {
                 umma::tmem_ld16(umma::lane_addr(tb, wq, part == 0 ? cdW1 : cdW3), v);
                 if (part == 0) {
 #pragma unroll
-                    for (int i = 0; i < kIn; i++) atomicAdd(&P.gW1[o * kIn + i], v[i]);
+                    for (int i = 0; i < kIn; i++) out[i * kHid + o] = v[i];
                 } else {
 #pragma unroll
-                    for (int i = 0; i < kOut; i++) atomicAdd(&P.gW3[i * kHid + o], v[i]);
+                    for (int i = 0; i < kOut; i++) out[kPartW3 + i * kHid + o] = v[i];
                 }
             }
         }
-        if (tid < 64) { atomicAdd(&P.gb1[tid], db1[tid]); atomicAdd(&P.gb2[tid], db2[tid]); }
-        else if (tid < 64 + kOut) atomicAdd(&P.gb3[tid - 64], db3[tid - 64]);
+        if (tid < 64) { out[kPartB1 + tid] = db1[tid]; out[kPartB2 + tid] = db2[tid]; }
+        else if (tid < 64 + kOut) out[kPartB3 + tid - 64] = db3[tid - 64];
         else if (tid == 96) atomicAdd(P.loss, sloss[0]);
     }
     if (sfail && tid == 0) {
@@ -590,22 +605,60 @@ __device__ __forceinline__ void put_images(int i, float x, unsigned char *img)
     }
 }
 
-// one Adam step of every parameter, its BF16 images, and its gradient sum back to zero
-// for the next step: one launch where a memset, the update and the images were three
-__global__ void k_adam(float *w, float *m, float *v, float *g, unsigned char *img, float lr, float b1, float b2,
-                       float eps, float c1, float c2)
+// gradient of 32 parameters (partial-layout indices 32*blockIdx.x ..) from the CTAs'
+// sums: eight warps add a share of the CTAs each, warp 0 adds those.  Returns the
+// parameter index of warp 0's lane, or -1.
+constexpr int kSumThreads = 256;
+__device__ __forceinline__ int sum_parts(const float *part, int nparts, float (&acc)[kSumThreads / 32][32], float &g)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kNParam) return;
-    const float gi = g[i];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = blockIdx.x * 32 + lane;
+    float s = 0.f;
+    if (q < kPartN) {
+#pragma unroll 8
+        for (int p = warp; p < nparts; p += kSumThreads / 32) s += part[(size_t)p * kPartStride + q];
+    }
+    acc[warp][lane] = s;
+    __syncthreads();
+    if (warp != 0 || q >= kPartN) return -1;
+    g = 0.f;
+#pragma unroll
+    for (int w = 0; w < kSumThreads / 32; w++) g += acc[w][lane];
+    if (q < kPartW2) return (q % kHid) * kIn + q / kHid;
+    if (q < kPartW3) return kOffW2 + ((q - kPartW2) % kHid) * kHid + (q - kPartW2) / kHid;
+    if (q < kPartB1) return kOffW3 + (q - kPartW3);
+    if (q < kPartB2) return kOffB1 + (q - kPartB1);
+    if (q < kPartB3) return kOffB2 + (q - kPartB2);
+    return kOffB3 + (q - kPartB3);
+}
+constexpr int kSumBlocks = (kPartN + 31) / 32;
+
+// one Adam step of every parameter, with its BF16 images
+__global__ void __launch_bounds__(kSumThreads) k_adam(float *w, float *m, float *v, const float *part, int nparts,
+                                                      unsigned char *img, float lr, float b1, float b2, float eps,
+                                                      float c1, float c2)
+{
+    __shared__ float acc[kSumThreads / 32][32];
+    grid_dep_launch();
+    grid_dep_wait();   // the training kernel's sums
+    float gi;
+    const int i = sum_parts(part, nparts, acc, gi);
+    if (i < 0) return;
     const float mi = b1 * m[i] + (1.f - b1) * gi;
     const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    g[i] = 0.f;
     const float x = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     w[i] = x;
     put_images(i, x, img);
+}
+
+// the gradient itself, in the parameter vector's order
+__global__ void __launch_bounds__(kSumThreads) k_grad_sum(const float *part, int nparts, float *g)
+{
+    __shared__ float acc[kSumThreads / 32][32];
+    float gi;
+    const int i = sum_parts(part, nparts, acc, gi);
+    if (i >= 0) g[i] = gi;
 }
 
 __global__ void k_weight_images(const float *w, unsigned char *img)
@@ -662,6 +715,7 @@ struct chan_closure {
     long long cap = 0, count = 0;
     float *w = nullptr, *m = nullptr, *v = nullptr, *g = nullptr;   // kNParam each
     unsigned char *img = nullptr;           // BF16 weight images
+    float *part = nullptr;                  // gradient sums of the training kernel's CTAs, [sms][kPartStride]
     float *norm = nullptr;                  // xmu[13] xsd[13] ymu[9] ysd[9]
     float *loss = nullptr;
     int *err = nullptr;
@@ -692,8 +746,7 @@ MlpParams base_params(chan_closure *m)
     P.wimg = m->img;
     P.b1 = m->w + kOffB1; P.b2 = m->w + kOffB2; P.b3 = m->w + kOffB3;
     P.xmu = m->norm; P.xsd = m->norm + 13; P.ymu = m->norm + 26; P.ysd = m->norm + 35;
-    P.gW1 = m->g; P.gb1 = m->g + kOffB1; P.gW2 = m->g + kOffW2; P.gb2 = m->g + kOffB2;
-    P.gW3 = m->g + kOffW3; P.gb3 = m->g + kOffB3;
+    P.part = m->part;
     P.loss = m->loss;
     P.err = m->err;
     P.out_limit = m->out_limit;
@@ -709,16 +762,39 @@ int refresh_images(chan_closure *m)
     return CHAN_OK;
 }
 
-int launch_mlp(chan_closure *m, const MlpParams &P, bool train, cudaStream_t st)
+int launch_infer(chan_closure *m, const MlpParams &P, cudaStream_t st)
 {
-    const long long ntiles = (P.rows + kTile - 1) / kTile;
-    const long long slots = (long long)m->sms * (train ? 1 : kInferCtas);
+    const long long ntiles = (P.rows + kTile - 1) / kTile, slots = (long long)m->sms * kInferCtas;
     const int grid = (int)(ntiles < slots ? ntiles : slots);
     if (grid < 1) return CHAN_OK;
-    if (train) k_mlp_train<<<grid, kTrainThreads, TrainSmem::bytes, st>>>(P);
-    else k_mlp_infer<<<grid, kTile, InferSmem::bytes, st>>>(P);
+    k_mlp_infer<<<grid, kTile, InferSmem::bytes, st>>>(P);
     CLK(m, cudaGetLastError());
     return CHAN_OK;
+}
+
+// a launch that may start while the stream's previous kernel still runs: the kernel
+// itself waits (grid_dep_wait) before it reads what that one writes
+template <typename... KArgs, typename... Args>
+cudaError_t launch_early(void (*k)(KArgs...), int grid, int block, size_t smem, cudaStream_t st, Args... args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, KArgs(args)...);
+}
+
+// CTAs of a training launch (one per SM, which is also how many sums m->part holds)
+int train_grid(const chan_closure *m, long long rows)
+{
+    const long long ntiles = (rows + kTile - 1) / kTile;
+    return (int)(ntiles < m->sms ? ntiles : m->sms);
 }
 
 int check_err(chan_closure *m)
@@ -738,7 +814,7 @@ int chan_internal_infer(chan_closure *m, const float *X, float *Y, long long n, 
     MlpParams P = base_params(m);
     P.X = X; P.Y = Y; P.n = n; P.rows = n; P.row0 = 0; P.flag = flag;
     if (soa) { P.xr = 1; P.xc = n; P.yr = 1; P.yc = n; }
-    return launch_mlp(m, P, false, stream);
+    return launch_infer(m, P, stream);
 }
 
 int chan_internal_closure_device(chan_closure *m) { return m ? m->dev : -1; }
@@ -792,6 +868,8 @@ int chan_closure_create(int32_t device, int64_t capacity, chan_closure **out)
     if (e == cudaSuccess && capacity > 0) e = cudaMalloc((void **)&m->T, (size_t)capacity * kOut * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&m->w, 4 * (size_t)kPStride * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&m->img, WImages::bytes);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&m->part, (size_t)m->sms * kPartStride * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&m->norm, 44 * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&m->loss, sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&m->err, sizeof(int));
@@ -802,7 +880,6 @@ int chan_closure_create(int32_t device, int64_t capacity, chan_closure **out)
         e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, TrainSmem::bytes);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_mlp_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, InferSmem::bytes);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) {
         g_cl_error = std::string("chan_closure_create: ") + cudaGetErrorString(e);
         chan_closure_free(m);
@@ -947,7 +1024,6 @@ int chan_closure_train(chan_closure *m, int32_t epochs, int32_t batch, double lr
     if (m->count < batch) { m->msg = "fewer samples than one batch"; return CHAN_EINVAL; }
     CLK(m, cudaSetDevice(m->dev));
     CLK(m, cudaMemsetAsync(m->err, 0, sizeof(int), m->stream));
-    CLK(m, cudaMemsetAsync(m->g, 0, (size_t)kNParam * sizeof(float), m->stream));   // k_adam leaves it zero
     const long long n = m->count, nb = n / batch;
     uint64_t st = seed;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
@@ -963,13 +1039,12 @@ int chan_closure_train(chan_closure *m, int32_t epochs, int32_t batch, double lr
             P.perm_a = a; P.perm_b = b;
             P.row0 = bi * batch; P.rows = batch;
             P.inv_count = 2.f / (9.f * (float)batch);
-            int r = launch_mlp(m, P, true, m->stream);
-            if (r) return r;
+            const int grid = train_grid(m, P.rows);
+            CLK(m, launch_early(k_mlp_train, grid, kTrainThreads, TrainSmem::bytes, m->stream, P));
             m->adam_t++;
             const float c1 = 1.f - std::pow(b1, (float)m->adam_t), c2 = 1.f - std::pow(b2, (float)m->adam_t);
-            k_adam<<<(kNParam + 255) / 256, 256, 0, m->stream>>>(m->w, m->m, m->v, m->g, m->img, (float)lr, b1, b2, eps,
-                                                                   c1, c2);
-            CLK(m, cudaGetLastError());
+            CLK(m, launch_early(k_adam, kSumBlocks, kSumThreads, 0, m->stream, m->w, m->m, m->v, m->part, grid, m->img,
+                                (float)lr, b1, b2, eps, c1, c2));
         }
         float l = 0.f;
         CLK(m, cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
@@ -990,13 +1065,17 @@ int chan_closure_grad(chan_closure *m, const float *X, const float *T, int64_t n
     CLK(m, cudaMalloc((void **)&dT, (size_t)n * kOut * sizeof(float)));
     CLK(m, cudaMemcpy(dX, X, (size_t)n * kIn * sizeof(float), cudaMemcpyHostToDevice));
     CLK(m, cudaMemcpy(dT, T, (size_t)n * kOut * sizeof(float), cudaMemcpyHostToDevice));
-    CLK(m, cudaMemsetAsync(m->g, 0, (size_t)kNParam * sizeof(float), m->stream));
     CLK(m, cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
     CLK(m, cudaMemsetAsync(m->err, 0, sizeof(int), m->stream));
     MlpParams P = base_params(m);
     P.X = dX; P.T = dT; P.n = n; P.rows = n;
     P.inv_count = 2.f / (9.f * (float)n);
-    int r = launch_mlp(m, P, true, m->stream);
+    const int grid = train_grid(m, n);
+    k_mlp_train<<<grid, kTrainThreads, TrainSmem::bytes, m->stream>>>(P);
+    CLK(m, cudaGetLastError());
+    k_grad_sum<<<kSumBlocks, kSumThreads, 0, m->stream>>>(m->part, grid, m->g);
+    CLK(m, cudaGetLastError());
+    int r = CHAN_OK;
     float l = 0.f;
     if (!r) r = check_err(m);
     if (!r && grads) CLK(m, cudaMemcpy(grads, m->g, (size_t)kNParam * sizeof(float), cudaMemcpyDeviceToHost));
@@ -1035,6 +1114,7 @@ void chan_closure_free(chan_closure *m)
     if (m->T) cudaFree(m->T);
     if (m->w) cudaFree(m->w);
     if (m->img) cudaFree(m->img);
+    if (m->part) cudaFree(m->part);
     if (m->norm) cudaFree(m->norm);
     if (m->loss) cudaFree(m->loss);
     if (m->err) cudaFree(m->err);
