@@ -23,6 +23,8 @@
 #include <stdint.h>
 #include <type_traits>
 
+#include "chan_internal.h"
+
 namespace chan {
 
 // Step counter and time of the step being computed, kept on the device for
@@ -1523,6 +1525,7 @@ __global__ void __launch_bounds__(StageShape<TI, TJ, R>::NT, StageShape<TI, TJ, 
     k_stage(const KParams P, const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUtensorMap tmb)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    grid_dep_enter();
     stage_body<TI, TJ, QI, QO, R, BUOY ? 1 : 0, false>(P, &tmq, &tmb, blockIdx.x, blockIdx.y, blockIdx.z, threadIdx.x,
                                                        threadIdx.y, smem_raw);
 }
@@ -1783,6 +1786,7 @@ template <typename QT>
 __global__ void __launch_bounds__(kWallBX * kWallBY, 4) k_wall(const KParams P)
 {
     __shared__ double sp[2][6][kWallHY][kWallHX];
+    grid_dep_enter();
     edge_body<QT, kWallBX * kWallBY>(P, blockIdx.x, threadIdx.x, sp);
 }
 
@@ -1936,6 +1940,7 @@ __global__ void __launch_bounds__(kStatThreads, 3) k_stats_part(const KParams P,
                                                              int do_tau, int S, double *part)
 {
     __shared__ double red[kStatThreads / 32][23];
+    grid_dep_enter();
     stats_part_body<kStatThreads>(P, q, do_moments, do_tau, S, part, blockIdx.x, threadIdx.x, red);
 }
 
@@ -1973,6 +1978,7 @@ __device__ __forceinline__ void stats_fin_body(const KParams &P, int do_moments,
 
 __global__ void k_stats_fin(const KParams P, int do_moments, int do_tau, int S, const double *part)
 {
+    grid_dep_enter();
     stats_fin_body(P, do_moments, do_tau, S, part, blockIdx.x, threadIdx.x);
 }
 
@@ -1998,6 +2004,7 @@ struct DiagParams {
 
 __global__ void __launch_bounds__(kStatThreads) k_diag_ke(const KParams P, const double *q, const DiagParams D)
 {
+    grid_dep_enter();
     __shared__ double red[kStatThreads / 32];
     const int n1 = P.n1, n2 = P.n2;
     const int k = blockIdx.x + 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -2024,6 +2031,7 @@ __global__ void __launch_bounds__(kStatThreads) k_diag_ke(const KParams P, const
 __global__ void __launch_bounds__(kStatThreads) k_diag_fin(const KParams P, const double *q, const DiagParams D,
                                                            double *rec, double time)
 {
+    grid_dep_enter();
     __shared__ double red[kStatThreads / 32];
     const int n1 = P.n1, n2 = P.n2, n3 = P.n3;
     const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -2335,6 +2343,7 @@ struct SgsSampling {
 // statistics step.
 __global__ void k_sgs_sample(const KParams P, const double *q, const SgsSampling S)
 {
+    grid_dep_enter();
     const long long n = (long long)S.ni * S.nj * S.nk;
     const double Lx = 1.0 / P.invdx, Ly = 1.0 / P.invdy;   // dx, dy
     const int n3 = P.n3;
@@ -2388,6 +2397,7 @@ __global__ void k_sgs_sample(const KParams P, const double *q, const SgsSampling
 // (the enthalpy flux gama*rho*u*T of the reference's energy equation).
 __global__ void k_sgs_div(const KParams P, const float *Y, double gama, double *S)
 {
+    grid_dep_enter();
     const int n1 = P.n1, n2 = P.n2, n3 = P.n3, m1 = n1 - 2, m2 = n2 - 2;
     const long long n = (long long)m1 * m2 * (n3 - 2);
     auto at = [&](int i, int j, int k, int c) -> double {
@@ -2417,6 +2427,7 @@ __global__ void k_sgs_div(const KParams P, const float *Y, double gama, double *
 // in y follow with the wall kernel's image blocks)
 __global__ void k_sgs_apply(const KParams P, double *qo, const double *S, double cdt)
 {
+    grid_dep_enter();
     const int n1 = P.n1, m1 = n1 - 2, m2 = P.n2 - 2, w = n1 + 2;
     const long long n = (long long)m1 * m2 * (P.n3 - 2), tot = (long long)w * m2 * (P.n3 - 2);
     for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < tot; s += (long long)gridDim.x * blockDim.x) {

@@ -90,6 +90,7 @@ struct chan_ctx {
     CUtensorMap tmf[CHAN_NTILES][2];
     CUtensorMap tmb[CHAN_NTILES];   // the RK base (the FP64 step state) by tile: box TI x TJ x 1 x 5
     int nstage = 2;
+    bool early = false;      // launch the step's kernels early (chan_internal.h)
     int cur = 0;             // buffer holding the latest state
     bool uploaded = false;
     long long nstep = 0;
@@ -356,12 +357,10 @@ int closure_source(chan_ctx *c)
     S.T = nullptr;
     S.soa = true;
     const long long n = (long long)S.ni * S.nj * S.nk;
-    chan::k_sgs_sample<<<1184, 128, 0, c->stream>>>(c->kp, (const double *)c->kp.qin, S);
-    CK(c, cudaGetLastError());
-    int r = chan_internal_infer(c->cl, c->sgsX, c->sgsY, n, true, c->stream, c->sgsflag);
+    CK(c, launch_kernel(c->early, chan::k_sgs_sample, 1184, 128, 0, c->stream, c->kp, (const double *)c->kp.qin, S));
+    int r = chan_internal_infer(c->cl, c->sgsX, c->sgsY, n, true, c->stream, c->sgsflag, c->early);
     if (r) { c->err = "closure inference"; return r; }
-    chan::k_sgs_div<<<1184, 256, 0, c->stream>>>(c->kp, c->sgsY, c->p.gama, c->sgsS);
-    CK(c, cudaGetLastError());
+    CK(c, launch_kernel(c->early, chan::k_sgs_div, 1184, 256, 0, c->stream, c->kp, c->sgsY, c->p.gama, c->sgsS));
     return CHAN_OK;
 }
 
@@ -383,23 +382,18 @@ int launch_stage(chan_ctx *c, int iter, bool check, long long step, double time)
         const StageSet &ss = kStageSets[c->tile];
         dim3 grid(c->ntx, c->nty, c->nchunks);
         const int v = !c->mixed ? 0 : (iter == 1 ? 1 : (last ? 3 : 2));
-        ss.k[c->kp.buoy_on ? 1 : 0][v]<<<grid, ss.block[v != 0], v == 0 ? ss.smem : ss.smemf, c->stream>>>(
-            c->kp, stage_map(c), c->tmb[c->tile]);
+        CK(c, launch_kernel(c->early, ss.k[c->kp.buoy_on ? 1 : 0][v], grid, ss.block[v != 0],
+                            v == 0 ? ss.smem : ss.smemf, c->stream, c->kp, stage_map(c), c->tmb[c->tile]));
     }
-    if (c->closure_on) {
-        chan::k_sgs_apply<<<1184, 256, 0, c->stream>>>(c->kp, (double *)c->kp.qout, c->sgsS, c->kp.rk_cdt);
-        CK(c, cudaGetLastError());
-    }
-    CK(c, cudaGetLastError());
+    if (c->closure_on)
+        CK(c, launch_kernel(c->early, chan::k_sgs_apply, 1184, 256, 0, c->stream, c->kp, (double *)c->kp.qout, c->sgsS,
+                            c->kp.rk_cdt));
     {
         ProfScope ps(c, 1);
         const int block = chan::kWallBX * chan::kWallBY, grid = chan::edge_blocks(c->n1, c->n2, c->n3);
-        if (c->mixed && !last)
-            chan::k_wall<float><<<grid, block, 0, c->stream>>>(c->kp);
-        else
-            chan::k_wall<double><<<grid, block, 0, c->stream>>>(c->kp);
+        CK(c, launch_kernel(c->early, c->mixed && !last ? chan::k_wall<float> : chan::k_wall<double>, grid, block, 0,
+                            c->stream, c->kp));
     }
-    CK(c, cudaGetLastError());
     return CHAN_OK;
 }
 
@@ -420,11 +414,10 @@ int launch_stats(chan_ctx *c, long long step, int moments, int tau)
 {
     c->kp.step = step;
     ProfScope ps(c, 2);
-    chan::k_stats_part<<<(c->n3 + 2) * c->nsplit, chan::kStatThreads, 0, c->stream>>>(c->kp, c->q[c->cur], moments,
-                                                                                     tau, c->nsplit, c->spart);
-    CK(c, cudaGetLastError());
-    chan::k_stats_fin<<<c->n3 + 2, 32, 0, c->stream>>>(c->kp, moments, tau, c->nsplit, c->spart);
-    CK(c, cudaGetLastError());
+    CK(c, launch_kernel(c->early, chan::k_stats_part, (c->n3 + 2) * c->nsplit, chan::kStatThreads, 0, c->stream, c->kp,
+                        c->q[c->cur], moments, tau, c->nsplit, c->spart));
+    CK(c, launch_kernel(c->early, chan::k_stats_fin, c->n3 + 2, 32, 0, c->stream, c->kp, moments, tau, c->nsplit,
+                        c->spart));
     return CHAN_OK;
 }
 
@@ -432,11 +425,9 @@ int launch_diag(chan_ctx *c, long long step, double time)
 {
     c->kp.step = step;
     double *rec = c->diag_rec + (size_t)(c->diag_count % c->diag_cap) * c->diag_reclen;
-    chan::k_diag_ke<<<c->n3, chan::kStatThreads, 0, c->stream>>>(c->kp, c->q[c->cur], c->dp);
-    CK(c, cudaGetLastError());
-    chan::k_diag_fin<<<1 + 3 * c->dp.nplanes, chan::kStatThreads, 0, c->stream>>>(c->kp, c->q[c->cur], c->dp, rec,
-                                                                                   time);
-    CK(c, cudaGetLastError());
+    CK(c, launch_kernel(c->early, chan::k_diag_ke, c->n3, chan::kStatThreads, 0, c->stream, c->kp, c->q[c->cur], c->dp));
+    CK(c, launch_kernel(c->early, chan::k_diag_fin, 1 + 3 * c->dp.nplanes, chan::kStatThreads, 0, c->stream, c->kp,
+                        c->q[c->cur], c->dp, rec, time));
     c->diag_count++;
     return CHAN_OK;
 }
@@ -448,6 +439,11 @@ int launch_diag(chan_ctx *c, long long step, double time)
 enum StepMode { kLaunch = 0, kCapture = 1, kCountOnly = 2 };
 int enqueue_steps(chan_ctx *c, int nsteps, int mode = kLaunch)
 {
+    {   // early launches, but plain kernel nodes in a captured step and per-kernel times when profiling
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        CK(c, cudaStreamIsCapturing(c->stream, &cap));
+        c->early = mode == kLaunch && !c->prof && cap == cudaStreamCaptureStatusNone;
+    }
     for (int s = 0; s < nsteps; s++) {
         const long long step = c->nstep + 1;
         if (mode == kCapture) {
@@ -477,6 +473,7 @@ int enqueue_steps(chan_ctx *c, int nsteps, int mode = kLaunch)
             }
         }
     }
+    c->early = false;
     return CHAN_OK;
 }
 

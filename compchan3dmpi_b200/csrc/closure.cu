@@ -187,11 +187,6 @@ constexpr int kPartW2 = kIn * kHid, kPartW3 = kPartW2 + kHid * kHid, kPartB1 = k
               kPartB2 = kPartB1 + kHid, kPartB3 = kPartB2 + kHid, kPartN = kPartB3 + kOut,
               kPartStride = (kPartN + 31) / 32 * 32;
 
-// a kernel launched with programmatic serialisation: the kernels before it are complete
-__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// the next kernel of the stream may be launched (it still waits before it reads)
-__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // v[i] of every lane summed over the warp; lane l gets the sum of v[l]
 __device__ __forceinline__ float warp_colsum32(float v[32], int lane)
 {
@@ -489,6 +484,7 @@ __global__ void __launch_bounds__(kTile, kInferCtas) k_mlp_infer(const MlpParams
     __shared__ uint32_t tbase;
     const int tid = threadIdx.x, warp = tid >> 5;
     float *fb1 = (float *)(sm + S::fl), *fb2 = fb1 + 64, *fb3 = fb2 + 64, *nrm = fb3 + 16;
+    grid_dep_enter();
     {   // weight images, biases, normalisation
         const uint4 *src = (const uint4 *)P.wimg;
         uint4 *dst = (uint4 *)sm;
@@ -638,8 +634,7 @@ __global__ void __launch_bounds__(kSumThreads) k_adam(float *w, float *m, float 
                                                       float c1, float c2)
 {
     __shared__ float acc[kSumThreads / 32][32];
-    grid_dep_launch();
-    grid_dep_wait();   // the training kernel's sums
+    grid_dep_enter();   // the training kernel's sums
     float gi;
     const int i = sum_parts(part, nparts, acc, gi);
     if (i < 0) return;
@@ -762,32 +757,13 @@ int refresh_images(chan_closure *m)
     return CHAN_OK;
 }
 
-int launch_infer(chan_closure *m, const MlpParams &P, cudaStream_t st)
+int launch_infer(chan_closure *m, const MlpParams &P, cudaStream_t st, bool early)
 {
     const long long ntiles = (P.rows + kTile - 1) / kTile, slots = (long long)m->sms * kInferCtas;
     const int grid = (int)(ntiles < slots ? ntiles : slots);
     if (grid < 1) return CHAN_OK;
-    k_mlp_infer<<<grid, kTile, InferSmem::bytes, st>>>(P);
-    CLK(m, cudaGetLastError());
+    CLK(m, launch_kernel(early, k_mlp_infer, grid, kTile, InferSmem::bytes, st, P));
     return CHAN_OK;
-}
-
-// a launch that may start while the stream's previous kernel still runs: the kernel
-// itself waits (grid_dep_wait) before it reads what that one writes
-template <typename... KArgs, typename... Args>
-cudaError_t launch_early(void (*k)(KArgs...), int grid, int block, size_t smem, cudaStream_t st, Args... args)
-{
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, KArgs(args)...);
 }
 
 // CTAs of a training launch (one per SM, which is also how many sums m->part holds)
@@ -809,12 +785,12 @@ int check_err(chan_closure *m)
 }  // namespace
 
 int chan_internal_infer(chan_closure *m, const float *X, float *Y, long long n, bool soa, cudaStream_t stream,
-                        int *flag)
+                        int *flag, bool early)
 {
     MlpParams P = base_params(m);
     P.X = X; P.Y = Y; P.n = n; P.rows = n; P.row0 = 0; P.flag = flag;
     if (soa) { P.xr = 1; P.xc = n; P.yr = 1; P.yc = n; }
-    return launch_infer(m, P, stream);
+    return launch_infer(m, P, stream, early);
 }
 
 int chan_internal_closure_device(chan_closure *m) { return m ? m->dev : -1; }
@@ -1040,10 +1016,10 @@ int chan_closure_train(chan_closure *m, int32_t epochs, int32_t batch, double lr
             P.row0 = bi * batch; P.rows = batch;
             P.inv_count = 2.f / (9.f * (float)batch);
             const int grid = train_grid(m, P.rows);
-            CLK(m, launch_early(k_mlp_train, grid, kTrainThreads, TrainSmem::bytes, m->stream, P));
+            CLK(m, launch_kernel(true, k_mlp_train, grid, kTrainThreads, TrainSmem::bytes, m->stream, P));
             m->adam_t++;
             const float c1 = 1.f - std::pow(b1, (float)m->adam_t), c2 = 1.f - std::pow(b2, (float)m->adam_t);
-            CLK(m, launch_early(k_adam, kSumBlocks, kSumThreads, 0, m->stream, m->w, m->m, m->v, m->part, grid, m->img,
+            CLK(m, launch_kernel(true, k_adam, kSumBlocks, kSumThreads, 0, m->stream, m->w, m->m, m->v, m->part, grid, m->img,
                                 (float)lr, b1, b2, eps, c1, c2));
         }
         float l = 0.f;
@@ -1095,7 +1071,7 @@ int chan_closure_infer(chan_closure *m, const float *X, int64_t n, float *Y)
     CLK(m, cudaMalloc((void **)&dY, (size_t)n * kOut * sizeof(float)));
     CLK(m, cudaMemcpy(dX, X, (size_t)n * kIn * sizeof(float), cudaMemcpyHostToDevice));
     CLK(m, cudaMemsetAsync(m->err, 0, sizeof(int), m->stream));
-    int r = chan_internal_infer(m, dX, dY, n, false, m->stream, nullptr);
+    int r = chan_internal_infer(m, dX, dY, n, false, m->stream, nullptr, false);
     if (!r) r = check_err(m);
     if (!r) CLK(m, cudaMemcpy(Y, dY, (size_t)n * kOut * sizeof(float), cudaMemcpyDeviceToHost));
     cudaFree(dX);
