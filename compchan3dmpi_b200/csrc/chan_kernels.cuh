@@ -1534,6 +1534,16 @@ __global__ void __launch_bounds__(StageShape<TI, TJ, R>::NT, StageShape<TI, TJ, 
 // Wall BC + pressure BC (main_v1.9.f90:623-720 on the two wall planes).
 // One thread per (i,j) of a wall plane, ghosts included.
 
+// point p of an n1 x n2 x .. box (i fastest), 0-based.  32-bit unsigned: device memory holds
+// fewer than 2^31 points, and the 64-bit quotients it replaces cost more than the loads
+__device__ __forceinline__ void split3(unsigned p, unsigned n1, unsigned n2, int &i, int &j, int &k)
+{
+    const unsigned r = p / n1, l = r / n2;
+    i = (int)(p - r * n1);
+    j = (int)(r - l * n2);
+    k = (int)l;
+}
+
 // var(u, v, T) of an interior point as the reference holds it (corner columns
 // keep their stale values)
 template <typename QT>
@@ -1999,96 +2009,79 @@ struct DiagParams {
     int planes[kDiagMaxPlanes];
     const double *x3q;   // x3 as the diagnostics see it (the deck's F10.6 column after a restart)
     double dy, Ayz;
-    double *part;        // nP3 per-plane KE sums
+    int split;           // blocks per plane of the KE sums
+    double *part;        // partial sums: KE [nP3][split], then the x-planes' [nplanes][3][nP3]
 };
 
-__global__ void __launch_bounds__(kStatThreads) k_diag_ke(const KParams P, const double *q, const DiagParams D)
+// Partial sums.  Block (k, y): y < split: the KE sum of a share of plane k; then the sums of
+// rho, u and rho*u over the cells between planes k and k+1 of x-plane y - split.  One block
+// per plane and one per x-plane quantity (each over all cells) left the chip idle: 73 us at
+// 101x75x83 with five x-planes, 10 us so split.
+__global__ void __launch_bounds__(kStatThreads) k_diag_part(const KParams P, const double *q, const DiagParams D)
 {
+    __shared__ double red[kStatThreads / 32][3];
     grid_dep_enter();
-    __shared__ double red[kStatThreads / 32];
-    const int n1 = P.n1, n2 = P.n2;
-    const int k = blockIdx.x + 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (frozen(P.status, kstep(P) + 1)) return;
-    double acc = 0.0;
-    const int np = n1 * n2;
-    for (int p = tid; p < np; p += kStatThreads) {
-        const int jj = p / n1, ii = p - jj * n1;
-        double x[7];
-        ref_var(P, q, ii + 1, jj + 1, k, x);
-        acc += (x[1] * x[1] + x[2] * x[2]) + x[3] * x[3];
-    }
-    const double s = warp_sum(acc);
-    if (lane == 0) red[warp] = s;
-    __syncthreads();
-    if (tid == 0) {
-        double t = 0.0;
-        for (int w = 0; w < kStatThreads / 32; w++) t += red[w];
-        D.part[k - 1] = t;
-    }
-}
-
-// block 0: KE from the per-plane sums; block 1+n*np+m: quantity n at plane m
-__global__ void __launch_bounds__(kStatThreads) k_diag_fin(const KParams P, const double *q, const DiagParams D,
-                                                           double *rec, double time)
-{
-    grid_dep_enter();
-    __shared__ double red[kStatThreads / 32];
     const int n1 = P.n1, n2 = P.n2, n3 = P.n3;
-    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (frozen(P.status, kstep(P) + 1)) {
-        if (b == 0 && tid == 0) rec[0] = -1.0;
-        return;
-    }
-    if (b == 0) {
-        if (tid == 0) {
-            double t = 0.0;
-            for (int k = 0; k < n3; k++) t += D.part[k];
-            rec[0] = (double)kstep(P);
-            rec[1] = time;
-            rec[2] = t / ((double)n1 * (double)n2 * (double)n3);
+    const int k = blockIdx.x + 1, y = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (frozen(P.status, kstep(P) + 1)) return;
+    double acc[3] = {0.0, 0.0, 0.0};
+    const int m = y - D.split;
+    if (m < 0) {
+        const unsigned np = (unsigned)n1 * n2;
+        for (unsigned p = y * kStatThreads + tid; p < np; p += D.split * kStatThreads) {
+            const int jj = (int)(p / (unsigned)n1), ii = (int)(p - (unsigned)jj * n1);
+            double x[7];
+            ref_var(P, q, ii + 1, jj + 1, k, x);
+            acc[0] += (x[1] * x[1] + x[2] * x[2]) + x[3] * x[3];
         }
-        return;
-    }
-    const int qn = (b - 1) / D.nplanes, m = (b - 1) % D.nplanes;
-    const int ip = D.planes[m];
-    double acc = 0.0;
-    if (ip > 2 && ip < n1 - 1) {
-        const int nj = n2 - 1, ncell = (n2 - 1) * (n3 - 1);
-        for (int c = tid; c < ncell; c += kStatThreads) {
-            const int j = 1 + c % nj, k = 1 + c / nj;
+    } else if (D.planes[m] > 2 && D.planes[m] < n1 - 1 && k < n3) {
+        const int ip = D.planes[m];
+        const double dAyz = D.dy * (D.x3q[k] - D.x3q[k - 1]);
+        for (int j = 1 + tid; j < n2; j += kStatThreads) {
             double a[7], bb[7], cc[7], d[7];
             ref_var(P, q, ip, j, k, a);
             ref_var(P, q, ip, j + 1, k, bb);
             ref_var(P, q, ip, j, k + 1, cc);
             ref_var(P, q, ip, j + 1, k + 1, d);
-            double f0, f1, f2, f3;
-            if (qn == 0) { f0 = a[0]; f1 = bb[0]; f2 = cc[0]; f3 = d[0]; }
-            else if (qn == 1) { f0 = a[1]; f1 = bb[1]; f2 = cc[1]; f3 = d[1]; }
-            else { f0 = a[0] * a[1]; f1 = bb[0] * bb[1]; f2 = cc[0] * cc[1]; f3 = d[0] * d[1]; }
-            const double dAyz = D.dy * (D.x3q[k] - D.x3q[k - 1]);
-            acc += (0.25 * (((f0 + f1) + f2) + f3)) * dAyz;
+            acc[0] += (0.25 * (((a[0] + bb[0]) + cc[0]) + d[0])) * dAyz;
+            acc[1] += (0.25 * (((a[1] + bb[1]) + cc[1]) + d[1])) * dAyz;
+            acc[2] += (0.25 * (((a[0] * a[1] + bb[0] * bb[1]) + cc[0] * cc[1]) + d[0] * d[1])) * dAyz;
         }
     }
-    const double s = warp_sum(acc);
-    if (lane == 0) red[warp] = s;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const double s = warp_sum(acc[c]);
+        if (lane == 0) red[warp][c] = s;
+    }
     __syncthreads();
-    if (tid == 0) {
+    if (tid < (m < 0 ? 1 : 3)) {
         double t = 0.0;
-        for (int w = 0; w < kStatThreads / 32; w++) t += red[w];
-        rec[3 + qn * D.nplanes + m] = t / D.Ayz;
+        for (int w = 0; w < kStatThreads / 32; w++) t += red[w][tid];
+        D.part[m < 0 ? (k - 1) * D.split + y : n3 * D.split + (3 * m + tid) * n3 + k - 1] = t;
     }
 }
 
-// fluctuation field var(i,j,k,:) - mean(k,:) (fluc.f90:63-69), in place on a
-// [7][N] device copy of var
-__global__ void k_fluctuation(double *var, const double *mean, int n1, int n2, int n3)
+// block 0: KE from the partial sums; block 1+n*np+m: quantity n at plane m.  One warp each.
+__global__ void k_diag_fin(const KParams P, const DiagParams D, double *rec, double time)
 {
-    const long long N = (long long)n1 * n2 * n3;
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
-         p += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(p / ((long long)n1 * n2));
-#pragma unroll
-        for (int m = 0; m < 7; m++) var[(size_t)m * N + p] -= mean[(size_t)m * n3 + k];
+    grid_dep_enter();
+    const int n3 = P.n3, b = blockIdx.x, lane = threadIdx.x;
+    if (frozen(P.status, kstep(P) + 1)) {
+        if (b == 0 && lane == 0) rec[0] = -1.0;
+        return;
+    }
+    const int qn = (b - 1) / max(D.nplanes, 1), m = (b - 1) - qn * D.nplanes;
+    const double *in = b == 0 ? D.part : D.part + (size_t)n3 * D.split + (size_t)(3 * m + qn) * n3;
+    double t = 0.0;
+    for (int e = lane; e < (b == 0 ? n3 * D.split : n3); e += 32) t += in[e];
+    t = warp_sum(t);
+    if (lane != 0) return;
+    if (b == 0) {
+        rec[0] = (double)kstep(P);
+        rec[1] = time;
+        rec[2] = t / ((double)P.n1 * (double)P.n2 * (double)n3);
+    } else {
+        rec[3 + qn * D.nplanes + m] = t / D.Ayz;
     }
 }
 
@@ -2099,12 +2092,10 @@ __global__ void k_fluctuation(double *var, const double *mean, int n1, int n2, i
 __global__ void k_qcrit(int n1, int n2, int n3, const double *u, const double *v, const double *w,
                         const double *x, const double *y, const double *z, double *Q)
 {
-    const long long N = (long long)n1 * n2 * n3;
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
-         p += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(p % n1);
-        const int j = (int)((p / n1) % n2);
-        const int k = (int)(p / ((long long)n1 * n2));
+    const unsigned N = (unsigned)n1 * n2 * n3;
+    for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) {
+        int i, j, k;
+        split3(p, n1, n2, i, j, k);
         if (i == 0 || i == n1 - 1 || j == 0 || j == n2 - 1 || k == 0 || k == n3 - 1) {
             Q[p] = 0.0;
             continue;
@@ -2145,12 +2136,10 @@ __global__ void k_qcrit(int n1, int n2, int n3, const double *u, const double *v
 __global__ void k_upload(const KParams P, const double *var, double *qa, double *qb, double *qc, double *cs)
 {
     const int n1 = P.n1, n2 = P.n2, n3 = P.n3;
-    const long long N = (long long)n1 * n2 * n3;
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
-         p += (long long)gridDim.x * blockDim.x) {
-        const int ii = (int)(p % n1);
-        const int jj = (int)((p / n1) % n2);
-        const int kk = (int)(p / ((long long)n1 * n2));
+    const unsigned N = (unsigned)n1 * n2 * n3;
+    for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) {
+        int ii, jj, kk;
+        split3(p, n1, n2, ii, jj, kk);
         const int i = ii + 1, j = jj + 1, k = kk + 1;
         // T and p (columns 5, 6) are read only on the wall planes and the
         // corner columns: the upload copies them only there
@@ -2217,20 +2206,19 @@ __global__ void k_fill_wall_ring(const KParams P)
         W[(size_t)m * P.plane + (long long)j * P.px + i] = W[(size_t)m * P.plane + (long long)sj * P.px + si];
 }
 
-// Download: state -> var(1:nP1,1:nP2,1:nP3,1:7) ([m][k][j][i])
-__global__ void k_download(const KParams P, const double *q, double *var)
+// Download: state -> var(1:nP1,1:nP2,1:nP3,1:7) ([m][k][j][i]); with mean [7][nP3] the
+// fluctuation field var(i,j,k,:) - mean(k,:) instead (fluc.f90:63-69)
+__global__ void k_download(const KParams P, const double *q, double *var, const double *mean)
 {
     const int n1 = P.n1, n2 = P.n2, n3 = P.n3;
-    const long long N = (long long)n1 * n2 * n3;
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
-         p += (long long)gridDim.x * blockDim.x) {
-        const int ii = (int)(p % n1);
-        const int jj = (int)((p / n1) % n2);
-        const int kk = (int)(p / ((long long)n1 * n2));
+    const unsigned N = (unsigned)n1 * n2 * n3;
+    for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) {
+        int ii, jj, kk;
+        split3(p, n1, n2, ii, jj, kk);
         double x[7];
         ref_var(P, q, ii + 1, jj + 1, kk + 1, x);
 #pragma unroll
-        for (int m = 0; m < 7; m++) var[(size_t)m * N + p] = x[m];
+        for (int m = 0; m < 7; m++) var[(size_t)m * N + p] = mean ? x[m] - mean[(size_t)m * n3 + kk] : x[m];
     }
 }
 
@@ -2238,12 +2226,10 @@ __global__ void k_download(const KParams P, const double *q, double *var)
 __global__ void k_check(const KParams P, const double *q)
 {
     const int n1 = P.n1, n2 = P.n2, n3 = P.n3;
-    const long long N = (long long)n1 * n2 * n3;
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
-         p += (long long)gridDim.x * blockDim.x) {
-        const int ii = (int)(p % n1);
-        const int jj = (int)((p / n1) % n2);
-        const int kk = (int)(p / ((long long)n1 * n2));
+    const unsigned N = (unsigned)n1 * n2 * n3;
+    for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) {
+        int ii, jj, kk;
+        split3(p, n1, n2, ii, jj, kk);
         double x[7];
         ref_var(P, q, ii + 1, jj + 1, kk + 1, x);
         if (x[0] < 0.0 || x[5] < 0.0) flag_blown(P.status, ii + 1, jj + 1, kk + 1, kstep(P));
@@ -2269,23 +2255,22 @@ __device__ __forceinline__ int wrap_any(int i, int n)
 }
 
 // primitives (rho, u, v, w, T) at (i, j, k): the wall-plane ring on the
-// walls, the conservative state elsewhere (exact divisions)
+// walls, the conservative state elsewhere (exact divisions).  The source is
+// selected, not branched to, so that the loads of several points overlap.
 __device__ __forceinline__ void prim_at(const KParams &P, const double *q, int i, int j, int k, double x[5])
 {
     i = wrap_any(i, P.n1);
     j = wrap_any(j, P.n2);
-    if (k <= 1 || k >= P.n3) {
-        const double *W = P.wp + (size_t)(k <= 1 ? 0 : 8) * P.plane + (long long)j * P.px + i;
-        x[0] = W[0]; x[1] = W[P.plane]; x[2] = W[2 * P.plane]; x[3] = W[3 * P.plane]; x[4] = W[5 * P.plane];
-        return;
-    }
-    const long long o = (long long)k * P.plane + (long long)j * P.px + i;
-    const double r = q[o], ri = 1.0 / r;
-    x[0] = r;
-    x[1] = q[P.vol + o] * ri;
-    x[2] = q[2 * P.vol + o] * ri;
-    x[3] = q[3 * P.vol + o] * ri;
-    x[4] = q[4 * P.vol + o] * ri - P.ggMh * ((x[1] * x[1] + x[2] * x[2]) + x[3] * x[3]);
+    const bool wall = k <= 1 || k >= P.n3;
+    const long long col = (long long)j * P.px + i, vs = wall ? P.plane : P.vol;
+    const double *a = wall ? P.wp + (size_t)(k <= 1 ? 0 : 8) * P.plane + col : q + (long long)k * P.plane + col;
+    const double c0 = a[0], c1 = a[vs], c2 = a[2 * vs], c3 = a[3 * vs], c4 = a[(wall ? 5 : 4) * vs];
+    const double ri = wall ? 1.0 : 1.0 / c0;
+    x[0] = c0;
+    x[1] = c1 * ri;
+    x[2] = c2 * ri;
+    x[3] = c3 * ri;
+    x[4] = wall ? c4 : c4 * ri - P.ggMh * ((x[1] * x[1] + x[2] * x[2]) + x[3] * x[3]);
 }
 
 // Favre-filtered (rho, u, v, w, T) at (i, j, k): a box of width fw (even)
@@ -2337,47 +2322,27 @@ struct SgsSampling {
     bool soa;                    // X as [13][n] instead (the closure run's layout)
 };
 
-// Features (and with T the filtered subgrid fluxes) at every sample point.
-// Gradients by central differences of the filtered fields at the sample
-// strides (the coarse grid's spacing); y+ from the wall shear of the last
-// statistics step.
-__global__ void k_sgs_sample(const KParams P, const double *q, const SgsSampling S)
+// Favre-filtered (rho, u, v, w, T) at the sample points and the ring around them (their
+// gradient neighbours): F [5][nk+2][nj+2][ni+2]; at the sample points also the subgrid
+// fluxes T.  Each filtered value is formed once: at every sample point and its six
+// neighbours it was formed seven times (256x192x97, strides 4, 3, 3, width 4: 187 us for
+// the samples, now 43 + 12 for the features below).
+__global__ void __launch_bounds__(128) k_sgs_filter(const KParams P, const double *q, const SgsSampling S, double *F)
 {
-    grid_dep_enter();
-    const long long n = (long long)S.ni * S.nj * S.nk;
-    const double Lx = 1.0 / P.invdx, Ly = 1.0 / P.invdy;   // dx, dy
-    const int n3 = P.n3;
-    const double tw = 0.5 * (P.stat[23 * n3] - P.stat[23 * n3 + 1]);
-    const double rw = 0.5 * (P.stat[0] + P.stat[n3 - 1]);
-    // before the first statistics step the sums are zero: y+ is then 0
-    const double ut = rw > 0.0 ? sqrt(fmax(tw, 0.0) / rw) : 0.0, muw = 0.5 * (P.muwb + P.muwt);
-    for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < n; s += (long long)gridDim.x * blockDim.x) {
-        const int a = (int)(s % S.ni), b = (int)((s / S.ni) % S.nj), c = (int)(s / ((long long)S.ni * S.nj));
-        const int i = S.i0 + S.sx * a, j = S.j0 + S.sy * b, k = S.k0 + S.sz * c;
-        double f0[5], prod[9], fxp[5], fxm[5], fyp[5], fym[5], fzp[5], fzm[5];
-        favre_at(P, q, i, j, k, S.fw, f0, S.T ? prod : nullptr);
-        favre_at(P, q, i + S.sx, j, k, S.fw, fxp, nullptr);
-        favre_at(P, q, i - S.sx, j, k, S.fw, fxm, nullptr);
-        favre_at(P, q, i, j + S.sy, k, S.fw, fyp, nullptr);
-        favre_at(P, q, i, j - S.sy, k, S.fw, fym, nullptr);
-        const int kp = min(k + S.sz, n3), km = max(k - S.sz, 1);
-        favre_at(P, q, i, j, kp, S.fw, fzp, nullptr);
-        favre_at(P, q, i, j, km, S.fw, fzm, nullptr);
-        const double cx = 1.0 / (2.0 * S.sx * Lx), cy = 1.0 / (2.0 * S.sy * Ly);
-        const double cz = 1.0 / (S.x3[kp - 1] - S.x3[km - 1]);
-        float *X = S.soa ? S.X + s : S.X + s * 13;
-        const long long xc = S.soa ? n : 1;
-        // du_a/dx_b, a = u, v, w (fields 1..3), b = x, spanwise, wall-normal; then dT/dx_b
-        for (int m = 0; m < 4; m++) {
-            X[(3 * m + 0) * xc] = (float)((fxp[m + 1] - fxm[m + 1]) * cx);
-            X[(3 * m + 1) * xc] = (float)((fyp[m + 1] - fym[m + 1]) * cy);
-            X[(3 * m + 2) * xc] = (float)((fzp[m + 1] - fzm[m + 1]) * cz);
-        }
-        const double d = fmin(S.x3[k - 1] - S.x3[0], S.x3[n3 - 1] - S.x3[k - 1]);
-        X[12 * xc] = (float)(rw * ut * d * (1.0 / P.invRe) / muw);
-        if (S.T) {
-            const double r = f0[0], u = f0[1], v = f0[2], w = f0[3], T = f0[4];
-            float *Tg = S.T + s * 9;
+    const int e1 = S.ni + 2, e2 = S.nj + 2;
+    const unsigned ne = (unsigned)e1 * e2 * (S.nk + 2);
+    for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < ne; p += gridDim.x * blockDim.x) {
+        int a, b, c;
+        split3(p, e1, e2, a, b, c);
+        const int k = min(max(S.k0 + S.sz * (c - 1), 1), P.n3);
+        const bool own = a >= 1 && a <= S.ni && b >= 1 && b <= S.nj && c >= 1 && c <= S.nk;
+        double f[5], prod[9];
+        favre_at(P, q, S.i0 + S.sx * (a - 1), S.j0 + S.sy * (b - 1), k, S.fw, f, own ? prod : nullptr);
+#pragma unroll
+        for (int m = 0; m < 5; m++) F[(size_t)m * ne + p] = f[m];
+        if (own) {
+            const double r = f[0], u = f[1], v = f[2], w = f[3], T = f[4];
+            float *Tg = S.T + (((size_t)(c - 1) * S.nj + (b - 1)) * S.ni + (a - 1)) * 9;
             Tg[0] = (float)(prod[0] - r * u * u);
             Tg[1] = (float)(prod[1] - r * v * v);
             Tg[2] = (float)(prod[2] - r * w * w);
@@ -2391,6 +2356,59 @@ __global__ void k_sgs_sample(const KParams P, const double *q, const SgsSampling
     }
 }
 
+// Features at every sample point, from the filtered fields F of k_sgs_filter
+// (FILTERED; q = F) or the state itself (q).  Gradients by central differences at the
+// sample strides (the coarse grid's spacing); y+ from the wall shear of the last
+// statistics step.
+template <bool FILTERED>
+__global__ void __launch_bounds__(128) k_sgs_features(const KParams P, const double *q, const SgsSampling S)
+{
+    grid_dep_enter();
+    const unsigned n = (unsigned)S.ni * S.nj * S.nk;
+    const size_t e1 = S.ni + 2, e12 = e1 * (S.nj + 2), ne = e12 * (S.nk + 2);
+    const double Lx = 1.0 / P.invdx, Ly = 1.0 / P.invdy;   // dx, dy
+    const int n3 = P.n3;
+    const double tw = 0.5 * (P.stat[23 * n3] - P.stat[23 * n3 + 1]);
+    const double rw = 0.5 * (P.stat[0] + P.stat[n3 - 1]);
+    // before the first statistics step the sums are zero: y+ is then 0
+    const double ut = rw > 0.0 ? sqrt(fmax(tw, 0.0) / rw) : 0.0, muw = 0.5 * (P.muwb + P.muwt);
+    const double cx = 1.0 / (2.0 * S.sx * Lx), cy = 1.0 / (2.0 * S.sy * Ly);
+    for (unsigned s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+        int a, b, c;
+        split3(s, S.ni, S.nj, a, b, c);
+        const int i = S.i0 + S.sx * a, j = S.j0 + S.sy * b, k = S.k0 + S.sz * c;
+        const int kp = min(k + S.sz, n3), km = max(k - S.sz, 1);
+        auto at = [&](int da, int db, int dc, double x[5]) {
+            if (FILTERED) {
+                const double *f = q + (c + 1 + dc) * e12 + (b + 1 + db) * e1 + (a + 1 + da);
+#pragma unroll
+                for (int m = 1; m < 5; m++) x[m] = f[m * ne];
+            } else {
+                prim_at(P, q, i + da * S.sx, j + db * S.sy, dc > 0 ? kp : (dc < 0 ? km : k), x);
+            }
+        };
+        double fxp[5], fxm[5], fyp[5], fym[5], fzp[5], fzm[5];
+        at(1, 0, 0, fxp);
+        at(-1, 0, 0, fxm);
+        at(0, 1, 0, fyp);
+        at(0, -1, 0, fym);
+        at(0, 0, 1, fzp);
+        at(0, 0, -1, fzm);
+        const double cz = 1.0 / (S.x3[kp - 1] - S.x3[km - 1]);
+        float *X = S.soa ? S.X + s : S.X + (size_t)s * 13;
+        const size_t xc = S.soa ? n : 1;
+        // du_a/dx_b, a = u, v, w (fields 1..3), b = x, spanwise, wall-normal; then dT/dx_b
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            X[(3 * m + 0) * xc] = (float)((fxp[m + 1] - fxm[m + 1]) * cx);
+            X[(3 * m + 1) * xc] = (float)((fyp[m + 1] - fym[m + 1]) * cy);
+            X[(3 * m + 2) * xc] = (float)((fzp[m + 1] - fzm[m + 1]) * cz);
+        }
+        const double d = fmin(S.x3[k - 1] - S.x3[0], S.x3[n3 - 1] - S.x3[k - 1]);
+        X[12 * xc] = (float)(rw * ut * d * (1.0 / P.invRe) / muw);
+    }
+}
+
 // Closure source at the interior points from the subgrid fluxes Y [9][n]
 // (n = (n1-2)(n2-2)(n3-2), index ((k-2)(n2-2) + (j-2))(n1-2) + i-2; zero on
 // the walls): S(rho u_a) = -d tau_ab / dx_b, S(rho E) = -gama d q_b / dx_b
@@ -2399,25 +2417,23 @@ __global__ void k_sgs_div(const KParams P, const float *Y, double gama, double *
 {
     grid_dep_enter();
     const int n1 = P.n1, n2 = P.n2, n3 = P.n3, m1 = n1 - 2, m2 = n2 - 2;
-    const long long n = (long long)m1 * m2 * (n3 - 2);
-    auto at = [&](int i, int j, int k, int c) -> double {
-        if (k <= 1 || k >= n3) return 0.0;
-        i = wrap_any(i, n1);
-        j = wrap_any(j, n2);
-        return (double)Y[(long long)c * n + (((long long)(k - 2) * m2) + (j - 2)) * m1 + (i - 2)];
-    };
+    const unsigned n = (unsigned)m1 * m2 * (n3 - 2);
     // flux component of (row a, direction b): tau_ab, or q_b for the energy row
-    auto comp = [](int a, int b) {
-        const int t[3][3] = {{0, 3, 4}, {3, 1, 5}, {4, 5, 2}};
-        return a < 3 ? t[a][b] : 6 + b;
-    };
-    for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < n; s += (long long)gridDim.x * blockDim.x) {
-        const int i = 2 + (int)(s % m1), j = 2 + (int)((s / m1) % m2), k = 2 + (int)(s / ((long long)m1 * m2));
-        const double cz = P.czh[k];
+    const auto comp = [](int a, int b) { return a == 3 ? 6 + b : (a == b ? a : 2 + a + b); };
+    for (unsigned s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+        int ii, jj, kk;
+        split3(s, m1, m2, ii, jj, kk);
+        const double cz = P.czh[kk + 2];
+        const unsigned pl = (unsigned)m1 * m2;
+        const unsigned xp = ii == m1 - 1 ? s - (m1 - 1) : s + 1, xm = ii == 0 ? s + (m1 - 1) : s - 1;
+        const unsigned yp = jj == m2 - 1 ? s - (pl - m1) : s + m1, ym = jj == 0 ? s + (pl - m1) : s - m1;
+        const bool top = kk == n3 - 3, bot = kk == 0;   // the fluxes vanish on the walls
+        const unsigned zp = top ? s : s + pl, zm = bot ? s : s - pl;
+#pragma unroll
         for (int a = 0; a < 4; a++) {
-            const double d = (at(i + 1, j, k, comp(a, 0)) - at(i - 1, j, k, comp(a, 0))) * P.hdx +
-                             (at(i, j + 1, k, comp(a, 1)) - at(i, j - 1, k, comp(a, 1))) * P.hdy +
-                             (at(i, j, k + 1, comp(a, 2)) - at(i, j, k - 1, comp(a, 2))) * cz;
+            const float *Yx = Y + (size_t)comp(a, 0) * n, *Yy = Y + (size_t)comp(a, 1) * n, *Yz = Y + (size_t)comp(a, 2) * n;
+            const double d = ((double)Yx[xp] - (double)Yx[xm]) * P.hdx + ((double)Yy[yp] - (double)Yy[ym]) * P.hdy +
+                             ((top ? 0.0 : (double)Yz[zp]) - (bot ? 0.0 : (double)Yz[zm])) * cz;
             S[(size_t)a * n + s] = a < 3 ? -d : -gama * d;
         }
     }
@@ -2429,12 +2445,12 @@ __global__ void k_sgs_apply(const KParams P, double *qo, const double *S, double
 {
     grid_dep_enter();
     const int n1 = P.n1, m1 = n1 - 2, m2 = P.n2 - 2, w = n1 + 2;
-    const long long n = (long long)m1 * m2 * (P.n3 - 2), tot = (long long)w * m2 * (P.n3 - 2);
-    for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < tot; s += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(s % w), r = (int)(s / w);       // r: row of S
-        const int j = 2 + r % m2, k = 2 + r / m2;
-        const long long src = (long long)r * m1 + (wrap_any(i, n1) - 2);
-        const long long o = (long long)k * P.plane + (long long)j * P.px + i;
+    const unsigned n = (unsigned)m1 * m2 * (P.n3 - 2), tot = (unsigned)w * m2 * (P.n3 - 2);
+    for (unsigned s = blockIdx.x * blockDim.x + threadIdx.x; s < tot; s += gridDim.x * blockDim.x) {
+        int i, jj, kk;
+        split3(s, w, m2, i, jj, kk);
+        const unsigned src = (unsigned)(kk * m2 + jj) * m1 + (wrap_any(i, n1) - 2);
+        const long long o = (long long)(kk + 2) * P.plane + (long long)(jj + 2) * P.px + i;
         // S rows: rho*u, rho*v, rho*w, rho*E (state variables 1..4)
 #pragma unroll
         for (int a = 0; a < 4; a++) qo[o + (a + 1) * P.vol] += cdt * S[(size_t)a * n + src];

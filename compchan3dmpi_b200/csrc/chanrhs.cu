@@ -357,7 +357,8 @@ int closure_source(chan_ctx *c)
     S.T = nullptr;
     S.soa = true;
     const long long n = (long long)S.ni * S.nj * S.nk;
-    CK(c, launch_kernel(c->early, chan::k_sgs_sample, 1184, 128, 0, c->stream, c->kp, (const double *)c->kp.qin, S));
+    CK(c, launch_kernel(c->early, chan::k_sgs_features<false>, 1184, 128, 0, c->stream, c->kp,
+                        (const double *)c->kp.qin, S));
     int r = chan_internal_infer(c->cl, c->sgsX, c->sgsY, n, true, c->stream, c->sgsflag, c->early);
     if (r) { c->err = "closure inference"; return r; }
     CK(c, launch_kernel(c->early, chan::k_sgs_div, 1184, 256, 0, c->stream, c->kp, c->sgsY, c->p.gama, c->sgsS));
@@ -425,9 +426,9 @@ int launch_diag(chan_ctx *c, long long step, double time)
 {
     c->kp.step = step;
     double *rec = c->diag_rec + (size_t)(c->diag_count % c->diag_cap) * c->diag_reclen;
-    CK(c, launch_kernel(c->early, chan::k_diag_ke, c->n3, chan::kStatThreads, 0, c->stream, c->kp, c->q[c->cur], c->dp));
-    CK(c, launch_kernel(c->early, chan::k_diag_fin, 1 + 3 * c->dp.nplanes, chan::kStatThreads, 0, c->stream, c->kp,
-                        c->q[c->cur], c->dp, rec, time));
+    CK(c, launch_kernel(c->early, chan::k_diag_part, dim3(c->n3, c->dp.split + c->dp.nplanes), chan::kStatThreads, 0,
+                        c->stream, c->kp, c->q[c->cur], c->dp));
+    CK(c, launch_kernel(c->early, chan::k_diag_fin, 1 + 3 * c->dp.nplanes, 32, 0, c->stream, c->kp, c->dp, rec, time));
     c->diag_count++;
     return CHAN_OK;
 }
@@ -936,7 +937,7 @@ int chan_download(chan_ctx *c, double *var)
     if (!c->uploaded) return CHAN_ESTATE;
     CK(c, cudaSetDevice(c->dev));
     const size_t N = (size_t)c->n1 * c->n2 * c->n3;
-    chan::k_download<<<1184, 256, 0, c->stream>>>(c->kp, c->q[c->cur], c->dvar);
+    chan::k_download<<<1184, 256, 0, c->stream>>>(c->kp, c->q[c->cur], c->dvar, nullptr);
     CK(c, cudaGetLastError());
     CK(c, cudaMemcpyAsync(var, c->dvar, 7 * N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
@@ -1378,9 +1379,10 @@ int chan_diag_enable(chan_ctx *c, const int32_t *planes, int32_t nplanes, int32_
     if (!(z[n3 - 1] > 0)) { c->err = "chan_diag_enable: x3(nP3) must be > 0"; return CHAN_EINVAL; }
     if (c->diag_rec) { cudaFree(c->diag_rec); c->diag_rec = nullptr; }
     if (!c->diag_part) {
-        CK(c, cudaMalloc((void **)&c->diag_part, (size_t)n3 * sizeof(double)));
+        const size_t np = (size_t)n3 * (c->nsplit + 3 * chan::kDiagMaxPlanes);
+        CK(c, cudaMalloc((void **)&c->diag_part, np * sizeof(double)));
         CK(c, cudaMalloc((void **)&c->diag_x3, (size_t)n3 * sizeof(double)));
-        c->dev_bytes += 2 * (size_t)n3 * sizeof(double);
+        c->dev_bytes += (np + n3) * sizeof(double);
     }
     const int reclen = 3 + 3 * nplanes;
     CK(c, cudaMalloc((void **)&c->diag_rec, (size_t)capacity * reclen * sizeof(double)));
@@ -1391,6 +1393,7 @@ int chan_diag_enable(chan_ctx *c, const int32_t *planes, int32_t nplanes, int32_
     D.x3q = c->diag_x3;
     D.dy = c->p.Ly / (double)(c->n2 - 1);
     D.Ayz = z[n3 - 1] * x2end;
+    D.split = c->nsplit;
     D.part = c->diag_part;
     c->diag_every = every;
     c->diag_cap = capacity;
@@ -1463,9 +1466,7 @@ int chan_fluctuation_q(chan_ctx *c, const double *mean, const double *x1, const 
     int r = upload_coords(c, x1, x2, x3, c->dxyz);
     if (r) return r;
     CK(c, cudaMemcpyAsync(dmean, mean, 7 * (size_t)c->n3 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    chan::k_download<<<1184, 256, 0, c->stream>>>(c->kp, c->q[c->cur], c->dvar);
-    CK(c, cudaGetLastError());
-    chan::k_fluctuation<<<1184, 256, 0, c->stream>>>(c->dvar, dmean, c->n1, c->n2, c->n3);
+    chan::k_download<<<1184, 256, 0, c->stream>>>(c->kp, c->q[c->cur], c->dvar, dmean);
     CK(c, cudaGetLastError());
     if (qcrit) {
         chan::k_qcrit<<<1184, 256, 0, c->stream>>>(c->n1, c->n2, c->n3, c->dvar + N, c->dvar + 2 * N,
@@ -2224,7 +2225,11 @@ int chan_internal_sample(chan_ctx *c, float *X, float *T, long long capacity, in
     S.X = X;
     S.T = T;
     // the state after whole steps: q[cur] in double
-    chan::k_sgs_sample<<<1184, 128, 0, c->stream>>>(c->kp, c->q[c->cur], S);
+    // (the download buffer, 7 doubles a point, holds the filtered fields: 5 per sample point
+    // and its ring, which has no more points than the grid)
+    chan::k_sgs_filter<<<1184, 128, 0, c->stream>>>(c->kp, c->q[c->cur], S, c->dvar);
+    CK(c, cudaGetLastError());
+    chan::k_sgs_features<true><<<1184, 128, 0, c->stream>>>(c->kp, c->dvar, S);
     CK(c, cudaGetLastError());
     CK(c, cudaStreamSynchronize(c->stream));
     *added = n;

@@ -662,27 +662,37 @@ __global__ void k_weight_images(const float *w, unsigned char *img)
     if (i < kNParam) put_images(i, w[i], img);
 }
 
-// column sums and sums of squares of an [n][ncol] array (double atomics)
-__global__ void k_colstats(const float *A, long long n, int ncol, double *sum, double *sumsq)
+// column sums and sums of squares of an [n][NCOL] array (double atomics, one per block
+// and sum; one per warp, and a run-time NCOL that put the sums in local memory, took 88 us
+// for 127,000 rows of 13)
+template <int NCOL>
+__global__ void __launch_bounds__(256) k_colstats(const float *A, long long n, double *sum, double *sumsq)
 {
-    double s[16], s2[16];
-    for (int c = 0; c < ncol; c++) s[c] = s2[c] = 0.0;
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < n; r += (long long)gridDim.x * blockDim.x)
-        for (int c = 0; c < ncol; c++) {
-            const double v = A[r * ncol + c];
+    __shared__ double red[8][2 * NCOL];
+    double s[NCOL], s2[NCOL];
+#pragma unroll
+    for (int c = 0; c < NCOL; c++) s[c] = s2[c] = 0.0;
+    for (long long r = blockIdx.x * 256LL + threadIdx.x; r < n; r += gridDim.x * 256LL)
+#pragma unroll
+        for (int c = 0; c < NCOL; c++) {
+            const double v = A[r * NCOL + c];
             s[c] += v;
             s2[c] += v * v;
         }
-    for (int c = 0; c < ncol; c++) {
-        double a = s[c], b = s2[c];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int c = 0; c < NCOL; c++) {
         for (int o = 16; o > 0; o >>= 1) {
-            a += __shfl_xor_sync(0xffffffffu, a, o);
-            b += __shfl_xor_sync(0xffffffffu, b, o);
+            s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+            s2[c] += __shfl_xor_sync(0xffffffffu, s2[c], o);
         }
-        if ((threadIdx.x & 31) == 0) {
-            atomicAdd(&sum[c], a);
-            atomicAdd(&sumsq[c], b);
-        }
+        if (lane == 0) { red[warp][c] = s[c]; red[warp][NCOL + c] = s2[c]; }
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * NCOL) {
+        double t = 0.0;
+        for (int w = 0; w < 8; w++) t += red[w][threadIdx.x];
+        atomicAdd(threadIdx.x < NCOL ? &sum[threadIdx.x] : &sumsq[threadIdx.x - NCOL], t);
     }
 }
 
@@ -773,6 +783,12 @@ int train_grid(const chan_closure *m, long long rows)
     return (int)(ntiles < m->sms ? ntiles : m->sms);
 }
 
+// the gradient sums' array, from the first training call on
+cudaError_t ensure_part(chan_closure *m)
+{
+    return m->part ? cudaSuccess : cudaMalloc((void **)&m->part, (size_t)m->sms * kPartStride * sizeof(float));
+}
+
 int check_err(chan_closure *m)
 {
     int h = 0;
@@ -845,7 +861,6 @@ int chan_closure_create(int32_t device, int64_t capacity, chan_closure **out)
     if (e == cudaSuccess) e = cudaMalloc((void **)&m->w, 4 * (size_t)kPStride * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&m->img, WImages::bytes);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&m->part, (size_t)m->sms * kPartStride * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&m->norm, 44 * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&m->loss, sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&m->err, sizeof(int));
@@ -918,8 +933,8 @@ int chan_closure_fit_normalization(chan_closure *m, float *norm_out)
     double *acc = nullptr;
     CLK(m, cudaMalloc((void **)&acc, 44 * sizeof(double)));
     CLK(m, cudaMemsetAsync(acc, 0, 44 * sizeof(double), m->stream));
-    k_colstats<<<4 * m->sms, 256, 0, m->stream>>>(m->X, m->count, kIn, acc, acc + 13);
-    k_colstats<<<4 * m->sms, 256, 0, m->stream>>>(m->T, m->count, kOut, acc + 26, acc + 35);
+    k_colstats<kIn><<<2 * m->sms, 256, 0, m->stream>>>(m->X, m->count, acc, acc + 13);
+    k_colstats<kOut><<<2 * m->sms, 256, 0, m->stream>>>(m->T, m->count, acc + 26, acc + 35);
     double h[44];
     cudaError_t e = cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, m->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
@@ -999,6 +1014,7 @@ int chan_closure_train(chan_closure *m, int32_t epochs, int32_t batch, double lr
     if (!m || epochs < 0 || batch < kTile || batch % kTile || !(lr > 0)) return CHAN_EINVAL;
     if (m->count < batch) { m->msg = "fewer samples than one batch"; return CHAN_EINVAL; }
     CLK(m, cudaSetDevice(m->dev));
+    CLK(m, ensure_part(m));
     CLK(m, cudaMemsetAsync(m->err, 0, sizeof(int), m->stream));
     const long long n = m->count, nb = n / batch;
     uint64_t st = seed;
@@ -1036,6 +1052,7 @@ int chan_closure_grad(chan_closure *m, const float *X, const float *T, int64_t n
 {
     if (!m || !X || !T || n < 1) return CHAN_EINVAL;
     CLK(m, cudaSetDevice(m->dev));
+    CLK(m, ensure_part(m));
     float *dX = nullptr, *dT = nullptr;
     CLK(m, cudaMalloc((void **)&dX, (size_t)n * kIn * sizeof(float)));
     CLK(m, cudaMalloc((void **)&dT, (size_t)n * kOut * sizeof(float)));
