@@ -28,7 +28,7 @@ def sources():
 
 
 def deps():
-    return sorted(SRC.glob("*.cu")) + sorted(SRC.glob("*.cuh")) + sorted(SRC.glob("*.cpp")) + \
+    return sorted(SRC.glob("*.cu")) + sorted(SRC.glob("*.cuh")) + sorted(SRC.glob("*.h")) + sorted(SRC.glob("*.cpp")) + \
         [ROOT / "include" / "chanrhs.h"]
 
 

@@ -2133,7 +2133,7 @@ __global__ void k_qcrit(int n1, int n2, int n3, const double *u, const double *v
 // ---------------------------------------------------------------------------
 // Upload: var(1:nP1,1:nP2,1:nP3,1:7) (device copy, [m][k][j][i]) -> state.
 // initSolV (main_v1.9.f90:284-294): Q = rho*(1,u,v,w,E) at every point.
-__global__ void k_upload(const KParams P, const double *var, double *qa, double *qb, double *qc, double *cs)
+__global__ void k_upload(const KParams P, const double *var, const double *cor, double *qa, double *qb, double *qc, double *cs)
 {
     const int n1 = P.n1, n2 = P.n2, n3 = P.n3;
     const unsigned N = (unsigned)n1 * n2 * n3;
@@ -2141,14 +2141,15 @@ __global__ void k_upload(const KParams P, const double *var, double *qa, double 
         int ii, jj, kk;
         split3(p, n1, n2, ii, jj, kk);
         const int i = ii + 1, j = jj + 1, k = kk + 1;
-        // T and p (columns 5, 6) are read only on the wall planes and the
-        // corner columns: the upload copies them only there
+        // T and p (columns 5, 6) are read only on the wall planes, and on the corner
+        // columns from cor [2][4][nP3]: the upload copies no others
         const bool wall = (k == 1 || k == n3), corner = (i == 1 || i == n1) && (j == 1 || j == n2);
         double x[7];
 #pragma unroll
         for (int m = 0; m < 5; m++) x[m] = var[(size_t)m * N + p];
-        x[5] = (wall || corner) ? var[(size_t)5 * N + p] : 0.0;
-        x[6] = (wall || corner) ? var[(size_t)6 * N + p] : 0.0;
+        const double *co = cor + (size_t)((i == 1 ? 0 : 1) + (j == 1 ? 0 : 2)) * n3 + kk;
+        x[5] = wall ? var[(size_t)5 * N + p] : (corner ? co[0] : 0.0);
+        x[6] = wall ? var[(size_t)6 * N + p] : (corner ? co[4 * n3] : 0.0);
         const long long o = (long long)k * P.plane + (long long)j * P.px + i;
         double q[5] = {x[0], x[0] * x[1], x[0] * x[2], x[0] * x[3], x[0] * x[4]};
 #pragma unroll

@@ -6,6 +6,7 @@
 #include "chanrhs.h"
 #include "chan_internal.h"
 #include "chan_kernels.cuh"
+#include "host_copy.h"
 
 #include <cudaTypedefs.h>
 
@@ -81,6 +82,8 @@ struct chan_ctx {
     double tavg_t0 = 0.0, tavg_t1 = 0.0;
     chan::DevStatus *status = nullptr;
     chan::DevStatus *h_status = nullptr;
+    double *h_stat = nullptr;                  // pinned, behind h_status: one copy of the statistics
+    std::shared_ptr<HostCopy> hc;              // staged copies (host_copy.h), from the first large one on
     int n1 = 0, n2 = 0, n3 = 0, px = 0, NJ = 0;
     long long plane = 0, vol = 0;
     int tile = CHAN_TILE_32x8, ntx = 0, nty = 0, nchunks = 1, kchunk = 1;   // stage-kernel launch shape
@@ -699,7 +702,11 @@ int chan_init(const chan_params *p, const double *x3, const double *jac, const d
     }
     e = cudaMalloc((void **)&c->status, sizeof(chan::DevStatus));
     if (e == cudaSuccess) e = cudaMemsetAsync(c->status, 0, sizeof(chan::DevStatus), c->stream);
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&c->h_status, sizeof(chan::DevStatus));
+    if (e == cudaSuccess) {
+        const size_t hs = (sizeof(chan::DevStatus) + 63) / 64 * 64;
+        e = cudaMallocHost((void **)&c->h_status, hs + (23 * (size_t)n3 + 2) * sizeof(double));
+        if (e == cudaSuccess) c->h_stat = (double *)((char *)c->h_status + hs);
+    }
     if (e != cudaSuccess) { fail(nullptr, "status allocation", e); chan_free(c); return CHAN_ENOMEM; }
 
     // mesh-derived tables (1-based k stored at index k)
@@ -809,19 +816,22 @@ int chan_upload(chan_ctx *c, const double *var, int64_t nstep, double time)
     // rho, u, v, w, E everywhere; T and p only where they are read: the two
     // wall planes and the four corner columns (the interior primitives are
     // derived from the conservative state)
-    CK(c, cudaMemcpyAsync(c->dvar, var, 5 * N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    for (int m = 5; m < 7; m++) {
+    CK(c, HostCopy::copy(c->hc, c->dev, c->dvar, var, 5 * N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    for (int m = 5; m < 7; m++)
         for (size_t k : {(size_t)0, (size_t)c->n3 - 1})
             CK(c, cudaMemcpyAsync(c->dvar + m * N + k * pl, var + m * N + k * pl, pl * sizeof(double),
                                   cudaMemcpyHostToDevice, c->stream));
-        for (size_t jc : {(size_t)0, (size_t)c->n2 - 1})
-            for (size_t ic : {(size_t)0, (size_t)c->n1 - 1}) {
-                const size_t o = m * N + jc * c->n1 + ic;
-                CK(c, cudaMemcpy2DAsync(c->dvar + o, pl * sizeof(double), var + o, pl * sizeof(double),
-                                        sizeof(double), c->n3, cudaMemcpyHostToDevice, c->stream));
-            }
-    }
-    chan::k_upload<<<1184, 256, 0, c->stream>>>(c->kp, c->dvar, c->q[0], c->mixed ? c->q[0] : c->q[1],
+    // the corner columns as one block [2][4][nP3] (as strided copies of single words they
+    // took longer than the rest), over interior planes of T, which are not read
+    std::vector<double> corner((size_t)8 * c->n3);
+    for (int m = 0; m < 2; m++)
+        for (int cc = 0; cc < 4; cc++) {
+            const double *src = var + (5 + m) * N + ((cc & 2) ? (size_t)(c->n2 - 1) * c->n1 : 0) + ((cc & 1) ? c->n1 - 1 : 0);
+            for (int k = 0; k < c->n3; k++) corner[((size_t)m * 4 + cc) * c->n3 + k] = src[k * pl];
+        }
+    double *dcorner = c->dvar + 5 * N + pl;
+    CK(c, cudaMemcpyAsync(dcorner, corner.data(), corner.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    chan::k_upload<<<1184, 256, 0, c->stream>>>(c->kp, c->dvar, dcorner, c->q[0], c->mixed ? c->q[0] : c->q[1],
                                                   c->mixed ? nullptr : c->q[2], c->cs);
     CK(c, cudaGetLastError());
     {
@@ -911,11 +921,12 @@ int chan_stats(chan_ctx *c, double *tau2, double *stat1, double *stat2, double *
     if (!c) return CHAN_EINVAL;
     CK(c, cudaSetDevice(c->dev));
     const size_t n3 = (size_t)c->n3;
-    if (tau2) CK(c, cudaMemcpyAsync(tau2, c->stat + 23 * n3, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    if (stat1) CK(c, cudaMemcpyAsync(stat1, c->stat, 7 * n3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    if (stat2) CK(c, cudaMemcpyAsync(stat2, c->stat + 7 * n3, 7 * n3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    if (corr) CK(c, cudaMemcpyAsync(corr, c->stat + 14 * n3, 9 * n3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    CK(c, cudaMemcpyAsync(c->h_stat, c->stat, (23 * n3 + 2) * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
+    if (tau2) memcpy(tau2, c->h_stat + 23 * n3, 2 * sizeof(double));
+    if (stat1) memcpy(stat1, c->h_stat, 7 * n3 * sizeof(double));
+    if (stat2) memcpy(stat2, c->h_stat + 7 * n3, 7 * n3 * sizeof(double));
+    if (corr) memcpy(corr, c->h_stat + 14 * n3, 9 * n3 * sizeof(double));
     return CHAN_OK;
 }
 
@@ -939,7 +950,7 @@ int chan_download(chan_ctx *c, double *var)
     const size_t N = (size_t)c->n1 * c->n2 * c->n3;
     chan::k_download<<<1184, 256, 0, c->stream>>>(c->kp, c->q[c->cur], c->dvar, nullptr);
     CK(c, cudaGetLastError());
-    CK(c, cudaMemcpyAsync(var, c->dvar, 7 * N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    CK(c, HostCopy::copy(c->hc, c->dev, var, c->dvar, 7 * N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
     return CHAN_OK;
 }
@@ -1095,7 +1106,7 @@ int chan_checkpoint_write(chan_ctx *c, const char *path)
                  nst = 23 * (size_t)c->n3 + 2;
     std::vector<double> hb(nq + nw + ncs + 2 * nst);
     double *o = hb.data();
-    CK(c, cudaMemcpyAsync(o, c->q[0], nq * sizeof(double), cudaMemcpyDeviceToHost, c->stream)); o += nq;
+    CK(c, HostCopy::copy(c->hc, c->dev, o, c->q[0], nq * sizeof(double), cudaMemcpyDeviceToHost, c->stream)); o += nq;
     CK(c, cudaMemcpyAsync(o, c->wp, nw * sizeof(double), cudaMemcpyDeviceToHost, c->stream)); o += nw;
     CK(c, cudaMemcpyAsync(o, c->cs, ncs * sizeof(double), cudaMemcpyDeviceToHost, c->stream)); o += ncs;
     CK(c, cudaMemcpyAsync(o, c->stat, nst * sizeof(double), cudaMemcpyDeviceToHost, c->stream)); o += nst;
@@ -1143,7 +1154,8 @@ int chan_checkpoint_read(chan_ctx *c, const char *path)
     if (!ok) { c->err = std::string("checkpoint truncated: ") + path; return CHAN_EIO; }
     const double *o = hb.data();
     for (int b = 0; b < (c->mixed ? 1 : 3); b++)
-        CK(c, cudaMemcpyAsync(c->q[b], o, nq * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+        CK(c, b == 0 ? HostCopy::copy(c->hc, c->dev, c->q[0], o, nq * sizeof(double), cudaMemcpyHostToDevice, c->stream)
+                     : cudaMemcpyAsync(c->q[b], c->q[0], nq * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     { int r = seed_float_stages(c); if (r) return r; }
     o += nq;
     CK(c, cudaMemcpyAsync(c->wp, o, nw * sizeof(double), cudaMemcpyHostToDevice, c->stream)); o += nw;
@@ -1410,14 +1422,20 @@ int chan_diag_read(chan_ctx *c, double *records, int32_t max_records, int32_t *n
     const long long avail = c->diag_count < c->diag_cap ? c->diag_count : c->diag_cap;
     if (!records) { *nrecords = (int32_t)avail; if (lost) *lost = c->diag_count - avail; return CHAN_OK; }
     if (max_records < avail) { c->err = "chan_diag_read: records buffer too small"; return CHAN_EINVAL; }
-    std::vector<double> ring((size_t)c->diag_cap * c->diag_reclen);
-    CK(c, cudaMemcpyAsync(ring.data(), c->diag_rec, ring.size() * sizeof(double), cudaMemcpyDeviceToHost,
-                          c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));
     const long long first = c->diag_count - avail;  // index of the oldest record kept
+    // the records in the order of writing: to the ring's end, then from its start
+    std::vector<double> ring((size_t)avail * c->diag_reclen);
+    const long long f0 = first % c->diag_cap, n0 = std::min<long long>(avail, c->diag_cap - f0);
+    const size_t rl = (size_t)c->diag_reclen;
+    if (n0 > 0)
+        CK(c, cudaMemcpyAsync(ring.data(), c->diag_rec + f0 * rl, n0 * rl * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    if (avail > n0)
+        CK(c, cudaMemcpyAsync(ring.data() + n0 * rl, c->diag_rec, (avail - n0) * rl * sizeof(double), cudaMemcpyDeviceToHost,
+                              c->stream));
+    CK(c, cudaStreamSynchronize(c->stream));
     int32_t n = 0;
-    for (long long r = first; r < c->diag_count; r++) {
-        const double *src = ring.data() + (size_t)(r % c->diag_cap) * c->diag_reclen;
+    for (long long r = 0; r < avail; r++) {
+        const double *src = ring.data() + (size_t)r * rl;
         if (src[0] < 0) continue;  // after a blow-up
         memcpy(records + (size_t)n * c->diag_reclen, src, c->diag_reclen * sizeof(double));
         n++;
@@ -1473,9 +1491,10 @@ int chan_fluctuation_q(chan_ctx *c, const double *mean, const double *x1, const 
                                                     c->dvar + 3 * N, c->dxyz, c->dxyz + c->n1,
                                                     c->dxyz + c->n1 + c->n2, c->dq);
         CK(c, cudaGetLastError());
-        CK(c, cudaMemcpyAsync(qcrit, c->dq, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+        CK(c, HostCopy::copy(c->hc, c->dev, qcrit, c->dq, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     }
-    if (fluc) CK(c, cudaMemcpyAsync(fluc, c->dvar, 7 * N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    if (fluc)
+        CK(c, HostCopy::copy(c->hc, c->dev, fluc, c->dvar, 7 * N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
     return CHAN_OK;
 }

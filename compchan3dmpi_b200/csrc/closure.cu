@@ -5,6 +5,7 @@
 // product through the C ABI.
 #include "chanrhs.h"
 #include "chan_internal.h"
+#include "host_copy.h"
 #include "umma.cuh"
 
 #include <cuda_bf16.h>
@@ -716,7 +717,9 @@ long long gcd_ll(long long a, long long b)
 struct chan_closure {
     int dev = 0;
     cudaStream_t stream = nullptr;
-    float *X = nullptr, *T = nullptr;       // [cap][13], [cap][9] samples
+    float *X = nullptr, *T = nullptr;       // [cap][13], [cap][9] samples (one allocation)
+    unsigned char *block = nullptr;         // what acc, w, img, norm, loss and err point into
+    double *acc = nullptr;                  // column sums [44]
     long long cap = 0, count = 0;
     float *w = nullptr, *m = nullptr, *v = nullptr, *g = nullptr;   // kNParam each
     unsigned char *img = nullptr;           // BF16 weight images
@@ -727,6 +730,10 @@ struct chan_closure {
     long long adam_t = 0;
     float out_limit = 50.f;
     int sms = 148;
+    float *ws = nullptr;                    // rows of infer and grad calls (Batch)
+    size_t ws_bytes = 0;
+    std::mutex ws_mu;
+    std::shared_ptr<HostCopy> hc;           // staged copies (host_copy.h), from the first large one on
     std::string msg;
 };
 
@@ -783,11 +790,51 @@ int train_grid(const chan_closure *m, long long rows)
     return (int)(ntiles < m->sms ? ntiles : m->sms);
 }
 
-// the gradient sums' array, from the first training call on
+// the gradient sums' array: beside the samples, or with room for none from the first
+// gradient on
 cudaError_t ensure_part(chan_closure *m)
 {
     return m->part ? cudaSuccess : cudaMalloc((void **)&m->part, (size_t)m->sms * kPartStride * sizeof(float));
 }
+
+// a copy to or from the host on the closure's stream, complete on return
+cudaError_t host_copy(chan_closure *m, void *dst, const void *src, size_t n, cudaMemcpyKind kind)
+{
+    const cudaError_t e = HostCopy::copy(m->hc, m->dev, dst, src, n, kind, m->stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(m->stream) : e;
+}
+
+// device arrays of one call's rows, X [n][13] and Y [n][9]: the closure's workspace, which
+// grows to kBatchKeep rows and stays (allocating and freeing both took 1.1 of the 1.6 ms of
+// 50,001 rows' inference); for more rows, or while another thread has it, the call's own
+// allocation
+constexpr long long kBatchKeep = 1 << 20;   // 92 MB
+struct Batch {
+    float *X = nullptr, *Y = nullptr, *own = nullptr;
+    cudaError_t e = cudaSuccess;
+    std::unique_lock<std::mutex> lock;
+    Batch(chan_closure *m, long long n) : lock(m->ws_mu, std::try_to_lock)
+    {
+        const size_t xw = ((size_t)n * kIn + 63) / 64 * 64, bytes = (xw + (size_t)n * kOut) * sizeof(float);
+        if (n > kBatchKeep || !lock.owns_lock()) {
+            e = cudaMalloc((void **)&own, bytes);
+            X = own;
+        } else {
+            if (m->ws_bytes < bytes) {
+                if (m->ws) cudaFree(m->ws);
+                m->ws = nullptr;
+                m->ws_bytes = 0;
+                e = cudaMalloc((void **)&m->ws, bytes);
+                if (e == cudaSuccess) m->ws_bytes = bytes;
+            }
+            X = m->ws;
+        }
+        Y = X ? X + xw : nullptr;
+    }
+    ~Batch() { if (own) cudaFree(own); }
+    Batch(const Batch &) = delete;
+    Batch &operator=(const Batch &) = delete;
+};
 
 int check_err(chan_closure *m)
 {
@@ -856,17 +903,30 @@ int chan_closure_create(int32_t device, int64_t capacity, chan_closure **out)
     m->cap = capacity;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess && capacity > 0) e = cudaMalloc((void **)&m->X, (size_t)capacity * kIn * sizeof(float));
-    if (e == cudaSuccess && capacity > 0) e = cudaMalloc((void **)&m->T, (size_t)capacity * kOut * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&m->w, 4 * (size_t)kPStride * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&m->img, WImages::bytes);
+    // two allocations: the samples, X then T, with the training kernel's sums, and everything
+    // small (each cudaMalloc and cudaFree takes 0.3 to 1 ms)
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&m->norm, 44 * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&m->loss, sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&m->err, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(m->w, 0, 4 * (size_t)kPStride * sizeof(float));
-    if (e == cudaSuccess) e = cudaMemset(m->img, 0, WImages::bytes);
-    if (e == cudaSuccess) e = cudaMemset(m->err, 0, sizeof(int));
+    const size_t xw = ((size_t)capacity * kIn + 63) / 64 * 64, tw = ((size_t)capacity * kOut + 63) / 64 * 64;
+    if (e == cudaSuccess && capacity > 0)
+        e = cudaMalloc((void **)&m->X, (xw + tw + (size_t)m->sms * kPartStride) * sizeof(float));
+    if (e == cudaSuccess && capacity > 0) {
+        m->T = m->X + xw;
+        m->part = m->T + tw;
+    }
+    constexpr size_t accOff = 0, wOff = 44 * sizeof(double) + 32, imgOff = wOff + 4 * (size_t)kPStride * sizeof(float),
+                     normOff = imgOff + WImages::bytes, lossOff = normOff + 48 * sizeof(float), errOff = lossOff + 16,
+                     small = errOff + 16;
+    static_assert(wOff % 128 == 0 && imgOff % 128 == 0 && normOff % 16 == 0, "alignment of a closure's arrays");
+    if (e == cudaSuccess) e = cudaMalloc((void **)&m->block, small);
+    if (e == cudaSuccess) e = cudaMemset(m->block, 0, small);
+    if (e == cudaSuccess) {
+        m->acc = (double *)(m->block + accOff);
+        m->w = (float *)(m->block + wOff);
+        m->img = m->block + imgOff;
+        m->norm = (float *)(m->block + normOff);
+        m->loss = (float *)(m->block + lossOff);
+        m->err = (int *)(m->block + errOff);
+    }
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, TrainSmem::bytes);
     if (e == cudaSuccess)
@@ -904,8 +964,8 @@ int chan_closure_add_data(chan_closure *m, const float *X, const float *T, int64
 {
     if (!m || !X || !T || n < 0 || m->count + n > m->cap) return CHAN_EINVAL;
     CLK(m, cudaSetDevice(m->dev));
-    CLK(m, cudaMemcpy(m->X + m->count * kIn, X, (size_t)n * kIn * sizeof(float), cudaMemcpyHostToDevice));
-    CLK(m, cudaMemcpy(m->T + m->count * kOut, T, (size_t)n * kOut * sizeof(float), cudaMemcpyHostToDevice));
+    CLK(m, host_copy(m, m->X + m->count * kIn, X, (size_t)n * kIn * sizeof(float), cudaMemcpyHostToDevice));
+    CLK(m, host_copy(m, m->T + m->count * kOut, T, (size_t)n * kOut * sizeof(float), cudaMemcpyHostToDevice));
     m->count += n;
     return CHAN_OK;
 }
@@ -921,8 +981,8 @@ int chan_closure_get_data(chan_closure *m, int64_t first, int64_t n, float *X, f
 {
     if (!m || first < 0 || n < 0 || first + n > m->count) return CHAN_EINVAL;
     CLK(m, cudaSetDevice(m->dev));
-    if (X) CLK(m, cudaMemcpy(X, m->X + first * kIn, (size_t)n * kIn * sizeof(float), cudaMemcpyDeviceToHost));
-    if (T) CLK(m, cudaMemcpy(T, m->T + first * kOut, (size_t)n * kOut * sizeof(float), cudaMemcpyDeviceToHost));
+    if (X) CLK(m, host_copy(m, X, m->X + first * kIn, (size_t)n * kIn * sizeof(float), cudaMemcpyDeviceToHost));
+    if (T) CLK(m, host_copy(m, T, m->T + first * kOut, (size_t)n * kOut * sizeof(float), cudaMemcpyDeviceToHost));
     return CHAN_OK;
 }
 
@@ -930,15 +990,13 @@ int chan_closure_fit_normalization(chan_closure *m, float *norm_out)
 {
     if (!m || m->count < 2) return CHAN_EINVAL;
     CLK(m, cudaSetDevice(m->dev));
-    double *acc = nullptr;
-    CLK(m, cudaMalloc((void **)&acc, 44 * sizeof(double)));
+    double *acc = m->acc;
     CLK(m, cudaMemsetAsync(acc, 0, 44 * sizeof(double), m->stream));
     k_colstats<kIn><<<2 * m->sms, 256, 0, m->stream>>>(m->X, m->count, acc, acc + 13);
     k_colstats<kOut><<<2 * m->sms, 256, 0, m->stream>>>(m->T, m->count, acc + 26, acc + 35);
     double h[44];
     cudaError_t e = cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, m->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
-    cudaFree(acc);
     if (e != cudaSuccess) return cfail(m, "normalization", e);
     float nrm[44];
     const double n = (double)m->count;
@@ -1053,11 +1111,11 @@ int chan_closure_grad(chan_closure *m, const float *X, const float *T, int64_t n
     if (!m || !X || !T || n < 1) return CHAN_EINVAL;
     CLK(m, cudaSetDevice(m->dev));
     CLK(m, ensure_part(m));
-    float *dX = nullptr, *dT = nullptr;
-    CLK(m, cudaMalloc((void **)&dX, (size_t)n * kIn * sizeof(float)));
-    CLK(m, cudaMalloc((void **)&dT, (size_t)n * kOut * sizeof(float)));
-    CLK(m, cudaMemcpy(dX, X, (size_t)n * kIn * sizeof(float), cudaMemcpyHostToDevice));
-    CLK(m, cudaMemcpy(dT, T, (size_t)n * kOut * sizeof(float), cudaMemcpyHostToDevice));
+    Batch b(m, n);
+    CLK(m, b.e);
+    float *dX = b.X, *dT = b.Y;
+    CLK(m, host_copy(m, dX, X, (size_t)n * kIn * sizeof(float), cudaMemcpyHostToDevice));
+    CLK(m, host_copy(m, dT, T, (size_t)n * kOut * sizeof(float), cudaMemcpyHostToDevice));
     CLK(m, cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
     CLK(m, cudaMemsetAsync(m->err, 0, sizeof(int), m->stream));
     MlpParams P = base_params(m);
@@ -1073,8 +1131,6 @@ int chan_closure_grad(chan_closure *m, const float *X, const float *T, int64_t n
     if (!r) r = check_err(m);
     if (!r && grads) CLK(m, cudaMemcpy(grads, m->g, (size_t)kNParam * sizeof(float), cudaMemcpyDeviceToHost));
     if (!r) CLK(m, cudaMemcpy(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost));
-    cudaFree(dX);
-    cudaFree(dT);
     if (loss_sum) *loss_sum = l;
     return r;
 }
@@ -1083,16 +1139,14 @@ int chan_closure_infer(chan_closure *m, const float *X, int64_t n, float *Y)
 {
     if (!m || !X || !Y || n < 1) return CHAN_EINVAL;
     CLK(m, cudaSetDevice(m->dev));
-    float *dX = nullptr, *dY = nullptr;
-    CLK(m, cudaMalloc((void **)&dX, (size_t)n * kIn * sizeof(float)));
-    CLK(m, cudaMalloc((void **)&dY, (size_t)n * kOut * sizeof(float)));
-    CLK(m, cudaMemcpy(dX, X, (size_t)n * kIn * sizeof(float), cudaMemcpyHostToDevice));
+    Batch b(m, n);
+    CLK(m, b.e);
+    float *dX = b.X, *dY = b.Y;
+    CLK(m, host_copy(m, dX, X, (size_t)n * kIn * sizeof(float), cudaMemcpyHostToDevice));
     CLK(m, cudaMemsetAsync(m->err, 0, sizeof(int), m->stream));
     int r = chan_internal_infer(m, dX, dY, n, false, m->stream, nullptr, false);
     if (!r) r = check_err(m);
-    if (!r) CLK(m, cudaMemcpy(Y, dY, (size_t)n * kOut * sizeof(float), cudaMemcpyDeviceToHost));
-    cudaFree(dX);
-    cudaFree(dY);
+    if (!r) CLK(m, host_copy(m, Y, dY, (size_t)n * kOut * sizeof(float), cudaMemcpyDeviceToHost));
     return r;
 }
 
@@ -1104,13 +1158,9 @@ void chan_closure_free(chan_closure *m)
     cudaSetDevice(m->dev);
     if (m->stream) cudaStreamSynchronize(m->stream);
     if (m->X) cudaFree(m->X);
-    if (m->T) cudaFree(m->T);
-    if (m->w) cudaFree(m->w);
-    if (m->img) cudaFree(m->img);
-    if (m->part) cudaFree(m->part);
-    if (m->norm) cudaFree(m->norm);
-    if (m->loss) cudaFree(m->loss);
-    if (m->err) cudaFree(m->err);
+    if (m->block) cudaFree(m->block);
+    if (m->part && !m->X) cudaFree(m->part);
+    if (m->ws) cudaFree(m->ws);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
 }
