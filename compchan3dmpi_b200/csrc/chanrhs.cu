@@ -295,9 +295,37 @@ void set_stage(chan_ctx *c, int iter)
     k.rk_eps = k.rk_a + (k.rk_b - 1.0);   // exact: both sums are
 }
 
-// stage-kernel launch shape: tile shape and number of k-chunks (0: the
-// chunk count whose CTAs fill whole waves of resident CTAs with the least
-// prologue overhead per marched plane)
+// the k-chunk count of a tile shape whose CTAs fill whole waves of resident CTAs with the
+// least prologue overhead per marched plane; *cost: its waves times planes per CTA, the
+// prologue counted as 2.5
+int best_chunks(chan_ctx *c, int tile, int *nchunks, double *cost)
+{
+    const StageSet &ss = kStageSets[tile];
+    const int nz = c->n3 - 2, v = c->mixed ? 2 : 0;
+    const long long tiles = (long long)((c->n1 - 2 + ss.ti - 1) / ss.ti) * ((c->n2 - 2 + ss.tj - 1) / ss.tj);
+    int sms = 148, occ = 1;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
+    CK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ss.k[0][v], ss.block[v != 0].x * ss.tj,
+                                                        v == 0 ? ss.smem : ss.smemf));
+    if (occ < 1) occ = 1;
+    const long long slots = (long long)sms * occ;
+    double best = -1.0;
+    for (int nc = 1; nc <= nz; nc++) {
+        const int chunk = (nz + nc - 1) / nc;
+        if ((nz + chunk - 1) / chunk != nc) continue;
+        const long long ctas = tiles * nc;
+        const long long waves = (ctas + slots - 1) / slots;
+        const double eff = (double)ctas / (double)(waves * slots) * (double)chunk / (chunk + 2.5);
+        if (eff > best + 1e-9) {
+            best = eff;
+            *nchunks = nc;
+            *cost = (double)waves * (chunk + 2.5);
+        }
+    }
+    return CHAN_OK;
+}
+
+// stage-kernel launch shape: tile shape and number of k-chunks (0: best_chunks)
 int set_launch(chan_ctx *c, int tile, int nchunks)
 {
     if (tile < 0 || tile >= CHAN_NTILES) { c->err = "unknown tile shape"; return CHAN_EINVAL; }
@@ -306,22 +334,9 @@ int set_launch(chan_ctx *c, int tile, int nchunks)
     if (nchunks < 0 || nchunks > nz) { c->err = "k-chunk count out of range"; return CHAN_EINVAL; }
     const int ntx = (c->n1 - 2 + ss.ti - 1) / ss.ti, nty = (c->n2 - 2 + ss.tj - 1) / ss.tj;
     if (nchunks == 0) {
-        int sms = 148, occ = 1;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
-        const int v = c->mixed ? 2 : 0;
-        CK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ss.k[0][v], ss.block[v != 0].x * ss.tj,
-                                                            v == 0 ? ss.smem : ss.smemf));
-        if (occ < 1) occ = 1;
-        const long long slots = (long long)sms * occ, tiles = (long long)ntx * nty;
-        double best = -1.0;
-        for (int nc = 1; nc <= nz; nc++) {
-            const int chunk = (nz + nc - 1) / nc;
-            if ((nz + chunk - 1) / chunk != nc) continue;
-            const long long ctas = tiles * nc;
-            const long long waves = (ctas + slots - 1) / slots;
-            const double eff = (double)ctas / (double)(waves * slots) * (double)chunk / (chunk + 2.5);
-            if (eff > best + 1e-9) { best = eff; nchunks = nc; }
-        }
+        double cost;
+        const int r = best_chunks(c, tile, &nchunks, &cost);
+        if (r) return r;
     }
     // the chunk count that a chunk length of ceil(nz/nchunks) really gives
     const int chunk = (nz + nchunks - 1) / nchunks;
@@ -333,6 +348,26 @@ int set_launch(chan_ctx *c, int tile, int nchunks)
     c->kp.kchunk = chunk;
     c->epoch++;
     return CHAN_OK;
+}
+
+// the shape chan_init picks: 32x8, or in FP64 16x16 where it covers the plane with enough
+// less padding.  Both have 256 points, and over 22 grids the 16x16 tile took 0.97 to 1.03
+// times the time where the costs are equal; where its cost is 0.78 to 0.85 of the other's
+// the stage took 0.81 to 0.88 of the time (101x75x83, cost 0.93: 0.95), where it is 1.1
+// and more 1.11 to 1.14.  In mixed precision the 16x16 tile is 4 to 13% slower at equal
+// cost, its pairs leaving rows of eight threads.
+int default_launch(chan_ctx *c)
+{
+    int tile = CHAN_TILE_32x8;
+    if (!c->mixed) {
+        int nc = 1;
+        double wide, square;
+        int r = best_chunks(c, CHAN_TILE_32x8, &nc, &wide);
+        if (!r) r = best_chunks(c, CHAN_TILE_16x16, &nc, &square);
+        if (r) return r;
+        if (square < 0.96 * wide) tile = CHAN_TILE_16x16;
+    }
+    return set_launch(c, tile, 0);
 }
 
 // device copy of x3 (closure features need the wall-normal coordinates)
@@ -798,7 +833,7 @@ int chan_init(const chan_params *p, const double *x3, const double *jac, const d
         // the tile's own points (no halo); the x origin 2 + TI*bx gives 16-byte aligned copies
         if ((r = make_state_map(c, &c->tmb[t], c->q[0], false, ti, tj, 0))) { g_init_error = c->err; chan_free(c); return r; }
     }
-    if (set_launch(c, CHAN_TILE_32x8, 0) != CHAN_OK) { g_init_error = c->err; chan_free(c); return CHAN_ECUDA; }
+    if (default_launch(c) != CHAN_OK) { g_init_error = c->err; chan_free(c); return CHAN_ECUDA; }
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
     c->nsplit = stats_split(sms, n1, n2, n3);

@@ -219,8 +219,9 @@ typedef struct chan_wall_bc {
 int chan_set_wall_bc(chan_ctx *c, int32_t wall, const chan_wall_bc *bc);
 
 /* Stage-kernel launch shape (no reference counterpart; it changes no result
- * bits).  tile: CHAN_TILE_32x8 (256 threads in FP64, 128 in mixed precision; the
- * default), CHAN_TILE_32x4 (half of that), CHAN_TILE_16x16 (as 32x8) or
+ * bits).  tile: CHAN_TILE_32x8 (256 threads in FP64, 128 in mixed precision; what
+ * chan_init picks unless, in FP64, CHAN_TILE_16x16 covers the plane with less padding),
+ * CHAN_TILE_32x4 (half of that), CHAN_TILE_16x16 (as 32x8) or
  * CHAN_TILE_32x16 (twice that; one CTA per SM in FP64) columns x rows per CTA;
  * nchunks: how many CTAs split the
  * wall-normal march of one tile column (1..nP3-2; 0 picks the count that fills

@@ -67,3 +67,21 @@ def test_mixed_edges_same_bits_and_near_oracle(nP, tile):
     for m in range(7):
         s = scale if m in (1, 2, 3) else np.max(np.abs(ref[m]))
         assert np.max(np.abs(base[m] - ref[m])) <= 2e-6 * s, m
+
+
+@pytest.mark.parametrize("nP,mixed,tile", [((24, 14, 19), False, 0), ((101, 75, 33), False, 2), ((101, 75, 33), True, 0)])
+def test_default_tile_changes_no_bits(nP, mixed, tile):
+    """The shape picked at creation against the 32x8 tile: the same results to the bit."""
+    p, x3, jac, inv, var = make_case(nP=nP, mesh="tanh", beta=2.2, rk=RK2, istat=2, quantize=False)
+    out = []
+    for forced in (False, True):
+        g = Channel(p.with_(mixed=mixed), x3, jac, inv)
+        if forced:
+            g.set_launch(0, 0)
+        else:
+            assert g.launch()[0] == tile
+        g.init_sol_v(var)
+        g.step(4)
+        out.append(g.download())
+        g.close()
+    assert np.array_equal(out[0], out[1])
