@@ -724,6 +724,7 @@ struct chan_closure {
     float *w = nullptr, *m = nullptr, *v = nullptr, *g = nullptr;   // kNParam each
     unsigned char *img = nullptr;           // BF16 weight images
     float *part = nullptr;                  // gradient sums of the training kernel's CTAs, [sms][kPartStride]
+    bool part_own = true;                   // its own allocation
     float *norm = nullptr;                  // xmu[13] xsd[13] ymu[9] ysd[9]
     float *loss = nullptr;
     int *err = nullptr;
@@ -790,8 +791,7 @@ int train_grid(const chan_closure *m, long long rows)
     return (int)(ntiles < m->sms ? ntiles : m->sms);
 }
 
-// the gradient sums' array: beside the samples, or with room for none from the first
-// gradient on
+// the gradient sums' array, unless it came with the samples
 cudaError_t ensure_part(chan_closure *m)
 {
     return m->part ? cudaSuccess : cudaMalloc((void **)&m->part, (size_t)m->sms * kPartStride * sizeof(float));
@@ -903,15 +903,18 @@ int chan_closure_create(int32_t device, int64_t capacity, chan_closure **out)
     m->cap = capacity;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
-    // two allocations: the samples, X then T, with the training kernel's sums, and everything
-    // small (each cudaMalloc and cudaFree takes 0.3 to 1 ms)
+    // two allocations: the samples, X then T, and everything small.  A cudaMalloc of 2 MB and
+    // more takes 0.3 to 1 ms, a smaller one shares a mapped block: the training kernel's sums
+    // (3.3 MB) come with samples that are as large anyway, else from the first training call
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device);
     const size_t xw = ((size_t)capacity * kIn + 63) / 64 * 64, tw = ((size_t)capacity * kOut + 63) / 64 * 64;
+    const bool big = (xw + tw) * sizeof(float) >= (2u << 20);
     if (e == cudaSuccess && capacity > 0)
-        e = cudaMalloc((void **)&m->X, (xw + tw + (size_t)m->sms * kPartStride) * sizeof(float));
+        e = cudaMalloc((void **)&m->X, (xw + tw + (big ? (size_t)m->sms * kPartStride : 0)) * sizeof(float));
     if (e == cudaSuccess && capacity > 0) {
         m->T = m->X + xw;
-        m->part = m->T + tw;
+        m->part = big ? m->T + tw : nullptr;
+        m->part_own = !big;
     }
     constexpr size_t accOff = 0, wOff = 44 * sizeof(double) + 32, imgOff = wOff + 4 * (size_t)kPStride * sizeof(float),
                      normOff = imgOff + WImages::bytes, lossOff = normOff + 48 * sizeof(float), errOff = lossOff + 16,
@@ -1159,7 +1162,7 @@ void chan_closure_free(chan_closure *m)
     if (m->stream) cudaStreamSynchronize(m->stream);
     if (m->X) cudaFree(m->X);
     if (m->block) cudaFree(m->block);
-    if (m->part && !m->X) cudaFree(m->part);
+    if (m->part && m->part_own) cudaFree(m->part);
     if (m->ws) cudaFree(m->ws);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;

@@ -73,9 +73,9 @@ def test_column_statistics(n):
     assert np.all(np.abs(out - ref) <= 2e-7 * scale)
 
 
-# rows of 52 bytes: below and from 4 MB on the copies are staged in 1 MB chunks; whole
+# rows of 52 bytes: below and from 16 MB on the copies are staged in 1 MB chunks; whole
 # chunks, and one row more
-@pytest.mark.parametrize("n", [1, 80659, 80660, 262144, 262145, 500001])
+@pytest.mark.parametrize("n", [1, 322638, 322639, 524288, 524289, 700001])
 def test_host_copies_round_trip(n):
     rng = np.random.default_rng(n)
 
