@@ -448,10 +448,14 @@ __device__ __forceinline__ void prims_from_q(const KParams &P, const double q[5]
 // The fused stage kernel.
 //
 // A CTA owns a TI x TJ tile of interior (i,j) columns and marches a chunk of
-// interior planes k = kb..ke.  A thread owns two neighbouring x columns (i, i+1),
-// i even, so that every shared and global access of its own pair, of its y
-// neighbours and of its x stencil is an aligned 16-byte (FP64) or 8-byte (float)
-// one.  Shared memory holds, for the tile plus a 2-point halo box
+// interior planes k = kb..ke.  A thread owns one x column (FP64) or two neighbouring
+// ones (float: i even, so that every access of its pair, of its y neighbours and of its
+// x stencil is an aligned 8-byte one in shared, 16-byte one in global memory).
+// Bound by instruction issue and latency, not by HBM: 256x193x192, a launch, FP64 0.604 ->
+// 0.505 ms and mixed 0.441 -> 0.346 ms with the plane's scattered per-thread loads (RK
+// base, tables, forcing density) by bulk copies, the wall-normal sum completed one plane
+// behind, the x images under one branch and the y images left to the wall launch.
+// Shared memory holds, for the tile plus a 2-point halo box
 // ((TI+4) x (TJ+4)):
 //   Q (5 vars)      of planes t, t+1, t+2   (3-slot ring; t+2 in flight)
 //   prims u,v,w,T   of planes t, t+1        (2-slot ring)
@@ -1000,11 +1004,12 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
             stp<PX>(MU + p, mu);
         };
         // the wall test taken once per plane, so that each loop's body is
-        // straight-line code; the per-thread box loads one pair at a time, with
-        // fewer loads in flight
+        // straight-line code (the per-thread box loads of both of a thread's pairs
+        // in flight at once; one pair at a time took 2.7% more of the mixed stage time, and
+        // loads held across the inviscid sums spill 676 bytes)
         auto loop = [&](bool wall_plane) {
             if (!TMA) {
-#pragma unroll 1
+#pragma unroll
                 for (int l = 0; l < NL; l++) one(l, wall_plane);
             } else {
 #pragma unroll
@@ -1220,7 +1225,7 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
         for (int a = 0; a < PX; a++) wq[a] = qk[a] ? w4[a] : -(wn[a] * s12p);
         if constexpr (!FOLD) {
             source(tz, um1, wm1, Tm1, qm1[0], s2, s4, s5);
-            if (need_base && staged) cp_async_wait<0>();
+            if (staged) cp_async_wait<0>();
         }
 #pragma unroll
         for (int c = 0; c < 5; c++) {
@@ -1240,6 +1245,8 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
                 if (TMA) {
 #pragma unroll
                     for (int a = 0; a < PX; a++) qs[a] = (double)qm1[c][a];
+                } else if (staged) {
+                    ldp<PX>(sQB + (c * NT + tid) * PX, qs);
                 } else {
                     ldgp<PX, PERSIST>(qin() + c * vol + off, qs);
                 }
@@ -1293,14 +1300,16 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
             }
         }
     };
-    // float rings: the own points' RK base of plane m starts its way into shared memory
+    // float rings: the own points' RK base of plane m starts its way into shared memory;
+    // in the stage that reads the double state, which has no other base, that state (read
+    // from memory by the update it took 2.3% more of the mixed stage time)
     auto fetch_base = [&](int m) {
-        if (!FOLD && need_base && out0) {
-            const double *src = P.qbase + (long long)m * plane + colo;
+        if (!FOLD && out0) {
+            const double *src = (TMA ? P.qbase : reinterpret_cast<const double *>(qin())) + (long long)m * plane + colo;
 #pragma unroll
             for (int c = 0; c < 5; c++) cp_async_d<PX>(sQB + (c * NT + tid) * PX, src + c * vol);
         }
-        if (!FOLD && need_base) cp_async_commit();
+        if (!FOLD) cp_async_commit();
     };
 
     // Iteration t forms the fluxes of plane t and completes plane t-1, whose
