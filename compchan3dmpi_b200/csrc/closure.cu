@@ -167,7 +167,7 @@ __device__ __forceinline__ void st_bf16x8(unsigned char *base, uint32_t off, con
 // columns, into one register per thread and layer.  The sample of a row needs no division: the
 // permutation is affine, so a group's next tile is a fixed step further.
 // 65,536 rows: 197 us in the earlier form (one tile per CTA, transposed copies, 128-bit
-// sample indices, a five-shuffle sum and an atomic per bias column).
+// sample indices, a five-shuffle sum and an atomic per bias column), 45 now.
 constexpr int kGroups = 2, kGroupThreads = 2 * kTile, kTrainThreads = kGroups * kGroupThreads + 32;
 struct TrainSmem {
     static constexpr int x = 0;                                      // X   [2][128][16], alternating by tile
