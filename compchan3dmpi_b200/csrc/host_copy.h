@@ -28,17 +28,19 @@ public:
             if (p) cudaFreeHost(p);
     }
 
-    // the process's instance: at most kThreads * 2 MB of pinned memory, shared by the handles
-    // that hold it and freed with the last of them; null if it cannot be had
-    static std::shared_ptr<HostCopy> get() noexcept
+    // the caller's hold on the process's instance, taken if it has none: at most kThreads * 2
+    // MB of pinned memory, shared by the handles that hold it and freed with the last of
+    // them; null if it cannot be had.  Two threads may make their first copies with one
+    // handle, so its hold is read and set under the instance's lock.
+    static std::shared_ptr<HostCopy> get(std::shared_ptr<HostCopy> &hold) noexcept
     {
         try {
             static std::mutex mu;
             static std::weak_ptr<HostCopy> one;
             std::lock_guard<std::mutex> l(mu);
-            std::shared_ptr<HostCopy> p = one.lock();
-            if (!p) one = p = std::make_shared<HostCopy>();
-            return p;
+            if (!hold) hold = one.lock();
+            if (!hold) one = hold = std::make_shared<HostCopy>();
+            return hold;
         } catch (...) {
             return nullptr;
         }
@@ -46,15 +48,15 @@ public:
 
     // cudaMemcpyAsync(dst, src, n, kind, st), kind to or from the host, on device dev.  A
     // large pageable array is staged, and then the copy is complete on return (as the
-    // driver's own is); anything else is the driver's.  hc: where the caller keeps its hold.
-    static cudaError_t copy(std::shared_ptr<HostCopy> &hc, int dev, void *dst, const void *src, size_t n,
+    // driver's own is); anything else is the driver's.  hold: where the caller keeps its hold.
+    static cudaError_t copy(std::shared_ptr<HostCopy> &hold, int dev, void *dst, const void *src, size_t n,
                             cudaMemcpyKind kind, cudaStream_t st) noexcept
     {
         // Below kMin the driver's copy is as fast: 6.9 MB back took 0.57 ms and varied little,
         // staged 0.43 to 0.59 with the threads' start; at 11 MB 1.04 to 1.22 and 0.99 to 1.14
         if (n >= kMin && pageable(kind == cudaMemcpyHostToDevice ? src : dst)) {
             cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-            if (!hc) hc = get();
+            const std::shared_ptr<HostCopy> hc = get(hold);
             if (hc && cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
                 std::unique_lock<std::mutex> l(hc->busy, std::try_to_lock);   // in use by another thread: not waited for
                 cudaError_t e = cudaSuccess;
