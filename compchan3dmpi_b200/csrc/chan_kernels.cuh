@@ -587,19 +587,18 @@ __device__ __forceinline__ void stp(T *p, const R in[PX])
         *p = (T)in[0];
     }
 }
-// the same from global memory, as doubles.  State written earlier in the same
-// launch by other CTAs (the persistent ensemble kernel, COHERENT) must not use
-// the read-only path.
-template <int PX, bool COHERENT, typename T>
+// the same from global memory, as doubles.  Plain loads, never the read-only path: an
+// early-launched CTA is resident while the kernel before it still writes this state (in
+// the persistent ensemble kernel, other CTAs of the same launch do).
+template <int PX, typename T>
 __device__ __forceinline__ void ldgp(const T *p, double out[PX])
 {
     if constexpr (PX == 2) {
-        const auto *q = reinterpret_cast<const typename Pair<T>::V *>(p);
-        const typename Pair<T>::V v = COHERENT ? *q : __ldg(q);
+        const typename Pair<T>::V v = *reinterpret_cast<const typename Pair<T>::V *>(p);
         out[0] = (double)v.x;
         out[1] = (double)v.y;
     } else {
-        out[0] = COHERENT ? (double)*p : (double)__ldg(p);
+        out[0] = (double)*p;
     }
 }
 
@@ -691,8 +690,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long *bar, unsig
 // One CTA's work of the stage kernel on tile (bx, by) and k-chunk bz, for
 // thread (tx, ty).  BUOYM: 0 no buoyancy term, 1 with it, 2 as P.buoy_on
 // says.  PERSIST: called from the persistent ensemble kernel, where the state
-// was written earlier in the same launch: coherent loads instead of the
-// read-only path, and a proxy fence before the first box copy.
+// was written earlier in the same launch: a proxy fence before the first box copy.
 template <int TI, int TJ, typename QI, typename QO, typename R, int BUOYM, bool PERSIST>
 __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *tmq, const CUtensorMap *tmb, int bx, int by,
                                            int bz, int tx, int ty, unsigned char *smem_raw)
@@ -967,7 +965,7 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
                 const long long off = (long long)m * plane + lo[l];
 #pragma unroll
                 for (int v = 0; v < 5; v++) {
-                    ldgp<PX, PERSIST>(qin() + v * vol + off, q[v]);
+                    ldgp<PX>(qin() + v * vol + off, q[v]);
                     stp<PX>(sq(s, v) + p, q[v]);
                 }
             }
@@ -1025,13 +1023,13 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
     auto center = [&](int m, double q[5][PX], double u[PX], double v[PX], double w[PX], double T[PX]) {
         const long long off = (long long)m * plane + colo;
 #pragma unroll
-        for (int c = 0; c < 5; c++) ldgp<PX, PERSIST>(qin() + c * vol + off, q[c]);
+        for (int c = 0; c < 5; c++) ldgp<PX>(qin() + c * vol + off, q[c]);
         if (m == 1 || m == n3) {
             const double *W = P.wp + (size_t)(m == 1 ? 0 : 8) * plane + colo;
-            ldgp<PX, true>(W + 1 * plane, u);
-            ldgp<PX, true>(W + 2 * plane, v);
-            ldgp<PX, true>(W + 3 * plane, w);
-            ldgp<PX, true>(W + 5 * plane, T);
+            ldgp<PX>(W + 1 * plane, u);
+            ldgp<PX>(W + 2 * plane, v);
+            ldgp<PX>(W + 3 * plane, w);
+            ldgp<PX>(W + 5 * plane, T);
         } else {
 #pragma unroll
             for (int a = 0; a < PX; a++) {
@@ -1248,11 +1246,11 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
                 } else if (staged) {
                     ldp<PX>(sQB + (c * NT + tid) * PX, qs);
                 } else {
-                    ldgp<PX, PERSIST>(qin() + c * vol + off, qs);
+                    ldgp<PX>(qin() + c * vol + off, qs);
                 }
                 if (need_base) {
                     if (staged) ldp<PX>(sQB + (c * NT + tid) * PX, qb);
-                    else ldgp<PX, PERSIST>(P.qbase + c * vol + off, qb);
+                    else ldgp<PX>(P.qbase + c * vol + off, qb);
                 }
 #pragma unroll
                 for (int a = 0; a < PX; a++) {
