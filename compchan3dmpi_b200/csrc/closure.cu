@@ -734,6 +734,7 @@ struct chan_closure {
     float *ws = nullptr;                    // rows of infer and grad calls (Batch)
     size_t ws_bytes = 0;
     std::mutex ws_mu;
+    std::mutex acc_mu;                      // one call at a time uses acc
     std::shared_ptr<HostCopy> hc;           // staged copies (host_copy.h), from the first large one on
     std::string msg;
 };
@@ -993,6 +994,7 @@ int chan_closure_fit_normalization(chan_closure *m, float *norm_out)
 {
     if (!m || m->count < 2) return CHAN_EINVAL;
     CLK(m, cudaSetDevice(m->dev));
+    std::lock_guard<std::mutex> lock(m->acc_mu);
     double *acc = m->acc;
     CLK(m, cudaMemsetAsync(acc, 0, 44 * sizeof(double), m->stream));
     k_colstats<kIn><<<2 * m->sms, 256, 0, m->stream>>>(m->X, m->count, acc, acc + 13);
