@@ -24,9 +24,10 @@ int chan_internal_sample(chan_ctx *c, float *X, float *T, long long capacity, in
 
 // MLP inference on device arrays: Y [n][9] in physical units from X [n][13]
 // (soa: X [13][n] and Y [9][n]); sets *flag (device) when a normalised output
-// exceeds the closure's limit.  Queued on `stream`, not synchronised.
+// exceeds the closure's limit, and *err (null: the closure's own word) when an MMA did
+// not complete in time.  Queued on `stream`, not synchronised.
 int chan_internal_infer(chan_closure *m, const float *X, float *Y, long long n, bool soa, cudaStream_t stream,
-                        int *flag, bool early);
+                        int *flag, bool early, int *err = nullptr);
 int chan_internal_closure_device(chan_closure *m);
 
 // ---- early launches.  A kernel of a step takes 5..30 us on a small grid, and a plain

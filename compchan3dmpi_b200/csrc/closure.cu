@@ -735,6 +735,7 @@ struct chan_closure {
     size_t ws_bytes = 0;
     std::mutex ws_mu;
     std::mutex acc_mu;                      // one call at a time uses acc
+    std::mutex sum_mu;                      // one call at a time uses part, g, loss and err
     std::shared_ptr<HostCopy> hc;           // staged copies (host_copy.h), from the first large one on
     std::string msg;
 };
@@ -812,11 +813,12 @@ cudaError_t host_copy(chan_closure *m, void *dst, const void *src, size_t n, cud
 constexpr long long kBatchKeep = 1 << 20;   // 92 MB
 struct Batch {
     float *X = nullptr, *Y = nullptr, *own = nullptr;
+    int *err = nullptr;   // the call's own error word, behind Y
     cudaError_t e = cudaSuccess;
     std::unique_lock<std::mutex> lock;
     Batch(chan_closure *m, long long n) : lock(m->ws_mu, std::try_to_lock)
     {
-        const size_t xw = ((size_t)n * kIn + 63) / 64 * 64, bytes = (xw + (size_t)n * kOut) * sizeof(float);
+        const size_t xw = ((size_t)n * kIn + 63) / 64 * 64, yw = (size_t)n * kOut, bytes = (xw + yw + 1) * sizeof(float);
         if (n > kBatchKeep || !lock.owns_lock()) {
             e = cudaMalloc((void **)&own, bytes);
             X = own;
@@ -831,16 +833,17 @@ struct Batch {
             X = m->ws;
         }
         Y = X ? X + xw : nullptr;
+        err = X ? (int *)(Y + yw) : nullptr;
     }
     ~Batch() { if (own) cudaFree(own); }
     Batch(const Batch &) = delete;
     Batch &operator=(const Batch &) = delete;
 };
 
-int check_err(chan_closure *m)
+int check_err(chan_closure *m, const int *err)
 {
     int h = 0;
-    CLK(m, cudaMemcpyAsync(&h, m->err, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+    CLK(m, cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
     CLK(m, cudaStreamSynchronize(m->stream));
     if (h) { m->msg = "tensor-core wait gave up"; return CHAN_ECUDA; }
     return CHAN_OK;
@@ -849,10 +852,11 @@ int check_err(chan_closure *m)
 }  // namespace
 
 int chan_internal_infer(chan_closure *m, const float *X, float *Y, long long n, bool soa, cudaStream_t stream,
-                        int *flag, bool early)
+                        int *flag, bool early, int *err)
 {
     MlpParams P = base_params(m);
     P.X = X; P.Y = Y; P.n = n; P.rows = n; P.row0 = 0; P.flag = flag;
+    if (err) P.err = err;
     if (soa) { P.xr = 1; P.xc = n; P.yr = 1; P.yc = n; }
     return launch_infer(m, P, stream, early);
 }
@@ -1077,6 +1081,7 @@ int chan_closure_train(chan_closure *m, int32_t epochs, int32_t batch, double lr
     if (!m || epochs < 0 || batch < kTile || batch % kTile || !(lr > 0)) return CHAN_EINVAL;
     if (m->count < batch) { m->msg = "fewer samples than one batch"; return CHAN_EINVAL; }
     CLK(m, cudaSetDevice(m->dev));
+    std::lock_guard<std::mutex> lock(m->sum_mu);
     CLK(m, ensure_part(m));
     CLK(m, cudaMemsetAsync(m->err, 0, sizeof(int), m->stream));
     const long long n = m->count, nb = n / batch;
@@ -1105,7 +1110,7 @@ int chan_closure_train(chan_closure *m, int32_t epochs, int32_t batch, double lr
         CLK(m, cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
         CLK(m, cudaStreamSynchronize(m->stream));
         if (losses) losses[ep] = (double)l / (9.0 * (double)batch * (double)nb);
-        int r = check_err(m);
+        int r = check_err(m, m->err);
         if (r) return r;
     }
     return CHAN_OK;
@@ -1115,6 +1120,7 @@ int chan_closure_grad(chan_closure *m, const float *X, const float *T, int64_t n
 {
     if (!m || !X || !T || n < 1) return CHAN_EINVAL;
     CLK(m, cudaSetDevice(m->dev));
+    std::lock_guard<std::mutex> lock(m->sum_mu);
     CLK(m, ensure_part(m));
     Batch b(m, n);
     CLK(m, b.e);
@@ -1133,7 +1139,7 @@ int chan_closure_grad(chan_closure *m, const float *X, const float *T, int64_t n
     CLK(m, cudaGetLastError());
     int r = CHAN_OK;
     float l = 0.f;
-    if (!r) r = check_err(m);
+    if (!r) r = check_err(m, m->err);
     if (!r && grads) CLK(m, cudaMemcpy(grads, m->g, (size_t)kNParam * sizeof(float), cudaMemcpyDeviceToHost));
     if (!r) CLK(m, cudaMemcpy(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost));
     if (loss_sum) *loss_sum = l;
@@ -1148,9 +1154,9 @@ int chan_closure_infer(chan_closure *m, const float *X, int64_t n, float *Y)
     CLK(m, b.e);
     float *dX = b.X, *dY = b.Y;
     CLK(m, host_copy(m, dX, X, (size_t)n * kIn * sizeof(float), cudaMemcpyHostToDevice));
-    CLK(m, cudaMemsetAsync(m->err, 0, sizeof(int), m->stream));
-    int r = chan_internal_infer(m, dX, dY, n, false, m->stream, nullptr, false);
-    if (!r) r = check_err(m);
+    CLK(m, cudaMemsetAsync(b.err, 0, sizeof(int), m->stream));
+    int r = chan_internal_infer(m, dX, dY, n, false, m->stream, nullptr, false, b.err);
+    if (!r) r = check_err(m, b.err);
     if (!r) CLK(m, host_copy(m, Y, dY, (size_t)n * kOut * sizeof(float), cudaMemcpyDeviceToHost));
     return r;
 }

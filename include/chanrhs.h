@@ -367,7 +367,11 @@ int chan_debug_canaries(chan_ctx *c, int64_t *corrupted);
  * Both are normalised by a per-column mean and standard deviation
  * (norm[44] = input means[13], input sds[13], output means[9], output sds[9]).
  * Parameters: W1[64][13] b1[64] W2[64][64] b2[64] W3[9][64] b3[9]
- * (chan_closure_nparams() floats). */
+ * (chan_closure_nparams() floats).
+ * Threading: chan_closure_infer, _grad, _train and _fit_normalization may be
+ * called on one closure by several threads (the last three take turns); calls
+ * that change its samples, parameters or normalisation, and chan_closure_free,
+ * must not overlap any other. */
 typedef struct chan_closure chan_closure;
 /* capacity: samples the device dataset holds (13 + 9 floats each) */
 int chan_closure_create(int32_t device, int64_t capacity, chan_closure **out);

@@ -37,3 +37,29 @@ def test_normalization():
         for outs in _both(lambda _: cl.fit_normalization(), (0, 1)):
             for out in outs:
                 np.testing.assert_allclose(out, ref, rtol=2.0 ** -22, atol=2e-7)
+
+
+def test_gradients():
+    """The same sums but for the order of the CTA's eight float additions per bias: 8 * 2^-24
+    of a group's norm, bounded by 1e-5."""
+    rng = np.random.default_rng(4)
+    data = [(rng.standard_normal((n, 13)).astype(np.float32), rng.standard_normal((n, 9)).astype(np.float32))
+            for n in (700, 5000)]
+    with _closure() as cl:
+        refs = [cl.grad(*d) for d in data]
+        for (lo, g), outs in zip(refs, _both(lambda d: cl.grad(*d), data)):
+            for l1, g1 in outs:
+                assert abs(l1 - lo) <= 1e-5 * abs(lo)
+                assert np.linalg.norm(g1 - g) <= 1e-5 * np.linalg.norm(g)
+
+
+@pytest.mark.parametrize("n", [700, 322639])     # rows of 52 bytes: 16 MB and more is staged
+def test_inference(n):
+    rng = np.random.default_rng(n)
+    X = [rng.standard_normal((m, 13)).astype(np.float32) for m in (n, n + 129)]
+    with _closure() as cl:
+        refs = [cl.infer(x) for x in X]
+        with ThreadPoolExecutor(2) as ex:
+            outs = list(ex.map(lambda x: [cl.infer(x) for _ in range(4)], X))
+    for ref, out in zip(refs, outs):
+        assert all(np.array_equal(y, ref) for y in out)
