@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "chan_internal.h"
+#include "phase_bits.h"
 
 namespace chan {
 
@@ -690,10 +691,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long *bar, unsig
 // One CTA's work of the stage kernel on tile (bx, by) and k-chunk bz, for
 // thread (tx, ty).  BUOYM: 0 no buoyancy term, 1 with it, 2 as P.buoy_on
 // says.  PERSIST: called from the persistent ensemble kernel, where the state
-// was written earlier in the same launch: a proxy fence before the first box copy.
+// was written earlier in the same launch: a proxy fence before the first box copy; *stuck
+// is set when the CTA must not use its shared memory again.
 template <int TI, int TJ, typename QI, typename QO, typename R, int BUOYM, bool PERSIST>
 __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *tmq, const CUtensorMap *tmb, int bx, int by,
-                                           int bz, int tx, int ty, unsigned char *smem_raw)
+                                           int bz, int tx, int ty, unsigned char *smem_raw, int *stuck)
 {
     using S = StageShape<TI, TJ, R>;
     using Slot = SlotT<R>;
@@ -765,7 +767,7 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
     // planes t, t+1, t+2; prims offsets of t, t+1; mu offsets of t, t+1
     int iZ = 1, iP = 2, iN = 0;
     int pZ = 0, pP = 4 * NB, mZ = 0, mP = NB;
-    unsigned ph = 0u;   // parity of the next wait, per barrier
+    PhaseBits ph;   // of the next wait, per barrier
     auto slot = [&](int o) -> Slot {
         return Slot{sPr + o, sPr + o + NB, sPr + o + 2 * NB, sPr + o + 3 * NB};
     };
@@ -804,21 +806,25 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
     };
     // wait for barrier s; false if its copies did not complete in time
     auto wait_slot = [&](int s) -> bool {
-        const bool ok = mbar_wait_bounded(&bar[s], (ph >> s) & 1u);
-        ph ^= 1u << s;
+        const bool ok = mbar_wait_bounded(&bar[s], ph.next(s));
+        ph.waited(s);
         if (ok && tid == 0) sflag[1] &= ~(1 << s);
         return ok;
     };
-    // after a timed-out copy: record it, give every copy still in flight one
-    // more bounded wait (so that none lands after the CTA has left), leave
-    auto give_up = [&]() {
+    // after a timed-out copy: record it and give every copy still in flight one more bounded
+    // wait, so that none lands after the CTA has left its shared memory; if one still may, a
+    // CTA of the persistent kernel takes up no other unit (*stuck).  waited: the slots whose
+    // latest copy has been waited for.
+    auto give_up = [&](int waited) {
+        if (!FOLD) cp_async_wait<0>();
         if (tid == 0) {
             atomicExch(&P.status->stall, 1);
             for (int s = 0; s < 4; s++)
-                if (sflag[1] & (1 << s)) mbar_wait_bounded(&bar[s], (ph >> s) & 1u);
+                if (sflag[1] & (1 << s)) {
+                    if (!mbar_wait_bounded(&bar[s], ph.open(s, (waited >> s) & 1)) && PERSIST) *stuck = 1;
+                }
         }
     };
-
 
     // own columns, carried from plane to plane: Q at t-1 and t-2, u, v, w, T at
     // t-1, w at t-2, hD at t-1; and what is known of plane t-1's update, which only
@@ -1145,7 +1151,7 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
     convert(kb - 1, 0, pP, mP, false);
     bad = !wait_slot(1) || bad;
     convert(kb, 1, pZ, mZ, false);
-    if (__syncthreads_or(bad)) { give_up(); return; }
+    if (__syncthreads_or(bad)) { give_up(3); return; }   // slots 0 and 1
 
     {
         const Slot sA = slot(pP), sB = slot(pZ);
@@ -1331,7 +1337,7 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
         bad = !wait_slot(iP) || bad;
         if (FOLD && need_base) bad = !wait_slot(3) || bad;
         convert(t + 1, iP, pP, mP, true, &Fxy);
-        if (__syncthreads_or(bad)) { give_up(); return; }
+        if (__syncthreads_or(bad)) { give_up(15); return; }   // every slot in use
         if (t < ke) {
             issue(t + 2, iN);
             issue_base(t + 1);
@@ -1534,7 +1540,7 @@ __global__ void __launch_bounds__(StageShape<TI, TJ, R>::NT, StageShape<TI, TJ, 
     extern __shared__ __align__(128) unsigned char smem_raw[];
     grid_dep_enter();
     stage_body<TI, TJ, QI, QO, R, BUOY ? 1 : 0, false>(P, &tmq, &tmb, blockIdx.x, blockIdx.y, blockIdx.z, threadIdx.x,
-                                                       threadIdx.y, smem_raw);
+                                                       threadIdx.y, smem_raw, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -2564,11 +2570,11 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 constexpr unsigned long long kDepWaitNs = 1000000000ull;
 
 template <int TI, int TJ, typename QI, typename QO, typename R>
-__device__ __forceinline__ void pstage(const PPhase &F, const KParams &P, int unit, int tid, unsigned char *smem)
+__device__ __forceinline__ void pstage(const PPhase &F, const KParams &P, int unit, int tid, unsigned char *smem, int *stuck)
 {
     using S = StageShape<TI, TJ, R>;
     const int bx = unit % F.nx, r = unit / F.nx, by = r % F.ny, bz = r / F.ny;
-    stage_body<TI, TJ, QI, QO, R, 2, true>(P, F.tm, F.tmb, bx, by, bz, tid % S::TX, tid / S::TX, smem);
+    stage_body<TI, TJ, QI, QO, R, 2, true>(P, F.tm, F.tmb, bx, by, bz, tid % S::TX, tid / S::TX, smem, stuck);
 }
 
 template <bool MIXED>
@@ -2597,13 +2603,16 @@ __global__ void __launch_bounds__(PersistShape<MIXED>::NT, PersistShape<MIXED>::
     extern __shared__ __align__(128) unsigned char smem_raw[];
     long long *s_item = reinterpret_cast<long long *>(smem_raw + PS::body);
     int *s_ok = reinterpret_cast<int *>(s_item + 1);
+    int *s_stuck = s_ok + 1;   // a stage's copy may still land in this CTA's shared memory
     const int tid = threadIdx.x;
+    if (tid == 0) *s_stuck = 0;
     for (;;) {
         if (tid == 0) {
             // the next unit of the work list; wait (bounded) until its member has
             // completed the units of its earlier phases
             long long it = (long long)atomicAdd(plan.next, 1ull);
-            if (it < plan.nitems && *(volatile int *)plan.err) it = plan.nitems;   // after an error: stop
+            // after an error, or with a copy that may still land here: stop
+            if (it < plan.nitems && (*(volatile int *)plan.err || *s_stuck)) it = plan.nitems;
             int ok = 1;
             if (it < plan.nitems) {
                 const PPhase &F = plan.phases[plan.items[it].phase];
@@ -2642,16 +2651,16 @@ __global__ void __launch_bounds__(PersistShape<MIXED>::NT, PersistShape<MIXED>::
             break;
         case kPStage:
             if (!MIXED) {
-                if (F.tile == 0) pstage<32, 8, double, double, double>(F, P, I.unit, tid, smem_raw);
-                else pstage<16, 16, double, double, double>(F, P, I.unit, tid, smem_raw);
+                if (F.tile == 0) pstage<32, 8, double, double, double>(F, P, I.unit, tid, smem_raw, s_stuck);
+                else pstage<16, 16, double, double, double>(F, P, I.unit, tid, smem_raw, s_stuck);
             } else if (F.tile == 0) {
-                if (F.variant == 1) pstage<32, 8, double, float, float>(F, P, I.unit, tid, smem_raw);
-                else if (F.variant == 2) pstage<32, 8, float, float, float>(F, P, I.unit, tid, smem_raw);
-                else pstage<32, 8, float, double, float>(F, P, I.unit, tid, smem_raw);
+                if (F.variant == 1) pstage<32, 8, double, float, float>(F, P, I.unit, tid, smem_raw, s_stuck);
+                else if (F.variant == 2) pstage<32, 8, float, float, float>(F, P, I.unit, tid, smem_raw, s_stuck);
+                else pstage<32, 8, float, double, float>(F, P, I.unit, tid, smem_raw, s_stuck);
             } else {
-                if (F.variant == 1) pstage<16, 16, double, float, float>(F, P, I.unit, tid, smem_raw);
-                else if (F.variant == 2) pstage<16, 16, float, float, float>(F, P, I.unit, tid, smem_raw);
-                else pstage<16, 16, float, double, float>(F, P, I.unit, tid, smem_raw);
+                if (F.variant == 1) pstage<16, 16, double, float, float>(F, P, I.unit, tid, smem_raw, s_stuck);
+                else if (F.variant == 2) pstage<16, 16, float, float, float>(F, P, I.unit, tid, smem_raw, s_stuck);
+                else pstage<16, 16, float, double, float>(F, P, I.unit, tid, smem_raw, s_stuck);
             }
             break;
         case kPWall: {
