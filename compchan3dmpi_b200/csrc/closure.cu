@@ -6,6 +6,7 @@
 #include "chanrhs.h"
 #include "chan_internal.h"
 #include "host_copy.h"
+#include "phase_bits.h"
 #include "umma.cuh"
 
 #include <cuda_bf16.h>
@@ -210,6 +211,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
     __shared__ __align__(8) uint64_t ready[kGroups], done[kGroups];
     __shared__ uint32_t tbase;
     __shared__ int sfail;
+    __shared__ CommitBits slog;   // the issuer's commits
     __shared__ float wloss[2][kGroups][4];   // loss sums of a tile's warps, by tile parity and group
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     float *fb1 = (float *)(sm + S::fl), *fb2 = fb1 + 64, *fb3 = fb2 + 64, *nrm = fb3 + 16;
@@ -250,6 +252,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
         if (lane == 0) {
             const int n0 = count(0), n1 = count(1);
             uint32_t ph[kGroups] = {0, 0};
+            CommitBits log{};
             bool acc2 = false, acc1 = false, acc3 = false, ok = true;
             float loss = 0.f;   // the CTA's tiles and their warps added in order: reproducible
             for (int it = 0; it <= n0 && ok; it++)
@@ -287,8 +290,10 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
                             acc2 = true;
                         }
                         umma::commit(&done[g]);
+                        log.committed(g);
                     }
             if (!ok) atomicExch(&sfail, 1);
+            slog = log;
             sloss[0] = loss;
         }
     } else {
@@ -453,9 +458,10 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
         else if (tid == 96) atomicAdd(P.loss, sloss[0]);
     }
     if (sfail && tid == 0) {
-        // an MMA did not signal completion: give the groups' barriers one more bounded
-        // wait each before the tensor memory they write is released
-        for (int g = 0; g < kGroups; g++) umma::mbar_wait(&done[g], 0, kWaitLimit);
+        // an MMA did not signal completion: give each group's last commit one more bounded
+        // wait before the tensor memory it writes is released
+        for (int g = 0; g < kGroups; g++)
+            if (slog.some(g)) umma::mbar_wait(&done[g], slog.last(g), kWaitLimit);
         atomicExch(P.err, 1);
     }
     umma::fence_before_sync();

@@ -19,3 +19,16 @@ struct PhaseBits {
     // that wait ran out, else the next.  (A test of the other parity succeeds at once.)
     CHAN_HD unsigned open(int s, bool ran_out) const { return ((bits >> s) & 1u) ^ (ran_out ? 1u : 0u); }
 };
+
+// The phases of up to 32 barriers that one thread's commits complete: whether a barrier has
+// had one, and the parity of its last, the one to wait for before leaving.
+struct CommitBits {
+    unsigned bits, any;   // start from {} (no initialisers: it is also a shared variable)
+    CHAN_HD void committed(int s)
+    {
+        bits ^= 1u << s;
+        any |= 1u << s;
+    }
+    CHAN_HD bool some(int s) const { return (any >> s) & 1u; }
+    CHAN_HD unsigned last(int s) const { return ((bits >> s) & 1u) ^ 1u; }
+};

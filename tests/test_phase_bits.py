@@ -48,6 +48,25 @@ int main()
 }
 """
 
+COMMITS = r"""
+int main()
+{
+    for (unsigned n = 1; n < 9; n++)
+        for (int s = 0; s < 2; s++) {
+            Barrier b[2];
+            CommitBits log{};
+            CHECK(!log.some(0) && !log.some(1));
+            for (unsigned k = 0; k < n; k++) log.committed(s);
+            CHECK(log.some(s) && !log.some(1 - s));
+            b[s].done = n - 1;                   // all but the last are complete
+            CHECK(!b[s].test(log.last(s)));
+            b[s].done = n;
+            CHECK(b[s].test(log.last(s)));
+        }
+    return 0;
+}
+"""
+
 
 def run(tmp_path, program):
     src, exe = tmp_path / "t.cpp", tmp_path / "t"
@@ -59,3 +78,7 @@ def run(tmp_path, program):
 
 def test_wait_that_ran_out_keeps_its_phase(tmp_path):
     run(tmp_path, WAITS)
+
+
+def test_wait_for_the_last_commit(tmp_path):
+    run(tmp_path, COMMITS)
