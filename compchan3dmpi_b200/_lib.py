@@ -119,6 +119,7 @@ SIGNATURES = [
     ("chan_selftest_umma", ctypes.c_int, [ctypes.POINTER(ctypes.c_uint16), ctypes.POINTER(ctypes.c_uint16),
                                           ctypes.POINTER(ctypes.c_float), ctypes.c_int32, ctypes.c_int32,
                                           ctypes.c_int32]),
+    ("chan_selftest_adam", ctypes.c_int, [_F, _F, _F, _F, ctypes.c_float, ctypes.c_int32, ctypes.c_int32]),
     ("chan_closure_create", ctypes.c_int, [ctypes.c_int32, ctypes.c_int64, ctypes.POINTER(ctypes.c_void_p)]),
     ("chan_closure_sample", ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32,
                                            ctypes.c_int32, ctypes.c_int32, _I64]),

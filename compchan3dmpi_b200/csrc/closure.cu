@@ -608,6 +608,17 @@ __device__ __forceinline__ void put_images(int i, float x, unsigned char *img)
     }
 }
 
+// parameter of entry q of a CTA's sums
+__host__ __device__ __forceinline__ int part_param(int q)
+{
+    if (q < kPartW2) return (q % kHid) * kIn + q / kHid;
+    if (q < kPartW3) return kOffW2 + ((q - kPartW2) % kHid) * kHid + (q - kPartW2) / kHid;
+    if (q < kPartB1) return kOffW3 + (q - kPartW3);
+    if (q < kPartB2) return kOffB1 + (q - kPartB1);
+    if (q < kPartB3) return kOffB2 + (q - kPartB2);
+    return kOffB3 + (q - kPartB3);
+}
+
 // gradient of 32 parameters (partial-layout indices 32*blockIdx.x ..) from the CTAs'
 // sums: eight warps add a share of the CTAs each, warp 0 adds those.  Returns the
 // parameter index of warp 0's lane, or -1.
@@ -626,30 +637,28 @@ __device__ __forceinline__ int sum_parts(const float *part, int nparts, float (&
     g = 0.f;
 #pragma unroll
     for (int w = 0; w < kSumThreads / 32; w++) g += acc[w][lane];
-    if (q < kPartW2) return (q % kHid) * kIn + q / kHid;
-    if (q < kPartW3) return kOffW2 + ((q - kPartW2) % kHid) * kHid + (q - kPartW2) / kHid;
-    if (q < kPartB1) return kOffW3 + (q - kPartW3);
-    if (q < kPartB2) return kOffB1 + (q - kPartB1);
-    if (q < kPartB3) return kOffB2 + (q - kPartB2);
-    return kOffB3 + (q - kPartB3);
+    return part_param(q);
 }
 constexpr int kSumBlocks = (kPartN + 31) / 32;
 
-// one Adam step of every parameter, with its BF16 images
+// one Adam step of every parameter, with its BF16 images; none after a training kernel
+// that gave up (*err), whose sums are not all there
 __global__ void __launch_bounds__(kSumThreads) k_adam(float *w, float *m, float *v, const float *part, int nparts,
-                                                      unsigned char *img, float lr, float b1, float b2, float eps,
-                                                      float c1, float c2)
+                                                      unsigned char *img, const int *err, float lr, float b1, float b2,
+                                                      float eps, float c1, float c2)
 {
     __shared__ float acc[kSumThreads / 32][32];
     grid_dep_enter();   // the training kernel's sums
     float gi;
     const int i = sum_parts(part, nparts, acc, gi);
     if (i < 0) return;
+    const int failed = *err;
     const float mi = b1 * m[i] + (1.f - b1) * gi;
     const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+    const float x = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    if (failed) return;   // after the loads, beside which its own costs nothing
     m[i] = mi;
     v[i] = vi;
-    const float x = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     w[i] = x;
     put_images(i, x, img);
 }
@@ -961,6 +970,36 @@ int chan_closure_create(int32_t device, int64_t capacity, chan_closure **out)
     return CHAN_OK;
 }
 
+int chan_selftest_adam(float *w, float *mom1, float *mom2, const float *grad, float lr, int32_t failed, int32_t device)
+{
+    if (!w || !mom1 || !mom2 || !grad || !(lr > 0)) return CHAN_EINVAL;
+    chan_closure *m = nullptr;
+    int r = chan_closure_create(device, 0, &m);
+    if (r) return r;
+    std::vector<float> part(kPartStride, 0.f);
+    for (int q = 0; q < kPartN; q++) part[q] = grad[part_param(q)];
+    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    const int err = failed ? 1 : 0;
+    constexpr size_t np = (size_t)kNParam * sizeof(float);
+    cudaError_t e = ensure_part(m);
+    if (e == cudaSuccess) e = cudaMemcpy(m->part, part.data(), kPartStride * sizeof(float), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(m->err, &err, sizeof(int), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(m->w, w, np, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(m->m, mom1, np, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(m->v, mom2, np, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    if (e == cudaSuccess)
+        e = launch_kernel(false, k_adam, kSumBlocks, kSumThreads, 0, m->stream, m->w, m->m, m->v, m->part, 1, m->img,
+                          m->err, lr, b1, b2, eps, 1.f - b1, 1.f - b2);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
+    if (e == cudaSuccess) e = cudaMemcpy(w, m->w, np, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(mom1, m->m, np, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(mom2, m->v, np, cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) g_cl_error = cudaGetErrorString(e);
+    chan_closure_free(m);
+    return e == cudaSuccess ? CHAN_OK : CHAN_ECUDA;
+}
+
 int chan_closure_sample(chan_closure *m, chan_ctx *dns, int32_t sx, int32_t sy, int32_t sz, int32_t fw,
                         int64_t *added)
 {
@@ -1110,7 +1149,7 @@ int chan_closure_train(chan_closure *m, int32_t epochs, int32_t batch, double lr
             m->adam_t++;
             const float c1 = 1.f - std::pow(b1, (float)m->adam_t), c2 = 1.f - std::pow(b2, (float)m->adam_t);
             CLK(m, launch_kernel(true, k_adam, kSumBlocks, kSumThreads, 0, m->stream, m->w, m->m, m->v, m->part, grid, m->img,
-                                (float)lr, b1, b2, eps, c1, c2));
+                                m->err, (float)lr, b1, b2, eps, c1, c2));
         }
         float l = 0.f;
         CLK(m, cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));

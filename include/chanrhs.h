@@ -425,6 +425,12 @@ int chan_closure_flag(chan_ctx *c, int32_t *flag, int32_t reset);
  * closure MLP uses (K and N multiples of 16 up to 256).  For tests. */
 int chan_selftest_umma(const uint16_t *A, const uint16_t *B, float *D, int32_t K, int32_t N, int32_t device);
 
+/* Self-test of the optimiser kernel: its first Adam step (lr; beta 0.9, 0.999; eps 1e-8)
+ * of parameters w with moments mom1, mom2 from the gradient grad, all
+ * chan_closure_nparams() floats; with failed != 0 as after a training kernel that gave
+ * up, when it must leave all three as they are. */
+int chan_selftest_adam(float *w, float *mom1, float *mom2, const float *grad, float lr, int32_t failed, int32_t device);
+
 /* Free device memory and the context.  NULL is allowed.  A context that is a
  * member of an ensemble is freed after its ensemble. */
 void chan_free(chan_ctx *c);
