@@ -1746,6 +1746,24 @@ int build_persistent(chan_ensemble *e)
 {
     const size_t n = e->m.size();
     const bool mixed = e->m[0]->mixed;
+    const void *fn = mixed ? (const void *)chan::k_ensemble<true> : (const void *)chan::k_ensemble<false>;
+    const int nth = mixed ? chan::PersistShape<true>::NT : chan::PersistShape<false>::NT;
+    const size_t smem = mixed ? chan::PersistShape<true>::bytes : chan::PersistShape<false>::bytes;
+    EK(e, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int occ = 0, sms = 148;
+    EK(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, nth, smem));
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev);
+    e->pgrid = std::max(1, occ) * sms;
+
+    // wall and image blocks per unit: as many as spread the members' blocks once over the
+    // CTAs, eight at most.  They are short, so a unit of eight saves its hand-out where there
+    // are many (16 cases of the stratified sweep: 93 ms for 30 steps, 97 one by one), but a
+    // member waits for its units: two members of 24x14x19 take 2.7 to 3.0 ms for 50 steps one
+    // by one and 4.7 to 5.7 by eight, one of 128x128x97 20 and 24 to 27.
+    long long edges = 0;
+    for (chan_ctx *c : e->m) edges += chan::edge_blocks(c->n1, c->n2, c->n3);
+    const int group = (int)std::min<long long>(8, (edges + e->pgrid - 1) / e->pgrid);
+
     std::vector<chan::KParams> kps;
     std::vector<CUtensorMap> maps, bmaps;   // per stage record: the input's map; per member: the RK base's
     std::vector<std::vector<chan::PPhase>> per(n);
@@ -1786,7 +1804,7 @@ int build_persistent(chan_ensemble *e)
                 chan::PPhase w{};
                 w.kind = chan::kPWall;
                 w.variant = (c->mixed && !last) ? 1 : 0;
-                w.group = 8;
+                w.group = group;
                 w.units = (chan::edge_blocks(c->n1, c->n2, c->n3) + w.group - 1) / w.group;
                 w.kp = kp0 + it - 1;
                 add(w);
@@ -1843,15 +1861,6 @@ int build_persistent(chan_ensemble *e)
     EK(e, cudaMemsetAsync(e->derr, 0, sizeof(int), e->origin));
     EK(e, cudaStreamSynchronize(e->origin));   // the host vectors are temporaries
     e->nitems = (long long)items.size();
-
-    const void *fn = mixed ? (const void *)chan::k_ensemble<true> : (const void *)chan::k_ensemble<false>;
-    const int nth = mixed ? chan::PersistShape<true>::NT : chan::PersistShape<false>::NT;
-    const size_t smem = mixed ? chan::PersistShape<true>::bytes : chan::PersistShape<false>::bytes;
-    EK(e, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int occ = 0, sms = 148;
-    EK(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, nth, smem));
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev);
-    e->pgrid = std::max(1, occ) * sms;
 
     chan::PPlan plan{};
     plan.phases = e->dph; plan.items = e->ditems; plan.nitems = e->nitems;
