@@ -4,8 +4,9 @@
 //   Q  [5][nP3+2][nP2+2][px]   conservative state rho,rho*u,rho*v,rho*w,rho*E.
 //                              Indices equal the reference's solV(0:nP1+1,
 //                              0:nP2+1,0:nP3+1,1:5) (v1.10/codes/main_v1.9.f90:43).
-//                              The 2-deep periodic ghosts are written by the
-//                              stage kernel itself, so every read is plain.
+//                              The 2-deep periodic ghosts in x are written by the
+//                              stage kernel itself, those in y by the kernel after
+//                              it, so every read is plain.
 //   WP [2][8][nP2+2][px]       primitive state of the two wall planes k=1, k=nP3:
 //                              rho,u,v,w,E,T,p,mu.  The wall pressure is a
 //                              state variable of its own (pressure BC).
@@ -15,7 +16,7 @@
 //                              statistics sum them; kept only for that.
 //
 // One RK stage = k_stage (fluxes + update, fused) + k_wall (wall BC +
-// pressure BC).  k_stats_part + k_stats_fin run every istat steps.
+// pressure BC, and the ghost rows in y).  k_stats_part + k_stats_fin run every istat steps.
 #pragma once
 
 #include <cuda.h>
@@ -500,7 +501,8 @@ struct StageShape {
     // share their loads, addresses and loop overhead (32% fewer instructions), but
     // need twice the registers: that pays in float (0.343 against 0.59 ms per launch at
     // 256x193x192 with one point, in 80 registers); in FP64 two points of 255 registers
-    // leave two warps per scheduler and spill (0.715 against 0.502 ms).
+    // leave two warps per scheduler and spill (0.715 against 0.502 ms; all four without
+    // the images' stores, with which the shipped ones take 0.346 and 0.505).
     static constexpr int PX = sizeof(R) == 4 ? 2 : 1;
     static constexpr int BX = TI + 4, BY = TJ + 4, NB = BX * BY, TX = TI / PX, NT = TX * TJ;
     // fD rows: [left halo, TI own points, right halo], padded so that own pairs are
@@ -530,8 +532,8 @@ struct StageShape {
     static constexpr size_t bytes = bar_off + 5 * sizeof(unsigned long long) + 2 * sizeof(int);
     // resident CTAs per SM the register budget is sized for: as many as the
     // 228 KB of shared memory per SM hold (1 KB of it reserved per CTA), and
-    // never fewer registers than a thread needs for its two points (MINR)
-    static constexpr int MINR = PX == 2 ? (sizeof(R) == 4 ? 128 : 224) : (sizeof(R) == 4 ? 80 : 128);
+    // never fewer registers than a thread needs (one point in double, two in float)
+    static constexpr int MINR = 128;
     static constexpr int minb_smem = (int)(233472 / (bytes + 1024));
     static constexpr int minb_regs = 65536 / (MINR * NT);
     static constexpr int minb = minb_regs < minb_smem ? minb_regs : minb_smem;
@@ -717,7 +719,9 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
     R *sT = reinterpret_cast<R *>(smem_raw + S::tab_off);               // [4][kTabWords]
     double *sRB = reinterpret_cast<double *>(smem_raw + S::rb_off);     // [4][2]
     R *sH = reinterpret_cast<R *>(smem_raw + S::hl_off);                // [2][NHL]
-    // (the 8-byte rounding is a no-op: bar_off is a multiple of 8)
+    // bar_off is a multiple of 8: the mask only keeps the compiler from folding the barriers'
+    // addresses into registers of their own (without it the FP64 32x8 kernel spills 56 + 88
+    // bytes instead of 12 + 12)
     unsigned long long *bar = reinterpret_cast<unsigned long long *>(reinterpret_cast<size_t>(smem_raw + S::bar_off) & ~(size_t)7);   // [4]: Q slots, RK base
     double *stau = reinterpret_cast<double *>(bar + 4);   // tauL - tauU
     int *sflag = reinterpret_cast<int *>(bar + 5);   // [0] the CTA leaves at once, [1] copies in flight
@@ -1007,18 +1011,13 @@ __device__ __forceinline__ void stage_body(const KParams &P, const CUtensorMap *
             stp<PX>((R *)sl.T + p, T);
             stp<PX>(MU + p, mu);
         };
-        // the wall test taken once per plane, so that each loop's body is
-        // straight-line code (the per-thread box loads of both of a thread's pairs
+        // the wall test taken once per plane, so that the loop's body is
+        // straight-line code (with per-thread box loads, both of a thread's pairs' are
         // in flight at once; one pair at a time took 2.7% more of the mixed stage time, and
         // loads held across the inviscid sums spill 676 bytes)
         auto loop = [&](bool wall_plane) {
-            if (!TMA) {
 #pragma unroll
-                for (int l = 0; l < NL; l++) one(l, wall_plane);
-            } else {
-#pragma unroll
-                for (int l = 0; l < NL; l++) one(l, wall_plane);
-            }
+            for (int l = 0; l < NL; l++) one(l, wall_plane);
             if (with_xy) inv_xy(m - 1, *Fxy);
         };
         if (wall) loop(true);

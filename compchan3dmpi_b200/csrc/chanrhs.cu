@@ -358,16 +358,13 @@ int set_launch(chan_ctx *c, int tile, int nchunks)
 // cost, its pairs leaving rows of eight threads.
 int default_launch(chan_ctx *c)
 {
-    int tile = CHAN_TILE_32x8;
-    if (!c->mixed) {
-        int nc = 1;
-        double wide, square;
-        int r = best_chunks(c, CHAN_TILE_32x8, &nc, &wide);
-        if (!r) r = best_chunks(c, CHAN_TILE_16x16, &nc, &square);
-        if (r) return r;
-        if (square < 0.96 * wide) tile = CHAN_TILE_16x16;
-    }
-    return set_launch(c, tile, 0);
+    int nc = 0, ncs = 0;
+    double wide, square;
+    int r = best_chunks(c, CHAN_TILE_32x8, &nc, &wide);
+    if (!r && !c->mixed) r = best_chunks(c, CHAN_TILE_16x16, &ncs, &square);
+    if (r) return r;
+    if (!c->mixed && square < 0.96 * wide) return set_launch(c, CHAN_TILE_16x16, ncs);
+    return set_launch(c, CHAN_TILE_32x8, nc);
 }
 
 // device copy of x3 (closure features need the wall-normal coordinates)

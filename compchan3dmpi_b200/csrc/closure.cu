@@ -254,7 +254,9 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
             uint32_t ph[kGroups] = {0, 0};
             CommitBits log{};
             bool acc2 = false, acc1 = false, acc3 = false, ok = true;
-            float loss = 0.f;   // the CTA's tiles and their warps added in order: reproducible
+            // the CTA's tiles and their warps are added in order; the CTAs' sums, and a CTA's
+            // bias sums, by float atomics in the order of arrival
+            float loss = 0.f;
             for (int it = 0; it <= n0 && ok; it++)
                 for (int step = 0; step < 5 && ok; step++)
                     for (int g = 0; g < kGroups && ok; g++) {
