@@ -499,10 +499,9 @@ template <int TI, int TJ, typename R>
 struct StageShape {
     // NT threads of PX neighbouring x points each, TX per row of the tile.  Two points
     // share their loads, addresses and loop overhead (32% fewer instructions), but
-    // need twice the registers: that pays in float (0.343 against 0.59 ms per launch at
+    // need twice the registers: that pays in float (0.344 against 0.398 ms per launch at
     // 256x193x192 with one point, in 80 registers); in FP64 two points of 255 registers
-    // leave two warps per scheduler and spill (0.715 against 0.502 ms; all four without
-    // the images' stores, with which the shipped ones take 0.346 and 0.505).
+    // leave two warps per scheduler (0.718 against 0.502 ms).
     static constexpr int PX = sizeof(R) == 4 ? 2 : 1;
     static constexpr int BX = TI + 4, BY = TJ + 4, NB = BX * BY, TX = TI / PX, NT = TX * TJ;
     // fD rows: [left halo, TI own points, right halo], padded so that own pairs are
